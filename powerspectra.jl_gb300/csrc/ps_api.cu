@@ -9,6 +9,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <thread>
 #include <vector>
 
@@ -33,14 +34,14 @@ struct ps_ctx {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     char err[512] = {0};
-    // warp task lists for the current (lmin, lmax): rows for the plain kernel,
-    // tiles for the chosen kernel
-    int2* d_tasks = nullptr;
-    size_t tasks_cap = 0;
-    int ntasks = 0, task_lmin = -1, task_lmax = -1;
+    // warp task list for the current (lmin, lmax)
     int2* d_tiles = nullptr;
     size_t tiles_cap = 0;
     int ntiles = 0, tile_lmin = -1, tile_lmax = -1;
+    // the plain kernels' HalfTable, for lmax up to half_lmax
+    double* d_half = nullptr;
+    size_t half_cap = 0;
+    int half_lmax = -1;
     // padded windows, raw inputs, spectra, outputs (element counts)
     double* d_win = nullptr;
     size_t win_cap = 0;
@@ -162,18 +163,8 @@ static int ensure_pinned(ps_ctx* c, size_t need)
     return PS_OK;
 }
 
-// The plain kernel's warp tasks: rows by decreasing l1 (longest families
-// first), 32 consecutive l2 per task from l2 = l1.
-static void row_task_list(int lmin, int lmax, std::vector<int2>& t)
-{
-    t.clear();
-    t.reserve((size_t)(lmax - lmin + 1) * ((lmax - lmin) / 32 + 1));
-    for (int l1 = lmax; l1 >= lmin; --l1)
-        for (int l2 = l1; l2 <= lmax; l2 += 32) t.push_back(make_int2(l1, l2));
-}
-
-// The chosen kernel's warp tasks, in tiles of kTileRows (one block): the
-// closed-form list of ps_tiles.h.  The kernel writes each tile's row halves as
+// The coupling kernels' warp tasks, in tiles of kTileRows (one block): the
+// closed-form list of ps_tiles.h.  The kernels write each tile's row halves as
 // runs of four doubles.
 static void tile_task_list(int lmin, int lmax, std::vector<int2>& t)
 {
@@ -202,19 +193,6 @@ static int upload_tasks(ps_ctx* c, const std::vector<int2>& t, int2** d, size_t*
     return PS_OK;
 }
 
-static int ensure_tasks(ps_ctx* c, int lmin, int lmax)
-{
-    if (c->task_lmin == lmin && c->task_lmax == lmax && c->d_tasks) return PS_OK;
-    std::vector<int2> t;
-    row_task_list(lmin, lmax, t);
-    c->task_lmin = c->task_lmax = -1;
-    if (int st = upload_tasks(c, t, &c->d_tasks, &c->tasks_cap)) return st;
-    c->ntasks = (int)t.size();
-    c->task_lmin = lmin;
-    c->task_lmax = lmax;
-    return PS_OK;
-}
-
 static int ensure_tiles(ps_ctx* c, int lmin, int lmax)
 {
     if (c->tile_lmin == lmin && c->tile_lmax == lmax && c->d_tiles) return PS_OK;
@@ -225,6 +203,49 @@ static int ensure_tiles(ps_ctx* c, int lmin, int lmax)
     c->ntiles = (int)t.size();
     c->tile_lmin = lmin;
     c->tile_lmax = lmax;
+    return PS_OK;
+}
+
+// C(n), U(n) and W(j) of ps::HalfTable in host memory, each rounded once: C(n + 2) = C(n) (n + 1) / (n + 2)
+// from C(0) = 1 and C(1) = 2 / pi, carried as a double and its error.
+static void half_table(int top, int nw, std::vector<double>& t)
+{
+    const double two_pi = 0x1.921fb54442d18p+2, two_pi_lo = 0x1.1a62633145c07p-52;
+    const double c1 = 0x1.45f306dc9c883p-1, c1_lo = -0x1.6b01ec5417056p-55;  // 2 / pi
+    t.assign(2 * ((size_t)top + 1) + nw, 0.0);
+    double *C = t.data(), *U = C + top + 1, *W = U + top + 1;
+    for (int par = 0; par < 2; ++par) {
+        double h = par ? c1 : 1.0, l = par ? c1_lo : 0.0;
+        for (int n = par; n <= top; n += 2) {
+            C[n] = h + l;
+            const double m = n + 1.0, g = h * m, ge = std::fma(h, m, -g) + l * m;  // C(n) (n + 1)
+            const double u = 1.0 / g;
+            U[n] = u + u * (std::fma(-u, g, 1.0) - u * ge);
+            const double d = n + 2.0, q = g / d, r = (std::fma(-q, d, g) + ge) / d;
+            h = q + r;
+            l = r - (h - q);
+        }
+    }
+    for (int j = 0; j < nw; ++j) {
+        const double m = 2.0 * j + 1.0, g = two_pi * m;
+        W[j] = g + (std::fma(two_pi, m, -g) + two_pi_lo * m);
+    }
+}
+
+// The context's HalfTable, long enough for lmax: v = 2 l2 + t reaches 4 lmax, j 2 lmax.
+static int ensure_half(ps_ctx* c, int lmax, ps::HalfTable* out)
+{
+    if (c->half_lmax < lmax) {
+        std::vector<double> t;
+        half_table(4 * lmax, 2 * lmax + 2, t);
+        c->half_lmax = -1;
+        if (int st = ensure(c, &c->d_half, &c->half_cap, t.size())) return st;
+        PS_CUDA(c, cudaMemcpyAsync(c->d_half, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        PS_CUDA(c, cudaStreamSynchronize(c->stream));
+        c->half_lmax = lmax;
+    }
+    const int top = 4 * c->half_lmax;
+    *out = ps::HalfTable{c->d_half, c->d_half + top + 1, c->d_half + 2 * ((size_t)top + 1), top};
     return PS_OK;
 }
 
@@ -341,11 +362,11 @@ void cov_window_spec(int kind, int k, int* product, int* parity)
 // bracket all of its coupling kernels (ps_last_kernel_ms).
 static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first = true, bool last = true)
 {
-    const bool chosen = mode == PS_MODE_CHOSEN;
-    int st = chosen ? ensure_tiles(c, p.lmin, p.lmax) : ensure_tasks(c, p.lmin, p.lmax);
+    int st = ensure_tiles(c, p.lmin, p.lmax);
     if (st) return st;
-    p.tasks = chosen ? c->d_tiles : c->d_tasks;
-    p.ntasks = chosen ? c->ntiles : c->ntasks;
+    p.tasks = c->d_tiles;
+    p.ntasks = c->ntiles;
+    if (mode != PS_MODE_CHOSEN && (st = ensure_half(c, p.lmax, &p.half))) return st;
     if (first) PS_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     if (mode == PS_MODE_CHOSEN)
         PS_CUDA(c, ps::launch_chosen(p, c->stream));
@@ -593,7 +614,7 @@ void ps_destroy(ps_ctx* c)
     if (!c) return;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    cudaFree(c->d_tasks);
+    cudaFree(c->d_half);
     cudaFree(c->d_tiles);
     cudaFree(c->d_win);
     cudaFree(c->d_raw);

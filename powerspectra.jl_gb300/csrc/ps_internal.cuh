@@ -5,10 +5,11 @@
 //               (2 l3 + 1) * W_k[l3] for l3 < nW and 0 beyond, so every family
 //               read (l3 <= l1 + l2 <= 2 lmax) stays in bounds without a branch.
 //   * tasks:    int2 (l1, l2_0) per warp, 32 consecutive l2 of one l1 row,
-//               heaviest rows first (the family length is 2 l1 + 1).  The
-//               plain kernel's list steps from l2 = l1 row by row; the chosen
-//               kernel's list is tiled, kTileRows consecutive rows per block
-//               over one 32-column block (see tile_task_list in ps_api.cu).
+//               heaviest rows first (the family length is 2 l1 + 1), tiled:
+//               kTileRows consecutive rows per block over one 32-column block
+//               (see tile_task_list in ps_api.cu).
+//   * half:     the plain kernels' table of C(n), 1 / (C(n) (n + 1)) and
+//               2 pi (2 j + 1) (HalfTable), kept per context.
 //   * outputs:  column-major (Julia) matrices, element (l1, l2) at
 //               (l1 - lmin) + (l2 - lmin) * ld.
 #pragma once
@@ -23,7 +24,7 @@ namespace ps {
 
 constexpr int kMaxWin = 8;       // windows (slots) per coupling launch
 constexpr int kWarpsPerBlock = 4;
-constexpr int kTileRows = 4;  // rows per tile of the chosen kernel's task list (one per warp)
+constexpr int kTileRows = 4;  // rows per tile of the task list (one per warp)
 constexpr double kInv4Pi = 0.079577471545947667884;  // 1 / (4 pi)
 
 // Family product a window is contracted with.
@@ -40,6 +41,14 @@ struct WinDesc {
     int parity;
 };
 
+// The factors of the squared (0 0 0) symbol (ps_plain_fp64.cu), for lmax: C[n] = Gamma((n + 1) / 2) /
+// (sqrt(pi) Gamma(n / 2 + 1)) and U[n] = 1 / (C[n] (n + 1)) for n = 0 .. top, and W[j] = 2 pi (2 j + 1)
+// for j = 0 .. 2 lmax + 1.
+struct HalfTable {
+    const double *C, *U, *W;
+    int top;
+};
+
 struct CouplingParams {
     int lmin, lmax;
     int nwin;
@@ -53,6 +62,7 @@ struct CouplingParams {
     int cov_kind;
     const double* S[4];  // covariance signal spectra (length >= lmax + 1), reference argument order
     const double* R[4];  // covariance noise ratios
+    HalfTable half;      // the plain kernel's factors (unset for the chosen kernel)
 };
 
 // One window of a batch: user spectrum -> padded (2l+1)W row and its split copy.

@@ -5,241 +5,322 @@
 // families (l1 l2 l3; 0 0 0) and (l1 l2 l3; -2 2 0) are generated in registers
 // and contracted with the windows on the fly.  No 3j value is ever stored.
 //
-// Mapping: one warp owns 32 consecutive l2 of one l1 row.  Every lane's family
-// has the same length 2 l1 + 1, so the lanes run in lockstep; lane i reads
-// l3 = (l2_0 + i) - l1 + t at step t, i.e. 32 consecutive window entries.
+// Mapping: one warp owns 32 consecutive l2 of one l1 row (the tiled task list of
+// ps_tiles.h: four rows per block).  Every lane's family has the same length
+// 2 l1 + 1, so the lanes run in lockstep.
 //
-// Recurrence.  With m3 = 0 and c = m2 - m1 (0 for the 00 family, 4 for 22),
-// the Schulten-Gordon relation divided by j(j+1) reads
-//     a(j+1) f(j+1) + c (2j+1) f(j) + a(j) f(j-1) = 0,
-//     a(j)^2 = P(j) = (j^2 - (l1-l2)^2) ((l1+l2+1)^2 - j^2),
-// where a(jmin) = a(jmax+1) = 0 start and stop it.  The family is run forward
-// from jmin (f = 1) over l1 + 1 points and backward from jmax (f = 1) over l1
-// points, matched by least squares on the two points jm = jmin + l1, jm + 1,
-// normalised by sum (2 l3 + 1) f^2 = 1 and sign-fixed by sgn f(jmax) =
-// (-1)^(l1 - l2) (Luscombe & Luban, Phys. Rev. E 57, 7274 (1998)).  The 00
-// family shares a(j) with the 22 family: f00(j+2) = -a(j+1)/a(j+2) f00(j).
+// Families.  With t counting the points (l3 = j = d + t forward from j = d =
+// l2 - l1, l3 = l1 + l2 - t backward), the squared (0 0 0) value is
+//     tau(t) = C(t) C(2 l1 - t) C(v - 2 l1) / (C(v) (v + 1)),   v = 2 l2 + t,
+//     C(n) = Gamma((n + 1) / 2) / (sqrt(pi) Gamma(n / 2 + 1)),
+// the closed form of the (0 0 0) symbol (Edmonds, Angular Momentum in Quantum
+// Mechanics, eq. 3.7.17) with the factorial ratios (2m)! / (4^m m!^2) = C(2m)
+// continued to odd t.  From C(n) C(n + 1) = 2 / (pi (n + 1)) it follows that
+//     tau(t) tau(t + 1) P(j + 1) = (2 / pi)^2,   P(j) = (j^2 - d^2) ((l1 + l2 + 1)^2 - j^2),
+// for even and odd t alike.  So the (2 -2 0) family f, which obeys the
+// Schulten-Gordon relation a(j+1) f(j+1) + 4 (2j+1) f(j) + a(j) f(j-1) = 0 with
+// a^2 = P, is f = sqrt(tau) h with
+//     h(t + 1) = -(2 pi (2j + 1) tau(t) h(t) + h(t - 1)):
+// no square root, no division, and with q = tau h the three products the
+// windows need are at hand, f00^2 = tau, f22^2 = q h, f00 f22 = +-q (f00 changes
+// sign from one even point to the next).  Both families have closed forms at
+// j = d and j = l1 + l2 (one term of the Racah sum),
+//     h(first)^2 = r1 / r2 forward, r1 r2 backward,  r = l (l - 1) / ((l + 1)(l + 2)),
+// with f00 and f22 of one sign there, so the two sweeps (forward over l1 + 1
+// points, backward over l1) need neither matching nor a normalisation sum.
 //
-// Only the two normalisation sums and the window sums are kept per pair, so
-// normalisation, matching and sign are applied once at the end.
+// tau factors into A(t) = C(t) C(2 l1 - t), the same for every lane of a row
+// (and for both sweeps), and B(v) = C(v - 2 l1) / (C(v) (v + 1)).  Per 32 points a
+// warp puts A and the B values its lanes meet into shared memory (one product
+// per 32 lanes and value); C and 1 / (C(v) (v + 1)) come from a table that the
+// context keeps (HalfTable, correctly rounded, so no error accumulates in tau).
+//
+// Bound: GB300's FP64 pipe (2 lanes per cycle and SM, measured 1.06 TFLOP/s),
+// which a warp instruction holds for 16 cycles; loads and integer work hide
+// behind it.  FP64 instructions per two points with all spin cases: 12 (tau, q,
+// h twice, two f22^2, four windows), where the square-root recurrence this
+// replaced took about 48 with its 1/sqrt, the normalisation sums and the
+// integer-to-double conversions.  Measured with it and now: all spin cases at lmax
+// 1999, lmin 2, 123.7 -> 34.9 ms (FP64 pipe 89 % busy); a whole host call, TT at lmax
+// 95 130 -> 47 us, EE/BB at lmax 767 8.04 -> 2.97 ms.  Errors against 128-bit
+// arithmetic are 2 to 4 times smaller (lmax 2000: 5e-15 at most, 1.5e-14 before).
 #include "ps_internal.cuh"
 #include "ps_epilogue.cuh"
 
+#include <type_traits>
+
 namespace ps {
+namespace {
 
-// P(j+1) at forward step t (j = jmin + t, jmin = d = l2 - l1), from exact integer factors:
-// (j+1-d)(j+1+d)(s-j-1)(s+j+1) = (t+1)(2d+t+1)(2l1-t)(2l2+t+2).
-__device__ __forceinline__ double fwd_P(int t, int d, int l1, int l2)
-{
-    long long u = (long long)(t + 1) * (long long)(2 * d + t + 1);
-    long long v = (long long)(2 * l1 - t) * (long long)(2 * l2 + t + 2);
-    return (double)(u * v);
-}
+constexpr int kPts = 32;   // points between refills of the shared factors
+constexpr int kHalf = 64;  // B ring: entries per parity of v (32 lanes x 32 points meet 47)
 
-// P(j) at backward step t (j = jmax - t): (2l1-t)(2l2-t)(1+t)(2l1+2l2+1-t).
-__device__ __forceinline__ double bwd_P(int t, int l1, int l2)
-{
-    long long u = (long long)(2 * l1 - t) * (long long)(2 * l2 - t);
-    long long v = (long long)(1 + t) * (long long)(2 * l1 + 2 * l2 + 1 - t);
-    return (double)(u * v);
-}
-
-struct Sums {
-    double acc[kMaxWin];
-    double n0, n2;
+struct Factors {
+    double A[kPts];
+    double F[2][kHalf], B[2][kHalf];  // by parity of v: forward sweep, backward sweep
 };
 
-// Point with l1 + l2 + l3 even: every window except ODD-parity ones takes a term.
-template <bool N00, bool N22>
-__device__ __forceinline__ void acc_even(Sums& s, const CouplingParams& p, double g0, double g2, double w, int j)
+// C(n) and 1 / (C(n) (n + 1)) for any n: indices outside the table belong to lanes that hold no pair
+__device__ __forceinline__ double tab_at(const double* __restrict__ t, int n, int top)
 {
-    double x00 = g0 * g0, x22 = g2 * g2, x02 = g0 * g2;
-    if (N00) s.n0 = fma(w, x00, s.n0);
-    if (N22) s.n2 = fma(w, x22, s.n2);
+    return __ldg(t + min(max(n, 0), top));
+}
+__device__ __forceinline__ void put_b(const CouplingParams& p, double (&ring)[2][kHalf], int v, int l1)
+{
+    ring[v & 1][(v >> 1) & (kHalf - 1)] = tab_at(p.half.C, v - 2 * l1, p.half.top) * tab_at(p.half.U, v, p.half.top);
+}
+__device__ __forceinline__ double flip(double x, int neg)  // -x where neg
+{
+    return __hiloint2double(__double2hiint(x) ^ (neg << 31), __double2loint(x));
+}
+
+// The windows of a launch by what they are contracted with: f00^2, f00 f22, and f22^2 at the even, the
+// odd or all points.  A predicated-off FP64 instruction holds the pipe like an executed one (all spin
+// cases at lmax 1999 with run-time window lists: 66.1 ms, with these forms 34.9 ms), so the kernels fix
+// the number of windows per class at compile time (kForms); a slot without a window repeats another's
+// values and its sum is dropped.
+enum Class : int { C00, C02, C22E, C22O, C22A, kClasses };
+struct PlainParams {
+    CouplingParams c;
+    const double* w[kClasses][kMaxWin];
+    signed char to[kClasses][kMaxWin];  // the window's index in c.win, or -1
+};
+
+template <int N00, int N02, int N22E, int N22O, int N22A>
+struct Sums {
+    double s00[N00 + 1], s02[N02 + 1], se[N22E + 1], so[N22O + 1], sa[N22A + 1];  // + 1: no empty arrays
+    __device__ __forceinline__ void zero()
+    {
 #pragma unroll
-    for (int k = 0; k < kMaxWin; ++k) {
-        if (k < p.nwin && p.win[k].parity != PAR_ODD) {
-            double ww = __ldg(p.win[k].wW + j);
-            double x = p.win[k].product == PROD_00_00 ? x00 : (p.win[k].product == PROD_22_22 ? x22 : x02);
-            s.acc[k] = fma(x, ww, s.acc[k]);
+        for (int k = 0; k < N00; ++k) s00[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < N02; ++k) s02[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < N22E; ++k) se[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < N22O; ++k) so[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < N22A; ++k) sa[k] = 0.0;
+    }
+    // A point with l1 + l2 + l3 even: tau = f00^2, q = tau h, f22 = sqrt(tau) h; neg: f00 < 0
+    __device__ __forceinline__ void even(const PlainParams& p, double tau, double q, double h, int neg, int j)
+    {
+#pragma unroll
+        for (int k = 0; k < N00; ++k) s00[k] = fma(tau, __ldg(p.w[C00][k] + j), s00[k]);
+        if (N02 > 0) {
+            const double x = flip(q, neg);
+#pragma unroll
+            for (int k = 0; k < N02; ++k) s02[k] = fma(x, __ldg(p.w[C02][k] + j), s02[k]);
+        }
+        if (N22E + N22A > 0) {
+            const double x = q * h;
+#pragma unroll
+            for (int k = 0; k < N22E; ++k) se[k] = fma(x, __ldg(p.w[C22E][k] + j), se[k]);
+#pragma unroll
+            for (int k = 0; k < N22A; ++k) sa[k] = fma(x, __ldg(p.w[C22A][k] + j), sa[k]);
+        }
+    }
+    __device__ __forceinline__ void odd(const PlainParams& p, double q, double h, int j)
+    {
+        if (N22O + N22A > 0) {
+            const double x = q * h;
+#pragma unroll
+            for (int k = 0; k < N22O; ++k) so[k] = fma(x, __ldg(p.w[C22O][k] + j), so[k]);
+#pragma unroll
+            for (int k = 0; k < N22A; ++k) sa[k] = fma(x, __ldg(p.w[C22A][k] + j), sa[k]);
+        }
+    }
+    // (this + o) / 4 pi into Xi, each sum to its window; the (2 -2 0) family vanishes for l1 < 2
+    __device__ __forceinline__ void give(const PlainParams& p, const Sums& o, int l1, double* Xi) const
+    {
+        const double u = l1 < 2 ? 0.0 : kInv4Pi;
+#pragma unroll
+        for (int i = 0; i < kMaxWin; ++i) {
+            Xi[i] = 0.0;
+#pragma unroll
+            for (int k = 0; k < N00; ++k)
+                if (p.to[C00][k] == i) Xi[i] = (s00[k] + o.s00[k]) * kInv4Pi;
+#pragma unroll
+            for (int k = 0; k < N02; ++k)
+                if (p.to[C02][k] == i) Xi[i] = l1 < 2 ? 0.0 : (s02[k] + o.s02[k]) * u;
+#pragma unroll
+            for (int k = 0; k < N22E; ++k)
+                if (p.to[C22E][k] == i) Xi[i] = l1 < 2 ? 0.0 : (se[k] + o.se[k]) * u;
+#pragma unroll
+            for (int k = 0; k < N22O; ++k)
+                if (p.to[C22O][k] == i) Xi[i] = l1 < 2 ? 0.0 : (so[k] + o.so[k]) * u;
+#pragma unroll
+            for (int k = 0; k < N22A; ++k)
+                if (p.to[C22A][k] == i) Xi[i] = l1 < 2 ? 0.0 : (sa[k] + o.sa[k]) * u;
+        }
+    }
+};
+
+// The (2 -2 0) family, and the (0 0 0) one with it: two sweeps, interleaved.
+template <class S>
+__device__ __forceinline__ void sweeps22(const PlainParams& P, Factors& fc, int l1, int l2_0, int l2, int lane, S& SF,
+                                         S& SB)
+{
+    const CouplingParams& p = P.c;
+    const int T = l1, d = l2 - l1, js = l1 + l2;
+    const double r1 = l1 >= 2 ? (double)l1 * (l1 - 1) / ((double)(l1 + 1) * (l1 + 2)) : 0.0;
+    const double r2 = l2 >= 2 ? (double)l2 * (l2 - 1) / ((double)(l2 + 1) * (l2 + 2)) : 1.0;
+    double hf = sqrt(r1 / r2), hb = sqrt(r1 * r2), pf = 0.0, pb = 0.0;  // |m| = 2 > l1: h = 0 throughout
+    for (int e = lane; e < 96; e += 32) {
+        put_b(p, fc.F, 2 * l2_0 + e, l1);
+        put_b(p, fc.B, 2 * (l1 + l2_0) - 31 + e, l1);
+    }
+    auto forward = [&](auto even, int t) {
+        constexpr bool E = decltype(even)::value;
+        const int v = 2 * l2 + t, j = d + t;
+        const double tau = fc.A[t & (kPts - 1)] * fc.F[!E][(v >> 1) & (kHalf - 1)], q = tau * hf;
+        if constexpr (E) SF.even(P, tau, q, hf, (t >> 1) & 1, j);
+        else SF.odd(P, q, hf, j);
+        const double n = -fma(__ldg(p.half.W + j), q, pf);
+        pf = hf;
+        hf = n;
+    };
+    auto backward = [&](auto even, int t) {
+        constexpr bool E = decltype(even)::value;
+        const int v = 2 * js - t, j = js - t;
+        const double tau = fc.A[t & (kPts - 1)] * fc.B[!E][(v >> 1) & (kHalf - 1)], q = tau * hb;
+        if constexpr (E) SB.even(P, tau, q, hb, (t >> 1) & 1, j);
+        else SB.odd(P, q, hb, j);
+        const double n = -fma(__ldg(p.half.W + j), q, pb);
+        pb = hb;
+        hb = n;
+    };
+    const std::true_type even;
+    const std::false_type odd;
+    for (int t0 = 0; t0 <= T; t0 += kPts) {
+        __syncwarp();
+        const int ta = t0 + lane;
+        fc.A[lane] = tab_at(p.half.C, ta, p.half.top) * tab_at(p.half.C, 2 * l1 - ta, p.half.top);
+        if (t0 > 0) {  // 62 of the values the lanes meet were there before
+            put_b(p, fc.F, 2 * l2_0 + t0 + 62 + lane, l1);
+            put_b(p, fc.B, 2 * (l1 + l2_0) - t0 - 31 + lane, l1);
+        }
+        __syncwarp();
+        const int end = min(t0 + kPts, T);  // both sweeps run for t < T
+        int t = t0;
+        for (; t + 1 < end; t += 2) {
+            forward(even, t);
+            backward(even, t);
+            forward(odd, t + 1);
+            backward(odd, t + 1);
+        }
+        if (t < end) {
+            forward(even, t);
+            backward(even, t);
+        }
+        if (T < t0 + kPts) {  // the middle point, t = T
+            if (T & 1) forward(odd, T);
+            else forward(even, T);
         }
     }
 }
 
-// Point with l1 + l2 + l3 odd: the 00 family vanishes, only 22^2 windows that
-// are not EVEN-only take a term.
-template <bool N22>
-__device__ __forceinline__ void acc_odd(Sums& s, const CouplingParams& p, double g2, double w, int j)
+// The (0 0 0) family alone: tau at every second point over the whole family, no recurrence.  Point
+// n has t = 2n; A and B by n = t / 2 and v / 2 = l2 + n.  Two sets of sums keep two chains.
+template <class S>
+__device__ __forceinline__ void points00(const PlainParams& P, Factors& fc, int l1, int l2_0, int l2, int lane, S& S0,
+                                         S& S1)
 {
-    if (!N22) return;
-    double x22 = g2 * g2;
-    s.n2 = fma(w, x22, s.n2);
-#pragma unroll
-    for (int k = 0; k < kMaxWin; ++k) {
-        if (k < p.nwin && p.win[k].product == PROD_22_22 && p.win[k].parity != PAR_EVEN) {
-            double ww = __ldg(p.win[k].wW + j);
-            s.acc[k] = fma(x22, ww, s.acc[k]);
-        }
-    }
-}
-
-template <bool N00, bool N22>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const CouplingParams p)
-{
-    const int gw = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    if (gw >= p.ntasks) return;  // warp-uniform
-    const int lane = threadIdx.x & 31;
-    const int2 task = p.tasks[gw];
-    const int l1 = task.x;
-    const int l2raw = task.y + lane;
-    const bool active = l2raw <= p.lmax;
-    const int l2 = active ? l2raw : p.lmax;
+    const CouplingParams& p = P.c;
     const int d = l2 - l1;
-    const int jmin = d, jmax = l1 + l2;
-    const int T = l1;
-    const bool fam22 = N22 && (l1 >= 2);
-
-    double Xi[kMaxWin];
-    if (T == 0) {
-        xi_single_term(p, l2, Xi);
-    } else {
-        // ---------------- forward from jmin: points jmin .. jm ----------------
-        Sums F;
-#pragma unroll
-        for (int k = 0; k < kMaxWin; ++k) F.acc[k] = 0.0;
-        F.n0 = F.n2 = 0.0;
-        double w = 2.0 * jmin + 1.0;
-        int j = jmin;
-        double g2c = 1.0, g2p = 0.0, aj = 0.0, g0 = 1.0;
-        int t = 0;
-        for (; t + 1 <= T; t += 2) {
-            acc_even<N00, N22>(F, p, g0, g2c, w, j);
-            double P1 = fwd_P(t, d, l1, l2);
-            double P2 = fwd_P(t + 1, d, l1, l2);
-            if (N22) {
-                double r1 = rsqrt(P1), a1 = P1 * r1;
-                double g2n = -fma(4.0 * w, g2c, aj * g2p) * r1;
-                acc_odd<N22>(F, p, g2n, w + 2.0, j + 1);
-                double r2 = rsqrt(P2), a2 = P2 * r2;
-                double g2nn = -fma(4.0 * (w + 2.0), g2n, a1 * g2c) * r2;
-                if (N00) g0 = -(a1 * r2) * g0;
-                g2p = g2n;
-                g2c = g2nn;
-                aj = a2;
-            } else {
-                // 00 alone: a(j+1)/a(j+2) = P1 / sqrt(P1 P2)
-                g0 = -(P1 * rsqrt(P1 * P2)) * g0;
-            }
-            j += 2;
-            w += 4.0;
+    put_b(p, fc.F, 2 * (l2_0 + lane), l1);
+    for (int n0 = 0; n0 <= l1; n0 += kPts) {
+        __syncwarp();
+        const int ta = 2 * (n0 + lane);
+        fc.A[lane] = tab_at(p.half.C, ta, p.half.top) * tab_at(p.half.C, 2 * l1 - ta, p.half.top);
+        put_b(p, fc.F, 2 * (l2_0 + n0 + 32 + lane), l1);
+        __syncwarp();
+        const int end = min(n0 + kPts, l1 + 1);
+        int n = n0;
+#pragma unroll 2
+        for (; n + 1 < end; n += 2) {
+            S0.even(P, fc.A[n - n0] * fc.F[0][(l2 + n) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n);
+            S1.even(P, fc.A[n + 1 - n0] * fc.F[0][(l2 + n + 1) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n + 2);
         }
-        double gm0 = 0.0, gm1 = 0.0;  // 22 at jm, jm + 1
-        if (t == T) {                 // T even: last point jm is an even point
-            acc_even<N00, N22>(F, p, g0, g2c, w, j);
-            if (N22) {
-                double P1 = fwd_P(t, d, l1, l2);
-                gm0 = g2c;
-                gm1 = -fma(4.0 * w, g2c, aj * g2p) * rsqrt(P1);
-            }
-        } else if (N22) {  // T odd: the loop stopped at jm + 1
-            gm0 = g2p;
-            gm1 = g2c;
-        }
-        const double g0s = g0;  // 00 at its non-zero matching point (jm if T even, jm + 1 if T odd)
-
-        // ---------------- backward from jmax: points jmax .. jm + 1 ----------------
-        Sums B;
-#pragma unroll
-        for (int k = 0; k < kMaxWin; ++k) B.acc[k] = 0.0;
-        B.n0 = B.n2 = 0.0;
-        double hw = 2.0 * jmax + 1.0;
-        int jb = jmax;
-        double h2c = 1.0, h2n = 0.0, an = 0.0, h0 = 1.0;
-        int tb = 0;
-        for (; tb + 2 <= T; tb += 2) {
-            acc_even<N00, N22>(B, p, h0, h2c, hw, jb);
-            double P1 = bwd_P(tb, l1, l2);
-            double P2 = bwd_P(tb + 1, l1, l2);
-            if (N22) {
-                double r1 = rsqrt(P1), a1 = P1 * r1;
-                double h2m = -fma(4.0 * hw, h2c, an * h2n) * r1;
-                acc_odd<N22>(B, p, h2m, hw - 2.0, jb - 1);
-                double r2 = rsqrt(P2), a2 = P2 * r2;
-                double h2mm = -fma(4.0 * (hw - 2.0), h2m, a1 * h2c) * r2;
-                if (N00) h0 = -(a1 * r2) * h0;
-                h2n = h2m;
-                h2c = h2mm;
-                an = a2;
-            } else {
-                h0 = -(P1 * rsqrt(P1 * P2)) * h0;
-            }
-            jb -= 2;
-            hw -= 4.0;
-        }
-        double hm0 = 0.0, hm1 = 0.0;
-        if (tb < T) {  // T odd: one more even point at jm + 1
-            acc_even<N00, N22>(B, p, h0, h2c, hw, jb);
-            if (N22) {
-                double P1 = bwd_P(tb, l1, l2);
-                hm1 = h2c;
-                hm0 = -fma(4.0 * hw, h2c, an * h2n) * rsqrt(P1);
-            }
-        } else if (N22) {
-            hm0 = h2c;
-            hm1 = h2n;
-        }
-        const double h0s = h0;
-
-        // ---------------- match, normalise, sign ----------------
-        double lam0 = N00 ? g0s / h0s : 0.0;
-        double lam2 = 0.0;
-        if (fam22) lam2 = (gm0 * hm0 + gm1 * hm1) / (hm0 * hm0 + hm1 * hm1);
-        double N0 = fma(lam0 * lam0, B.n0, F.n0);
-        double N2 = fma(lam2 * lam2, B.n2, F.n2);
-        double inv0 = N00 ? kInv4Pi / N0 : 0.0;
-        double inv2 = fam22 ? kInv4Pi / N2 : 0.0;
-        double inv02 = 0.0;
-        if (N00 && fam22) {
-            double sg = ((lam0 < 0.0) != (lam2 < 0.0)) ? -1.0 : 1.0;
-            inv02 = sg * kInv4Pi * rsqrt(N0 * N2);
-        }
-#pragma unroll
-        for (int k = 0; k < kMaxWin; ++k) {
-            Xi[k] = 0.0;
-            if (k < p.nwin) {
-                int pr = p.win[k].product;
-                if (pr != PROD_00_00 && !fam22)
-                    Xi[k] = 0.0;  // |m| = 2 > l1: the 22 family is identically zero
-                else if (pr == PROD_00_00)
-                    Xi[k] = fma(lam0 * lam0, B.acc[k], F.acc[k]) * inv0;
-                else if (pr == PROD_22_22)
-                    Xi[k] = fma(lam2 * lam2, B.acc[k], F.acc[k]) * inv2;
-                else
-                    Xi[k] = fma(lam0 * lam2, B.acc[k], F.acc[k]) * inv02;
-            }
-        }
+        if (n < end) S0.even(P, fc.A[n - n0] * fc.F[0][(l2 + n) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n);
     }
-
-    if (active) write_pair(p, l1, l2, Xi);
 }
+
+template <int N00, int N02, int N22E, int N22O, int N22A>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const PlainParams P)
+{
+    __shared__ Factors sf[kWarpsPerBlock];
+    __shared__ double stage[kWarpsPerBlock][kMaxWin * 32];
+    __shared__ TileRows rows;
+    const CouplingParams& p = P.c;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the task list is tiled: kTileRows tasks per block, rows outside [lmin, lmax] as l1 = -1
+    const int gw = (int)(blockIdx.x * (unsigned)kWarpsPerBlock) + warp;
+    const int2 task = gw < p.ntasks ? p.tasks[gw] : make_int2(-1, 0);
+    const int l1 = task.x, l2raw = task.y + lane;
+    const bool active = l1 >= 0 && l2raw >= l1 && l2raw <= p.lmax;
+    double Xi[kMaxWin];
+    if (l1 >= 0) {  // warp-uniform
+        const int l2 = min(max(l2raw, l1), p.lmax);  // lanes outside compute values nobody writes
+        using S = Sums<N00, N02, N22E, N22O, N22A>;
+        S a, b;
+        a.zero();
+        b.zero();
+        if constexpr (N02 + N22E + N22O + N22A > 0) sweeps22(P, sf[warp], l1, task.y, l2, lane, a, b);
+        else points00(P, sf[warp], l1, task.y, l2, lane, a, b);
+        a.give(P, b, l1, Xi);
+    }
+    write_tile<kMaxWin>(p, l1, task.y, active, Xi, &stage[0][0], kMaxWin * 32, rows, warp, lane);
+}
+
+struct Form {
+    int n[kClasses];
+    void (*kernel)(PlainParams);
+};
+#define PS_FORM(a, b, c, d, e) Form{{a, b, c, d, e}, k_coupling_fp64<a, b, c, d, e>}
+// Cheapest first.  They cover the mode-coupling cases of one call (up to one window per class), the
+// covariance kinds (8, 4 or 2 windows of one class, TETE's 4 and 1), ps_xi (one class), and the groups
+// that ps_mcm_set makes: whole windows (at most 4 of a class when it mixes classes), or ++ and --.
+const Form kForms[] = {
+    PS_FORM(1, 0, 0, 0, 0), PS_FORM(2, 0, 0, 0, 0), PS_FORM(4, 0, 0, 0, 0), PS_FORM(8, 0, 0, 0, 0),
+    PS_FORM(0, 1, 0, 0, 0), PS_FORM(0, 0, 1, 0, 0), PS_FORM(0, 0, 0, 1, 0), PS_FORM(1, 1, 0, 0, 0),
+    PS_FORM(0, 0, 1, 1, 0), PS_FORM(0, 0, 0, 0, 1), PS_FORM(0, 4, 0, 0, 0), PS_FORM(1, 0, 1, 1, 0),
+    PS_FORM(0, 0, 4, 0, 0), PS_FORM(1, 4, 0, 0, 0), PS_FORM(1, 1, 1, 1, 0), PS_FORM(0, 8, 0, 0, 0),
+    PS_FORM(0, 0, 8, 0, 0), PS_FORM(0, 0, 0, 8, 0), PS_FORM(2, 2, 2, 2, 0), PS_FORM(0, 0, 4, 4, 0),
+    PS_FORM(0, 0, 8, 8, 0), PS_FORM(0, 0, 0, 0, 8), PS_FORM(4, 4, 4, 4, 0),
+};
+#undef PS_FORM
+
+}  // namespace
 
 cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s)
 {
-    bool n00 = false, n22 = false;
-    for (int k = 0; k < p.nwin; ++k) {
-        if (p.win[k].product != PROD_22_22) n00 = true;
-        if (p.win[k].product != PROD_00_00) n22 = true;
-    }
     const int threads = kWarpsPerBlock * 32;
     const unsigned blocks = (unsigned)((p.ntasks + kWarpsPerBlock - 1) / kWarpsPerBlock);
     if (blocks == 0) return cudaSuccess;
-    if (n00 && n22)
-        k_coupling_fp64<true, true><<<blocks, threads, 0, s>>>(p);
-    else if (n22)
-        k_coupling_fp64<false, true><<<blocks, threads, 0, s>>>(p);
-    else
-        k_coupling_fp64<true, false><<<blocks, threads, 0, s>>>(p);
-    return cudaGetLastError();
+    PlainParams P;
+    P.c = p;
+    int n[kClasses] = {0, 0, 0, 0, 0};
+    for (int c = 0; c < kClasses; ++c)
+        for (int k = 0; k < kMaxWin; ++k) {
+            P.w[c][k] = p.win[0].wW;
+            P.to[c][k] = -1;
+        }
+    for (int k = 0; k < p.nwin; ++k) {
+        const int pr = p.win[k].product, par = p.win[k].parity;
+        if (pr != PROD_22_22 && par == PAR_ODD) continue;  // f00 vanishes at odd points: Xi = 0
+        const int c = pr == PROD_00_00 ? C00 : (pr == PROD_00_22 ? C02 : (par == PAR_EVEN ? C22E : (par == PAR_ODD ? C22O : C22A)));
+        P.w[c][n[c]] = p.win[k].wW;
+        P.to[c][n[c]++] = (signed char)k;
+    }
+    for (const Form& f : kForms) {
+        bool fits = true;
+        for (int c = 0; c < kClasses; ++c) fits = fits && n[c] <= f.n[c];
+        if (!fits) continue;
+        f.kernel<<<blocks, threads, 0, s>>>(P);
+        return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------------------
