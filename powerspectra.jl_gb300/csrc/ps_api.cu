@@ -420,6 +420,7 @@ static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* 
     int wlen = 2 * lmax + 2;
     p.wlen = wlen;
     long long nuse = nW < (int64_t)(2 * lmax + 1) ? nW : (int64_t)(2 * lmax + 1);
+    p.nw = (int)nuse;
     int st = ensure(c, &c->d_win, &c->win_cap, (size_t)K * wlen);
     if (st) return st;
     if (host) {
@@ -1004,6 +1005,7 @@ int ps_coupledcov_set_device(ps_ctx* c, int nblk, const int* kinds, const double
                 p.lmax = lmax;
                 p.epilogue = ps::EPI_XI;
                 p.wlen = wlen;
+                p.nw = (int)nuse;
                 p.nwin = (int)std::min(js.size() - i0, (size_t)ps::kMaxWin);
                 for (int q = 0; q < p.nwin; ++q) {
                     const int j = js[i0 + q];
@@ -1080,6 +1082,7 @@ int ps_mcm_set_device(ps_ctx* c, unsigned cases, const double* const* dW, int K,
             }
         }
         base.wlen = wlen;
+        base.nw = (int)nuse;
         // chosen mode: the TT slots (00 family) and the ++ / -- slots (22 family) of a set, each
         // kind with at least mma_min_slots slots, go to the tensor-core kernels, up to kMmaMaxSlots
         // windows per launch; the rest go to the CUDA-core kernels in groups of up to 8
@@ -1301,6 +1304,7 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
             g.epilogue = ps::EPI_MCM;
             g.nwin = (int)grp.size();
             g.wlen = wlen;
+            g.nw = (int)nuse;
             g.ldo = P.ldm;
             bool f00 = false, f22 = false;
             for (size_t q = 0; q < grp.size(); ++q) {

@@ -59,6 +59,7 @@ struct CouplingParams {
     double* out[kMaxWin];  // EPI_MCM / EPI_XI: one matrix per window; EPI_COV: out[0]
     long long ldo;
     int wlen;  // length of the padded window arrays
+    int nw;    // their entries at l3 >= nw are zero
     int cov_kind;
     const double* S[4];  // covariance signal spectra (length >= lmax + 1), reference argument order
     const double* R[4];  // covariance noise ratios

@@ -117,6 +117,7 @@ extern "C" int ps_mcm_multi_device_noalloc(unsigned cases, const double* const d
     p.wlen = 2 * lmax + 2;
     p.ldo = ldm;
     const long long nuse = nW < (int64_t)(2 * lmax + 1) ? nW : (int64_t)(2 * lmax + 1);
+    p.nw = (int)nuse;
     int K = 0;
     for (int sp = 0; sp < 4; ++sp) {
         if (!(cases & (1u << sp))) continue;

@@ -9,8 +9,8 @@
 // ps_tiles.h: four rows per block).  Every lane's family has the same length
 // 2 l1 + 1, so the lanes run in lockstep.
 //
-// Families.  With t counting the points (l3 = j = d + t forward from j = d =
-// l2 - l1, l3 = l1 + l2 - t backward), the squared (0 0 0) value is
+// Families.  With t counting the points (l3 = j = d + t from j = d = l2 - l1 to l1 + l2),
+// the squared (0 0 0) value is
 //     tau(t) = C(t) C(2 l1 - t) C(v - 2 l1) / (C(v) (v + 1)),   v = 2 l2 + t,
 //     C(n) = Gamma((n + 1) / 2) / (sqrt(pi) Gamma(n / 2 + 1)),
 // the closed form of the (0 0 0) symbol (Edmonds, Angular Momentum in Quantum
@@ -23,27 +23,28 @@
 //     h(t + 1) = -(2 pi (2j + 1) tau(t) h(t) + h(t - 1)):
 // no square root, no division, and with q = tau h the three products the
 // windows need are at hand, f00^2 = tau, f22^2 = q h, f00 f22 = +-q (f00 changes
-// sign from one even point to the next).  Both families have closed forms at
-// j = d and j = l1 + l2 (one term of the Racah sum),
-//     h(first)^2 = r1 / r2 forward, r1 r2 backward,  r = l (l - 1) / ((l + 1)(l + 2)),
-// with f00 and f22 of one sign there, so the two sweeps (forward over l1 + 1
-// points, backward over l1) need neither matching nor a normalisation sum.
+// sign from one even point to the next).  At j = d both families have closed
+// forms (one term of the Racah sum) of one sign, h(0)^2 = r1 / r2 with
+// r = l (l - 1) / ((l + 1)(l + 2)), so there is nothing to match or to
+// normalise, and the sweep ends where the windows do (p.nw).
 //
-// tau factors into A(t) = C(t) C(2 l1 - t), the same for every lane of a row
-// (and for both sweeps), and B(v) = C(v - 2 l1) / (C(v) (v + 1)).  Per 32 points a
-// warp puts A and the B values its lanes meet into shared memory (one product
-// per 32 lanes and value); C and 1 / (C(v) (v + 1)) come from a table that the
-// context keeps (HalfTable, correctly rounded, so no error accumulates in tau).
+// tau factors into A(t) = C(t) C(2 l1 - t), the same for every lane of a row, and
+// B(v) = C(v - 2 l1) / (C(v) (v + 1)).  Per 32 points a warp puts A and the B values
+// its lanes meet into shared memory (one product per 32 lanes and value); C and
+// 1 / (C(v) (v + 1)) come from a table that the context keeps (HalfTable, correctly
+// rounded, so no error accumulates in tau).
 //
 // Bound: GB300's FP64 pipe (2 lanes per cycle and SM, measured 1.06 TFLOP/s),
 // which a warp instruction holds for 16 cycles; loads and integer work hide
 // behind it.  FP64 instructions per two points with all spin cases: 12 (tau, q,
 // h twice, two f22^2, four windows), where the square-root recurrence this
 // replaced took about 48 with its 1/sqrt, the normalisation sums and the
-// integer-to-double conversions.  Measured with it and now: all spin cases at lmax
-// 1999, lmin 2, 123.7 -> 34.9 ms (FP64 pipe 89 % busy); a whole host call, TT at lmax
-// 95 130 -> 47 us, EE/BB at lmax 767 8.04 -> 2.97 ms.  Errors against 128-bit
-// arithmetic are 2 to 4 times smaller (lmax 2000: 5e-15 at most, 1.5e-14 before).
+// integer-to-double conversions.  Measured with it, with this form in two sweeps
+// that meet in the middle, and now: all spin cases at lmax 1999, lmin 2, nW 3999
+// 123.7, 34.9 and 32.1 ms; a whole host call (nW = lmax + 1, so that a quarter of the family lies beyond
+// the windows), TT at lmax 95 130, 47 and 44 us, EE/BB at lmax 767 8.0, 3.0 and 2.8 ms.  Errors against 128-bit
+// arithmetic are smaller than the recurrence's (lmax 2000, all points: 7e-15 at
+// most, 1.5e-14 before).
 #include "ps_internal.cuh"
 #include "ps_epilogue.cuh"
 
@@ -57,7 +58,7 @@ constexpr int kHalf = 64;  // B ring: entries per parity of v (32 lanes x 32 poi
 
 struct Factors {
     double A[kPts];
-    double F[2][kHalf], B[2][kHalf];  // by parity of v: forward sweep, backward sweep
+    double B[2][kHalf];  // by parity of v
 };
 
 // C(n) and 1 / (C(n) (n + 1)) for any n: indices outside the table belong to lanes that hold no pair
@@ -65,9 +66,9 @@ __device__ __forceinline__ double tab_at(const double* __restrict__ t, int n, in
 {
     return __ldg(t + min(max(n, 0), top));
 }
-__device__ __forceinline__ void put_b(const CouplingParams& p, double (&ring)[2][kHalf], int v, int l1)
+__device__ __forceinline__ void put_b(const CouplingParams& p, Factors& fc, int v, int l1)
 {
-    ring[v & 1][(v >> 1) & (kHalf - 1)] = tab_at(p.half.C, v - 2 * l1, p.half.top) * tab_at(p.half.U, v, p.half.top);
+    fc.B[v & 1][(v >> 1) & (kHalf - 1)] = tab_at(p.half.C, v - 2 * l1, p.half.top) * tab_at(p.half.U, v, p.half.top);
 }
 __device__ __forceinline__ double flip(double x, int neg)  // -x where neg
 {
@@ -76,7 +77,7 @@ __device__ __forceinline__ double flip(double x, int neg)  // -x where neg
 
 // The windows of a launch by what they are contracted with: f00^2, f00 f22, and f22^2 at the even, the
 // odd or all points.  A predicated-off FP64 instruction holds the pipe like an executed one (all spin
-// cases at lmax 1999 with run-time window lists: 66.1 ms, with these forms 34.9 ms), so the kernels fix
+// cases at lmax 1999 in two sweeps: 66.1 ms with run-time window lists, 34.9 ms with these forms), so the kernels fix
 // the number of windows per class at compile time (kForms); a slot without a window repeats another's
 // values and its sum is dropped.
 enum Class : int { C00, C02, C22E, C22O, C22A, kClasses };
@@ -156,93 +157,73 @@ struct Sums {
     }
 };
 
-// The (2 -2 0) family, and the (0 0 0) one with it: two sweeps, interleaved.
+// The (2 -2 0) family, and the (0 0 0) one with it, over the points t = 0 .. n.  Even and odd points
+// alternate between two sets of sums.
 template <class S>
-__device__ __forceinline__ void sweeps22(const PlainParams& P, Factors& fc, int l1, int l2_0, int l2, int lane, S& SF,
-                                         S& SB)
-{
-    const CouplingParams& p = P.c;
-    const int T = l1, d = l2 - l1, js = l1 + l2;
-    const double r1 = l1 >= 2 ? (double)l1 * (l1 - 1) / ((double)(l1 + 1) * (l1 + 2)) : 0.0;
-    const double r2 = l2 >= 2 ? (double)l2 * (l2 - 1) / ((double)(l2 + 1) * (l2 + 2)) : 1.0;
-    double hf = sqrt(r1 / r2), hb = sqrt(r1 * r2), pf = 0.0, pb = 0.0;  // |m| = 2 > l1: h = 0 throughout
-    for (int e = lane; e < 96; e += 32) {
-        put_b(p, fc.F, 2 * l2_0 + e, l1);
-        put_b(p, fc.B, 2 * (l1 + l2_0) - 31 + e, l1);
-    }
-    auto forward = [&](auto even, int t) {
-        constexpr bool E = decltype(even)::value;
-        const int v = 2 * l2 + t, j = d + t;
-        const double tau = fc.A[t & (kPts - 1)] * fc.F[!E][(v >> 1) & (kHalf - 1)], q = tau * hf;
-        if constexpr (E) SF.even(P, tau, q, hf, (t >> 1) & 1, j);
-        else SF.odd(P, q, hf, j);
-        const double n = -fma(__ldg(p.half.W + j), q, pf);
-        pf = hf;
-        hf = n;
-    };
-    auto backward = [&](auto even, int t) {
-        constexpr bool E = decltype(even)::value;
-        const int v = 2 * js - t, j = js - t;
-        const double tau = fc.A[t & (kPts - 1)] * fc.B[!E][(v >> 1) & (kHalf - 1)], q = tau * hb;
-        if constexpr (E) SB.even(P, tau, q, hb, (t >> 1) & 1, j);
-        else SB.odd(P, q, hb, j);
-        const double n = -fma(__ldg(p.half.W + j), q, pb);
-        pb = hb;
-        hb = n;
-    };
-    const std::true_type even;
-    const std::false_type odd;
-    for (int t0 = 0; t0 <= T; t0 += kPts) {
-        __syncwarp();
-        const int ta = t0 + lane;
-        fc.A[lane] = tab_at(p.half.C, ta, p.half.top) * tab_at(p.half.C, 2 * l1 - ta, p.half.top);
-        if (t0 > 0) {  // 62 of the values the lanes meet were there before
-            put_b(p, fc.F, 2 * l2_0 + t0 + 62 + lane, l1);
-            put_b(p, fc.B, 2 * (l1 + l2_0) - t0 - 31 + lane, l1);
-        }
-        __syncwarp();
-        const int end = min(t0 + kPts, T);  // both sweeps run for t < T
-        int t = t0;
-        for (; t + 1 < end; t += 2) {
-            forward(even, t);
-            backward(even, t);
-            forward(odd, t + 1);
-            backward(odd, t + 1);
-        }
-        if (t < end) {
-            forward(even, t);
-            backward(even, t);
-        }
-        if (T < t0 + kPts) {  // the middle point, t = T
-            if (T & 1) forward(odd, T);
-            else forward(even, T);
-        }
-    }
-}
-
-// The (0 0 0) family alone: tau at every second point over the whole family, no recurrence.  Point
-// n has t = 2n; A and B by n = t / 2 and v / 2 = l2 + n.  Two sets of sums keep two chains.
-template <class S>
-__device__ __forceinline__ void points00(const PlainParams& P, Factors& fc, int l1, int l2_0, int l2, int lane, S& S0,
-                                         S& S1)
+__device__ __forceinline__ void sweep22(const PlainParams& P, Factors& fc, int l1, int l2_0, int l2, int n, int lane,
+                                        S& S0, S& S1)
 {
     const CouplingParams& p = P.c;
     const int d = l2 - l1;
-    put_b(p, fc.F, 2 * (l2_0 + lane), l1);
-    for (int n0 = 0; n0 <= l1; n0 += kPts) {
+    const double r1 = l1 >= 2 ? (double)l1 * (l1 - 1) / ((double)(l1 + 1) * (l1 + 2)) : 0.0;
+    const double r2 = l2 >= 2 ? (double)l2 * (l2 - 1) / ((double)(l2 + 1) * (l2 + 2)) : 1.0;
+    double h = sqrt(r1 / r2), hp = 0.0;  // |m| = 2 > l1: h = 0 throughout
+    for (int e = lane; e < 96; e += 32) put_b(p, fc, 2 * l2_0 + e, l1);
+    auto point = [&](auto even, int t, int neg, S& sum) {
+        constexpr bool E = decltype(even)::value;
+        const int j = d + t;
+        const double tau = fc.A[t & (kPts - 1)] * fc.B[!E][((2 * l2 + t) >> 1) & (kHalf - 1)], q = tau * h;
+        if constexpr (E) sum.even(P, tau, q, h, neg, j);
+        else sum.odd(P, q, h, j);
+        const double next = -fma(__ldg(p.half.W + j), q, hp);
+        hp = h;
+        h = next;
+    };
+    const std::true_type even;
+    const std::false_type odd;
+    for (int t0 = 0; t0 <= n; t0 += kPts) {
+        __syncwarp();
+        const int ta = t0 + lane;
+        fc.A[lane] = tab_at(p.half.C, ta, p.half.top) * tab_at(p.half.C, 2 * l1 - ta, p.half.top);
+        if (t0 > 0) put_b(p, fc, 2 * l2_0 + t0 + 62 + lane, l1);  // the other 62 were there before
+        __syncwarp();
+        const int end = min(t0 + kPts, n + 1);
+        int t = t0;
+        for (; t + 3 < end; t += 4) {
+            point(even, t, 0, S0);
+            point(odd, t + 1, 0, S0);
+            point(even, t + 2, 1, S1);
+            point(odd, t + 3, 0, S1);
+        }
+        if (t < end) point(even, t, 0, S0);
+        if (t + 1 < end) point(odd, t + 1, 0, S0);
+        if (t + 2 < end) point(even, t + 2, 1, S1);
+    }
+}
+
+// The (0 0 0) family alone: tau at every second point t <= n2, no recurrence.  Point n has t = 2n; A
+// and B by n = t / 2 and v / 2 = l2 + n.  Two sets of sums keep two chains.
+template <class S>
+__device__ __forceinline__ void points00(const PlainParams& P, Factors& fc, int l1, int l2_0, int l2, int n2, int lane,
+                                         S& S0, S& S1)
+{
+    const CouplingParams& p = P.c;
+    const int d = l2 - l1;
+    put_b(p, fc, 2 * (l2_0 + lane), l1);
+    for (int n0 = 0; 2 * n0 <= n2; n0 += kPts) {
         __syncwarp();
         const int ta = 2 * (n0 + lane);
         fc.A[lane] = tab_at(p.half.C, ta, p.half.top) * tab_at(p.half.C, 2 * l1 - ta, p.half.top);
-        put_b(p, fc.F, 2 * (l2_0 + n0 + 32 + lane), l1);
+        put_b(p, fc, 2 * (l2_0 + n0 + 32 + lane), l1);
         __syncwarp();
-        const int end = min(n0 + kPts, l1 + 1);
+        const int end = min(n0 + kPts, n2 / 2 + 1);
         int n = n0;
 #pragma unroll 2
         for (; n + 1 < end; n += 2) {
-            S0.even(P, fc.A[n - n0] * fc.F[0][(l2 + n) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n);
-            S1.even(P, fc.A[n + 1 - n0] * fc.F[0][(l2 + n + 1) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n + 2);
+            S0.even(P, fc.A[n - n0] * fc.B[0][(l2 + n) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n);
+            S1.even(P, fc.A[n + 1 - n0] * fc.B[0][(l2 + n + 1) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n + 2);
         }
-        if (n < end) S0.even(P, fc.A[n - n0] * fc.F[0][(l2 + n) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n);
+        if (n < end) S0.even(P, fc.A[n - n0] * fc.B[0][(l2 + n) & (kHalf - 1)], 0.0, 0.0, 0, d + 2 * n);
     }
 }
 
@@ -266,8 +247,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const Pla
         S a, b;
         a.zero();
         b.zero();
-        if constexpr (N02 + N22E + N22O + N22A > 0) sweeps22(P, sf[warp], l1, task.y, l2, lane, a, b);
-        else points00(P, sf[warp], l1, task.y, l2, lane, a, b);
+        // the points whose j a window reaches, for the warp's smallest d (the others' windows end in zeros)
+        const int n = min(p.nw - 1 - (max(task.y, l1) - l1), 2 * l1);
+        if constexpr (N02 + N22E + N22O + N22A > 0) sweep22(P, sf[warp], l1, task.y, l2, n, lane, a, b);
+        else points00(P, sf[warp], l1, task.y, l2, n, lane, a, b);
         a.give(P, b, l1, Xi);
     }
     write_tile<kMaxWin>(p, l1, task.y, active, Xi, &stage[0][0], kMaxWin * 32, rows, warp, lane);
