@@ -186,7 +186,7 @@ static_assert(((S_PPMM2 >> 8) & 0xffu) == S_PPMM && ((S_PPMM2 >> 4) & 0xfu) == W
 constexpr uint32_t S_TETE = W02 | (W00 << 4) | (W02 << 8) | (W02 << 12) | (W02 << 16);
 
 struct Sweep {
-    ff f2, f2o;   // 22 family at the current point and at the previous one
+    ff f2, f2o;   // (-1)^t times the 22 family at the current point and at the previous one
     ff f0;        // 00 family at the last even point
     float w;      // ws (2j + 1) at the current point, ws = 4 or 1 (exact in FP32)
 };
@@ -267,13 +267,15 @@ __device__ __forceinline__ void sweep_acc(const WinCfg<NWIN>& p, const Sweep& s,
 // float-float P, 1/sqrt(P) and a(j).  G'(t-1)/G'(t) = G(t)/G(t+1), built from
 // the same two products (each commutative), so one G table serves both sweeps.
 constexpr int kFEnt = kChunk / 2 + 32;  // F entries per parity of u (or v)
+// The F entries hold -rho, so that the step g(t+1) = r w g(t) + (-rho) g(t-1) of g(t) = (-1)^t f(t) and
+// the (0 0 0) step -rho f take no negation.
 struct __align__(16) ffpair {
     ff rho, r;  // loaded together (one 16-byte shared load)
 };
 struct CoefTab {
     ffpair g[kChunk];       // sqrt(G(t)/G(t+1)), 1/sqrt(G(t+1)); both sweeps
-    ffpair fF[2][kFEnt];    // forward: sqrt(F(u)/F(u+1)), 1/sqrt(F(u+1))
-    ffpair fB[2][kFEnt];    // backward: sqrt(F'(v+1)/F'(v)), 1/sqrt(F'(v))
+    ffpair fF[2][kFEnt];    // forward: -sqrt(F(u)/F(u+1)), 1/sqrt(F(u+1))
+    ffpair fB[2][kFEnt];    // backward: -sqrt(F'(v+1)/F'(v)), 1/sqrt(F'(v))
 };
 
 // rho = sqrt(X / Y) for X >= 0, Y > 0 (float-float); 0 for X = 0
@@ -297,7 +299,7 @@ __device__ __forceinline__ void f_fwd(CoefTab& tb, int e, int t0, int l1, int l2
     const ff Y = two_prod((float)(2 * d0 + 1) + u, (float)(2 * l2_0 + 2) + u);
     ff a, b;
     sqrt_ratio(X, Y, a, b);
-    tb.fF[e & 1][e >> 1] = ffpair{a, b};
+    tb.fF[e & 1][e >> 1] = ffpair{ff_neg(a), b};
 }
 __device__ __forceinline__ void f_bwd(CoefTab& tb, int e, int t0, int l1, int l2_0)
 {
@@ -307,7 +309,7 @@ __device__ __forceinline__ void f_bwd(CoefTab& tb, int e, int t0, int l1, int l2
     if (2 * l2_0 + v > 0)
         sqrt_ratio(two_prod((float)(2 * l2_0 + 1) + fv, (float)(2 * l1 + 2 * l2_0 + 2) + fv),
                    two_prod((float)(2 * l2_0) + fv, (float)(2 * l1 + 2 * l2_0 + 1) + fv), a, b);
-    tb.fB[e & 1][e >> 1] = ffpair{a, b};
+    tb.fB[e & 1][e >> 1] = ffpair{ff_neg(a), b};
 }
 // Without the (2 -2 0) family only the odd steps of the (0 0 0) recurrence use
 // the tables, and only rho: odd e forward (fF[1]) and even e backward (fB[0]).
@@ -326,7 +328,7 @@ __device__ __forceinline__ void f_rho_odd_steps(CoefTab& tb, int e, int t0, int 
     const float y2 = fwd ? (float)(2 * l2_0 + 2) + u : (float)(2 * l1 + 2 * l2_0 + 1) + fv;
     ff rho = sqrt_ratio_rho(two_prod(x1, x2), two_prod(y1, y2));
     if (!fwd && 2 * l2_0 + v <= 0) rho = ff_make(0.0f);
-    (fwd ? tb.fF[1][e >> 1] : tb.fB[0][e >> 1]).rho = rho;
+    (fwd ? tb.fF[1][e >> 1] : tb.fB[0][e >> 1]).rho = ff_neg(rho);
 }
 
 // The F entries of a task's first chunk (t0 = 0), formed in full.
@@ -388,7 +390,9 @@ __device__ __forceinline__ void build_tables(CoefTab& tb, int t0, int T, int l1,
     }
 }
 
-// One table-driven step: f(next) = -(4 (2j+1) f(cur) r + rho f(prev)).  With
+// One table-driven step: g(next) = 4 (2j+1) r g(cur) - rho g(prev) for g(t) = (-1)^t f(t), with -rho
+// from the tables: no negations (measured against f itself, same bits: all spin cases at lmax 3071
+// 18.80 -> 18.47 ms, TT at lmax 767 109.3 -> 107.7 us).  With
 // WS4 the sweep carries w = 4 (2j+1) and the step saves the multiply by 4.
 // Both forms give the same bits (4 (2j+1) is exact); which one a slot list
 // uses is a measured choice: the compiler schedules the all-spins list
@@ -397,16 +401,18 @@ __device__ __forceinline__ void build_tables(CoefTab& tb, int t0, int T, int l1,
 template <int NWIN, uint32_t SPEC>
 constexpr bool weight_times4() { return !(NWIN == 4 && SPEC == S_MCM4); }
 template <bool N00, bool N22, bool ODD_STEP, bool WS4>
-__device__ __forceinline__ void tab_step(Sweep& s, ff rho, ff r, float dw)
+__device__ __forceinline__ void tab_step(Sweep& s, const ffpair& g, const ffpair& f, float dw)
 {
     if (N22) {
-        ff u = ff_mul_raw(ff_mulf_raw(s.f2, WS4 ? s.w : 4.0f * s.w), r);
-        ff v = ff_mul_raw(rho, s.f2o);
-        ff nf = ff_neg(ff_add_raw(u, v));
+        const ff rho = ff_mul_raw(g.rho, f.rho), r = ff_mul_raw(g.r, f.r);
+        const ff u = ff_mul_raw(ff_mulf_raw(s.f2, WS4 ? s.w : 4.0f * s.w), r);
+        const ff n = ff_add_raw(u, ff_mul_raw(rho, s.f2o));
         s.f2o = s.f2;
-        s.f2 = nf;
+        s.f2 = n;
+        if (N00 && ODD_STEP) s.f0 = ff_mul_raw(rho, s.f0);
+    } else if (N00 && ODD_STEP) {
+        s.f0 = ff_mul_raw(ff_mul_raw(g.rho, f.rho), s.f0);
     }
-    if (N00 && ODD_STEP) s.f0 = ff_neg(ff_mul_raw(rho, s.f0));
     s.w += dw;
 }
 
@@ -414,10 +420,7 @@ template <bool N00, bool N22, bool ODD_STEP, bool WS4>
 __device__ __forceinline__ void tab_fwd(Sweep& s, const CoefTab& tb, int st, int lane)
 {
     const int e = lane + (st >> 1);  // (u - t0) / 2; u - t0 = 2 lane + st has the parity of the step
-    const ffpair g = tb.g[st], f = tb.fF[ODD_STEP][e];
-    ff rho = ff_mul_raw(g.rho, f.rho);
-    ff r = ff_mul_raw(g.r, f.r);
-    tab_step<N00, N22, ODD_STEP, WS4>(s, rho, r, WS4 ? 8.0f : 2.0f);
+    tab_step<N00, N22, ODD_STEP, WS4>(s, tb.g[st], tb.fF[ODD_STEP][e], WS4 ? 8.0f : 2.0f);
 }
 
 template <bool N00, bool N22, bool ODD_STEP, bool WS4>
@@ -425,10 +428,7 @@ __device__ __forceinline__ void tab_bwd(Sweep& s, const CoefTab& tb, int st, int
 {
     // v - (-t0 - 31) = 2 lane - st + 31: odd for even steps, half of it lane + 15 - st / 2
     const int e = lane + (kChunk / 2 - 1) - (st >> 1);
-    const ffpair g = tb.g[st], f = tb.fB[!ODD_STEP][e];
-    ff rho = ff_mul_raw(g.rho, f.rho);
-    ff r = ff_mul_raw(g.r, f.r);
-    tab_step<N00, N22, ODD_STEP, WS4>(s, rho, r, WS4 ? -8.0f : -2.0f);
+    tab_step<N00, N22, ODD_STEP, WS4>(s, tb.g[st], tb.fB[!ODD_STEP][e], WS4 ? -8.0f : -2.0f);
 }
 
 // The Xi of pair (l1, l2_0 + lane) into Xi[]; returns whether the lane holds a
@@ -559,9 +559,16 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
     }
     double FN0 = SFN0.get(), FN2 = SFN2.get(), BN0 = SBN0.get(), BN2 = SBN2.get();
 
-    // last forward point t = T (j = jm), in FP64; its parity is that of T
+    // last forward point t = T (j = jm), in FP64; its parity is that of T.  The sweeps hold (-1)^t f.
     const int jm = jmin + T;
     const bool evenT = (T & 1) == 0;
+    if (evenT) {
+        F.f2o = ff_neg(F.f2o);
+        B.f2o = ff_neg(B.f2o);
+    } else {
+        F.f2 = ff_neg(F.f2);
+        B.f2 = ff_neg(B.f2);
+    }
     {
         double g2d = ff_to_double(F.f2), g0d = (N00 && evenT) ? ff_to_double(F.f0) : 0.0;
         double x22 = g2d * g2d, x00 = g0d * g0d, x02 = g0d * g2d, w = 2.0 * jm + 1.0;
