@@ -58,7 +58,7 @@ struct ps_ctx {
     size_t alm_cap = 0;
     double* d_part = nullptr;  // alm2cl partial sums
     size_t part_cap = 0;
-    double* d_qp = nullptr;  // chosen QuickPol scratch: W as floats and its exponent
+    double* d_qp = nullptr;  // QuickPol scratch: tables over l' (plain), W as floats and its exponent (chosen)
     size_t qp_cap = 0;
     // covariance sets: the windows of the tensor-core launches (padded, split) and their Xi
     double* d_cwin = nullptr;
@@ -1568,8 +1568,12 @@ static int quickpol_run(ps_ctx* c, const double* dW, long long nW, int lmax, int
                                           (float*)c->d_qp, (int*)(c->d_qp + nf), c->stream));
         c->launches += 2;
     } else {
-        PS_CUDA(c, ps::launch_quickpol(dW, nW, lmax, bl, bu, nu1, nu2, s1, s2, c->d_out, (long long)n, c->stream));
-        c->launches++;
+        ps::HalfTable half;
+        int st = ensure_half(c, lmax, &half);
+        if (st || (st = ensure(c, &c->d_qp, &c->qp_cap, ps::quickpol_scratch(lmax)))) return st;
+        PS_CUDA(c, ps::launch_quickpol(dW, nW, lmax, bl, bu, nu1, nu2, s1, s2, c->d_out, (long long)n, half, c->d_qp,
+                                       c->stream));
+        c->launches += 2;
     }
     return PS_OK;
 }

@@ -100,8 +100,10 @@ cudaError_t launch_split_windows(int2* dst, const double* wW, int wlen, cudaStre
 constexpr int kZeroExp = -100000;
 cudaError_t launch_fma_probe(int fp64, double* sink, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_transpose(double* dst, const double* src, int n, cudaStream_t s);
+// scratch: quickpol_scratch(lmax) doubles; half: for lmax
+size_t quickpol_scratch(int lmax);
 cudaError_t launch_quickpol(const double* W, long long nW, int lmax, int bl, int bu, int nu1, int nu2, int s1, int s2,
-                            double* Xi, long long ldx, cudaStream_t s);
+                            double* Xi, long long ldx, const HalfTable& half, double* scratch, cudaStream_t s);
 // The chosen-arithmetic QuickPol Xi (ps_quickpol_ff.cu); wf: nW floats, e: one int of scratch.
 cudaError_t launch_quickpol_ff(const double* W, long long nW, int lmax, int bl, int bu, int nu1, int nu2, int s1,
                                int s2, double* Xi, long long ldx, float* wf, int* e, cudaStream_t s);

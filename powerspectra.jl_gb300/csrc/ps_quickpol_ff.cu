@@ -125,6 +125,9 @@ __global__ void __launch_bounds__(1024) k_quickpol_stage(const double* __restric
     if (threadIdx.x == 0) *E_out = E;
 }
 
+// SAME: equal spins (s1 = s2, nu1 = nu2) give equal families, and one is run (the same bits; measured,
+// 1000 x 1000 with band (100, 100), nu = 0, s = 2, as a whole host call: 1.63 -> 0.98 ms).
+template <bool SAME>
 __global__ void __launch_bounds__(128, 5) k_quickpol_ff(const float* __restrict__ Wf, const int* __restrict__ E_in,
                                                      long long nW, int lmax, int bl, int bu, int nu1, int nu2, int s1,
                                                      int s2, double* Xi, long long ldx)
@@ -182,10 +185,10 @@ __global__ void __launch_bounds__(128, 5) k_quickpol_ff(const float* __restrict_
             if (it < nfwd) {
                 const int j = jlo + it;
                 if (fwd0 && j == F[0].jmin) fc0 = one;
-                if (fwd1 && j == F[1].jmin) fc1 = one;
-                const float g0 = ff_round(fc0), g1 = ff_round(fc1), w = __fmaf_rn(2.0f, jf, 1.0f);
+                if (!SAME && fwd1 && j == F[1].jmin) fc1 = one;
+                const float g0 = ff_round(fc0), g1 = SAME ? g0 : ff_round(fc1), w = __fmaf_rn(2.0f, jf, 1.0f);
                 nf0 = __fmaf_rn(w, __fmul_rn(g0, g0), nf0);
-                nf1 = __fmaf_rn(w, __fmul_rn(g1, g1), nf1);
+                if (!SAME) nf1 = __fmaf_rn(w, __fmul_rn(g1, g1), nf1);
                 if (j < nW) sf = __fmaf_rn(__fmul_rn(__ldg(Wf + j), g0), g1, sf);
                 const QShared qn = qp_shared(jf + 1.0f, adf, spf);
                 const ff jsq = two_prod(jf, jf);
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(128, 5) k_quickpol_ff(const float* __restrict_
                     fp0 = fc0;
                     fc0 = n;
                 }
-                if (fwd1 && j >= F[1].jmin) {
+                if (!SAME && fwd1 && j >= F[1].jmin) {
                     const ff n = qp_fwd(jf, F[1], qc, qn, jsq, fc1, fp1, af1);
                     fp1 = fc1;
                     fc1 = n;
@@ -204,10 +207,10 @@ __global__ void __launch_bounds__(128, 5) k_quickpol_ff(const float* __restrict_
             if (it < nbwd) {
                 const int j = jmax - it;
                 const bool in0 = j >= (fwd0 ? jm + 1 : F[0].jmin), in1 = j >= (fwd1 ? jm + 1 : F[1].jmin);
-                const float v0 = in0 ? ff_round(hc0) : 0.0f, v1 = in1 ? ff_round(hc1) : 0.0f;
+                const float v0 = in0 ? ff_round(hc0) : 0.0f, v1 = SAME ? v0 : (in1 ? ff_round(hc1) : 0.0f);
                 const float w = __fmaf_rn(2.0f, jbf, 1.0f);
                 nb0 = __fmaf_rn(w, __fmul_rn(v0, v0), nb0);
-                nb1 = __fmaf_rn(w, __fmul_rn(v1, v1), nb1);
+                if (!SAME) nb1 = __fmaf_rn(w, __fmul_rn(v1, v1), nb1);
                 if (j < nW) sb = __fmaf_rn(__fmul_rn(__ldg(Wf + j), v0), v1, sb);
                 const QShared qb = qp_shared(jbf, adf, spf);
                 const ff j1sq = two_prod(jbf + 1.0f, jbf + 1.0f);
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(128, 5) k_quickpol_ff(const float* __restrict_
                     hc0 = n;
                     if (j == jm + 1) hm0_0 = hc0;
                 }
-                if (in1 && j > F[1].jmin) {
+                if (!SAME && in1 && j > F[1].jmin) {
                     if (j == jm + 1) hm1_1 = hc1;
                     const ff n = qp_bwd(jbf, F[1], qb, j1sq, hc1, hn1, ab1);
                     hn1 = hc1;
@@ -238,8 +241,8 @@ __global__ void __launch_bounds__(128, 5) k_quickpol_ff(const float* __restrict_
         const double a0 = ff_to_double(hm0_0), b0 = ff_to_double(hm1_0), a1 = ff_to_double(hm0_1),
                      b1 = ff_to_double(hm1_1);
         const double lam0 = fwd0 ? (p0 * a0 + c0 * b0) / (a0 * a0 + b0 * b0) : 1.0;
-        const double lam1 = fwd1 ? (p1 * a1 + c1 * b1) / (a1 * a1 + b1 * b1) : 1.0;
-        const double N0 = fma(lam0 * lam0, NB0, NF0), N1 = fma(lam1 * lam1, NB1, NF1);
+        const double lam1 = SAME ? lam0 : (fwd1 ? (p1 * a1 + c1 * b1) / (a1 * a1 + b1 * b1) : 1.0);
+        const double N0 = fma(lam0 * lam0, NB0, NF0), N1 = SAME ? N0 : fma(lam1 * lam1, NB1, NF1);
         const double cs0 = ((l1 - l2 - F[0].m3) & 1) ? -1.0 : 1.0, cs1 = ((l1 - l2 - F[1].m3) & 1) ? -1.0 : 1.0;
         const double sg0 = (lam0 < 0.0) ? -cs0 : cs0, sg1 = (lam1 < 0.0) ? -cs1 : cs1;
         xi = ldexp(fma(lam0 * lam1, SB, SF) * sg0 * sg1 * rsqrt(N0 * N1), *E_in);
@@ -262,7 +265,11 @@ cudaError_t launch_quickpol_ff(const double* W, long long nW, int lmax, int bl, 
     bu = bu < lmax ? bu : lmax;
     const int width = bl + bu + 1;
     const long long total = (long long)(lmax - 1) * width;  // < 2^31 for lmax <= 16383
-    k_quickpol_ff<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(wf, e, nW, lmax, bl, bu, nu1, nu2, s1, s2, Xi, ldx);
+    const unsigned blocks = (unsigned)((total + 127) / 128);
+    if (s1 == s2 && nu1 == nu2)
+        k_quickpol_ff<true><<<blocks, 128, 0, st>>>(wf, e, nW, lmax, bl, bu, nu1, nu2, s1, s2, Xi, ldx);
+    else
+        k_quickpol_ff<false><<<blocks, 128, 0, st>>>(wf, e, nW, lmax, bl, bu, nu1, nu2, s1, s2, Xi, ldx);
     return cudaGetLastError();
 }
 
