@@ -144,13 +144,14 @@ __device__ __forceinline__ int b_off(int n, int k) { return (n >> 3) * 256 + (k 
 
 __device__ __forceinline__ uint32_t bf2_bits(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
-// Three-part BF16 split of two values (low half: a, high half: b).
+// Three-part BF16 split of two values (low half: a, high half: b).  The parts are widened by shift and
+// mask: the conversion functions cost more (7 TT and 13 ++/-- windows at lmax 8191: 454.3 -> 444.5 ms).
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&w)[kPlanes])
 {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    const float ra = a - __low2float(h), rb = b - __high2float(h);
+    const float ra = a - __uint_as_float(bf2_bits(h) << 16), rb = b - __uint_as_float(bf2_bits(h) & 0xffff0000u);
     const __nv_bfloat162 m = __floats2bfloat162_rn(ra, rb);
-    const float qa = ra - __low2float(m), qb = rb - __high2float(m);
+    const float qa = ra - __uint_as_float(bf2_bits(m) << 16), qb = rb - __uint_as_float(bf2_bits(m) & 0xffff0000u);
     const __nv_bfloat162 l = __floats2bfloat162_rn(qa, qb);
     w[0] = bf2_bits(h);
     w[1] = bf2_bits(m);
@@ -353,6 +354,36 @@ __device__ __forceinline__ RingIdx ring_idx(int tf_even, int tb_even, int l2)
                    kGuard + ring_slot(u0 - 1)};
 }
 // forward step of parity p in pair k: g[t] and f[2 l2 + t]
+// The same entries as addresses, for the loop of a steady block: they move with the steps, which spares
+// it the index arithmetic (with moving indices in the (0 0 0) loop, the 20 matrices at lmax 8191: 440.5 ->
+// 426.1 ms; in the checked loop the addresses cost registers that the 16-column kernel does not have).
+struct RingPtr {
+    const ffpair *g, *f, *gb, *fb0, *fb1;
+    __device__ __forceinline__ void next(int pairs)
+    {
+        g += pairs;
+        f += pairs;
+        gb += pairs;
+        fb0 -= pairs;
+        fb1 -= pairs;
+    }
+};
+__device__ __forceinline__ RingPtr ring_ptr(const CoefRing& R, const RingIdx& q)
+{
+    return RingPtr{R.g[0] + q.g, R.f[0] + q.f, R.g[0] + q.gb, R.fb[0] + q.fb0, R.fb[1] + q.fb1};
+}
+constexpr int kRow = kRing + kGuard;  // entries from the table of the even values to that of the odd ones
+__device__ __forceinline__ void fwd_step(Sweep22& S, const RingPtr& r, int p, int k)
+{
+    const ffpair g = r.g[p * kRow + k], f = r.f[p * kRow + k];
+    step22(S, ff_mul_raw(g.rho, f.rho), ff_mul_raw(g.r, f.r), 8.0f);
+}
+__device__ __forceinline__ void bwd_step(Sweep22& S, const RingPtr& r, int p, int k)
+{
+    const ffpair g = r.gb[p * kRow + k], f = (p ? r.fb1 : r.fb0)[-k];
+    step22(S, ff_mul_raw(g.rho, f.rho), ff_mul_raw(g.r, f.r), -8.0f);
+}
+// forward step of parity p in pair k: g[t] and f[2 l2 + t]
 __device__ __forceinline__ void fwd_step(Sweep22& S, const CoefRing& R, int p, const RingIdx& q, int k)
 {
     const ffpair g = R.g[p][q.g + k], f = R.f[p][q.f + k];
@@ -369,7 +400,7 @@ __device__ __forceinline__ void bwd_step(Sweep22& S, const CoefRing& R, int p, c
 // The (0 0 0) family vanishes where l1 + l2 + l3 is odd, so its sweeps step two points at a
 // time: f(j + 2) = -rho f(j) with rho the product of the odd-t entries of the (2 -2 0) step
 // (forward g[t] f[2 l2 + t], backward g[t] fb[2 l2 - t], t = 2n + 1 at step n), whose rho alone
-// is needed.  Each warp keeps them as rings of 64 odd values; a 32-step block reads 63
+// is needed, negative in f and fb.  Each warp keeps them as rings of 64 odd values; a 32-step block reads 63
 // consecutive ones of each table, 32 of them new, built at its start.
 constexpr int kGuard00 = kBlk;  // a block's 32 steps read 32 consecutive slots of each table
 struct __align__(16) Ring00 {
@@ -390,13 +421,13 @@ __device__ __forceinline__ void ring00_gf(Ring00& R, int x, bool isf, int l1)
 {
     const float a0 = (float)(isf ? x - 2 * l1 : x), b0 = (float)(isf ? x + 1 : 2 * l1 + 1 - x);
     const ff rho = rho_entry(two_prod(a0, b0), two_prod(a0 + 1.0f, isf ? b0 + 1.0f : b0 - 1.0f));
-    put_up<kGuard00>(isf ? R.f : R.g, ring_slot(x), rho);
+    put_up<kGuard00>(isf ? R.f : R.g, ring_slot(x), isf ? ff_neg(rho) : rho);
 }
 // One entry of fb at odd u: sqrt(Fb(u + 1) / Fb(u)), Fb(u) = u (2 l1 + 1 + u)
 __device__ __forceinline__ void ring00_fb(Ring00& R, int u, int l1)
 {
     const float a0 = (float)u, b0 = (float)(2 * l1 + 1 + u);
-    put_down<kGuard00>(R.fb, ring_slot(u), rho_entry(two_prod(a0 + 1.0f, b0 + 1.0f), two_prod(a0, b0)));
+    put_down<kGuard00>(R.fb, ring_slot(u), ff_neg(rho_entry(two_prod(a0 + 1.0f, b0 + 1.0f), two_prod(a0, b0))));
 }
 __device__ __forceinline__ void build_rings00_first(Ring00& R, int tb, int w, int l1, int c0, int lane)
 {
@@ -420,6 +451,13 @@ __device__ __forceinline__ void build_rings00_next(Ring00& R, int tb, int w, int
 // u = 2 l2 - t (slot l2 - n - 1).  Step j of the block reads g and f at + j and fb at - j.
 struct RingIdx00 {
     int g, f, gb, fb;
+    __device__ __forceinline__ void next(int steps)
+    {
+        g += steps;
+        f += steps;
+        gb += steps;
+        fb -= steps;
+    }
 };
 __device__ __forceinline__ RingIdx00 ring00_idx(int nf, int nb, int l2)
 {
@@ -428,11 +466,11 @@ __device__ __forceinline__ RingIdx00 ring00_idx(int nf, int nb, int l2)
 }
 __device__ __forceinline__ void fwd_step00c(ff& f, const Ring00& R, const RingIdx00& q, int j)
 {
-    f = ff_neg(ff_mul_raw(ff_mul_raw(R.g[q.g + j], R.f[q.f + j]), f));
+    f = ff_mul_raw(ff_mul_raw(R.g[q.g + j], R.f[q.f + j]), f);
 }
 __device__ __forceinline__ void bwd_step00c(ff& f, const Ring00& R, const RingIdx00& q, int j)
 {
-    f = ff_neg(ff_mul_raw(ff_mul_raw(R.g[q.gb + j], R.fb[q.fb - j]), f));
+    f = ff_mul_raw(ff_mul_raw(R.g[q.gb + j], R.fb[q.fb - j]), f);
 }
 
 // sqrt(X / Y) for the last forward points (X, Y up to 2^64: the scaling keeps X Y in range)
@@ -506,20 +544,21 @@ __device__ __forceinline__ float sq(const ff& f)
 // most four blocks between renormalisations: at most four roundings of 2^-24 relative to those
 // blocks' sum, against one rounding of the tensor core's truncating accumulation per block.
 template <int R, int NC>
-__device__ __forceinline__ void renorm(ff (&t)[NC], int ncols)
+__device__ __forceinline__ void renorm(ff (&t)[NC])
 {
 #pragma unroll
-    for (int n = R; n < NC; n += 4)
-        if (n < ncols) t[n] = two_sum(t[n].h, t[n].l);
+    for (int n = R; n < NC; n += 4) t[n] = two_sum(t[n].h, t[n].l);
 }
 
 template <bool F00>
 using RingT = typename std::conditional<F00, Ring00, CoefRing>::type;
 
 // NC: columns folded into the totals (8 or 16; at least nslot + 1).  STAGE: the outputs are
-// in host memory (MmaParams::stage_rows).
+// in host memory (MmaParams::stage_rows).  The register bounds are measured choices (four blocks reside
+// per SM whatever they say): asked for four blocks the (0 0 0) kernels take more registers (7 TT windows at
+// lmax 6143 41.5 -> 40.9 ms), and the (2 -2 0) one of 16 columns spills (143 -> 146 ms for 13 windows).
 template <bool F00, int NC, bool STAGE>
-__global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
+__global__ void __launch_bounds__(128, F00 ? 4 : (NC == 8 ? 5 : 0)) k_coupling_mma(const MmaParams p)
 {
     __shared__ Smem sm;
     extern __shared__ __align__(16) unsigned char dyn[];  // the warps' coefficient rings
@@ -634,7 +673,9 @@ __global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
 #pragma unroll
                 for (int n = 0; n < NC; ++n) dv[n] = __fadd_rn(dv[n], dv[n + 8]);
             }
-            // D in units of 2^(block exponent), brought to the running exponent (an exact power of two)
+            // D in units of 2^(block exponent), brought to the running exponent (an exact power of two).
+            // Columns not in use hold zeros: folding them costs less than testing for them (445.4 -> 440.5
+            // ms at lmax 8191).
             const float4* ds = reinterpret_cast<const float4*>(&sm.dscale[q % 3][s][0]);
 #pragma unroll
             for (int v = 0; v < NC / 4; ++v) {
@@ -642,13 +683,13 @@ __global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
                 const float dw[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (4 * v + j < ncols) tot[s][4 * v + j].l = __fmaf_rn(dv[4 * v + j], dw[j], tot[s][4 * v + j].l);
+                    tot[s][4 * v + j].l = __fmaf_rn(dv[4 * v + j], dw[j], tot[s][4 * v + j].l);
             }
             switch (q & 3) {
-                case 0: renorm<0>(tot[s], ncols); break;
-                case 1: renorm<1>(tot[s], ncols); break;
-                case 2: renorm<2>(tot[s], ncols); break;
-                default: renorm<3>(tot[s], ncols); break;
+                case 0: renorm<0>(tot[s]); break;
+                case 1: renorm<1>(tot[s]); break;
+                case 2: renorm<2>(tot[s]); break;
+                default: renorm<3>(tot[s]); break;
             }
         }
     };
@@ -680,6 +721,8 @@ __global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
         RingIdx ix22;
         if constexpr (F00) ix00 = ring00_idx(tb + fofs, tb + bofs, l2);
         else ix22 = ring_idx(tb + fofs, tb + bofs, l2);
+        RingPtr rp;
+        if constexpr (!F00) rp = ring_ptr(R, ix22);  // the steady loop's
         // One step pair of the block: the steps of both sweeps, and x of both as split words.  In
         // a block whose steps all lie in the steady state, every lane that runs is inside both
         // sweeps, so both steps run unconditionally (their dependency chains interleave).  Lanes
@@ -719,8 +762,8 @@ __global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
                     if (steady) {
                         xf[e] = sq(F.f);
                         xb[e] = sq(B.f);
-                        fwd_step(F, R, e, ix22, k);
-                        bwd_step(B, R, e, ix22, k);
+                        fwd_step(F, rp, e, k);
+                        bwd_step(B, rp, e, k);
                     } else {
                         xf[e] = 0.0f;
                         xb[e] = 0.0f;
@@ -740,12 +783,13 @@ __global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
         };
         // Two step pairs (s2 .. s2 + 3), then their x into tensor memory: step pairs k and k + 1
         // of the block in two consecutive columns of each sweep and plane, one store each.
+        uint32_t col = 0;  // step pairs of the block before the current ones
         auto two_pairs = [&](int s2, bool steady) {
             uint32_t wf0[kPlanes], wb0[kPlanes], wf1[kPlanes], wb1[kPlanes];
             pair(s2, steady, wf0, wb0);
             pair(s2 + 2, steady, wf1, wb1);
             __syncwarp();  // the stores below are warp-collective (.sync.aligned)
-            const uint32_t k = (uint32_t)(s2 >> 1);  // the first step pair
+            const uint32_t k = (uint32_t)(s2 >> 1) + col;  // the first step pair
 #pragma unroll
             for (int pl = 0; pl < kPlanes; ++pl) {
                 umma::st_x2(tlane + a_col(0, pl) + k, wf0[pl], wf1[pl]);
@@ -756,7 +800,12 @@ __global__ void __launch_bounds__(128) k_coupling_mma(const MmaParams p)
         const bool steady = F00 ? (tb >= 34 && t1 <= steady00) : (tb >= kSteady && t1 <= r0 + kLead - 1);
         if (steady) {
 #pragma unroll 1
-            for (int s2 = 0; s2 < kBlk; s2 += 4) two_pairs(s2, true);
+            for (int s2 = 0; s2 < kBlk; s2 += 4) {  // four steps from entries that move along
+                two_pairs(0, true);
+                col += 2;
+                if constexpr (F00) ix00.next(4);
+                else rp.next(2);
+            }
         } else {
 #pragma unroll 1
             for (int s2 = 0; s2 < kBlk; s2 += 4) two_pairs(s2, false);
