@@ -1,56 +1,68 @@
 // ps_cov_epilogue.cuh -- per-pair combination of the Xi_k into a covariance
-// element, one formula per loop_cov*! kernel of the reference.  The
-// expressions keep the reference's operand order (left-associative products)
-// so the FP64 results agree with it to rounding.
+// element, one formula per loop_cov*! kernel of the reference.
 #pragma once
 
 #include "ps_internal.cuh"
 
 namespace ps {
 
-// X[k] are the Xi of windows W1..Wk (already divided by 4pi); a = l1, b = l2.
-__device__ __forceinline__ double cov_combine(int kind, const double* const* S, const double* const* R,
-                                              const double* X, int a, int b)
+// X[k] are the Xi of windows W1..Wk (already divided by 4pi), Sa, Sb, Ra, Rb the spectra and noise
+// ratios at l1 = a and l2 = b, g[i] = sqrt(Sa[i] Sb[i]) for the spectra that need it (cov_roots).  The
+// reference's sqrt of a product of two such pairs is the product of their roots here (equal to rounding;
+// a pair of unequal signs makes the element NaN either way, through the terms with its own root).
+__device__ __forceinline__ double cov_form(int kind, const double* Sa, const double* Sb, const double* g,
+                                           const double* Ra, const double* Rb, const double* X)
 {
     switch (kind) {
     case PS_COV_TTTT:
-    case PS_COV_EEEE: {  // src/covariance.jl:110-118 (TTTT), :171-179 (EEEE)
-        const double *ip = S[0], *jq = S[1], *iq = S[2], *jp = S[3];
-        const double *rip = R[0], *rjq = R[1], *riq = R[2], *rjp = R[3];
-        return sqrt(ip[a] * ip[b] * jq[a] * jq[b]) * X[0] + sqrt(iq[a] * iq[b] * jp[a] * jp[b]) * X[1] +
-               sqrt(ip[a] * ip[b]) * X[2] * rjq[a] * rjq[b] + sqrt(jq[a] * jq[b]) * X[3] * rip[a] * rip[b] +
-               sqrt(iq[a] * iq[b]) * X[4] * rjp[a] * rjp[b] + sqrt(jp[a] * jp[b]) * X[5] * riq[a] * riq[b] +
-               X[6] * rip[a] * rjq[a] * rip[b] * rjq[b] + X[7] * riq[a] * rjp[a] * riq[b] * rjp[b];
+    case PS_COV_EEEE: {  // src/covariance.jl:110-118 (TTTT), :171-179 (EEEE); ip, jq, iq, jp
+        const double ip = Ra[0] * Rb[0], jq = Ra[1] * Rb[1], iq = Ra[2] * Rb[2], jp = Ra[3] * Rb[3];
+        return g[0] * g[1] * X[0] + g[2] * g[3] * X[1] + g[0] * X[2] * jq + g[1] * X[3] * ip + g[2] * X[4] * jp +
+               g[3] * X[5] * iq + X[6] * (ip * jq) + X[7] * (iq * jp);
     }
-    case PS_COV_TTTE: {  // src/covariance.jl:225-230
-        const double *TTip = S[0], *TTjp = S[1], *TEiq = S[2], *TEjq = S[3];
-        const double *rip = R[0], *rjp = R[1];
-        return (sqrt(TTip[a] * TTip[b]) * (TEjq[a] + TEjq[b]) * X[0] +
-                sqrt(TTjp[a] * TTjp[b]) * (TEiq[a] + TEiq[b]) * X[1] + (TEjq[a] + TEjq[b]) * X[2] * rip[a] * rip[b] +
-                (TEiq[a] + TEiq[b]) * X[3] * rjp[a] * rjp[b]) /
-               2;
-    }
-    case PS_COV_TETE: {  // src/covariance.jl:292-297
-        const double *TTip = S[0], *EEjq = S[1], *TEiq = S[2], *TEjp = S[3];
-        const double *rT = R[0], *rP = R[1];
-        return sqrt(TTip[a] * TTip[b] * EEjq[a] * EEjq[b]) * X[0] +
-               0.5 * (TEiq[a] * TEjp[b] + TEjp[a] * TEiq[b]) * X[1] + sqrt(TTip[a] * TTip[b]) * X[2] * rP[a] * rP[b] +
-               sqrt(EEjq[a] * EEjq[b]) * X[3] * rT[a] * rT[b] + X[4] * rT[a] * rT[b] * rP[a] * rP[b];
+    case PS_COV_TTTE:  // src/covariance.jl:225-230; TTip, TTjp, TEiq, TEjq; r_ip, r_jp
+        return (g[0] * (Sa[3] + Sb[3]) * X[0] + g[1] * (Sa[2] + Sb[2]) * X[1] + (Sa[3] + Sb[3]) * X[2] * Ra[0] * Rb[0] +
+                (Sa[2] + Sb[2]) * X[3] * Ra[1] * Rb[1]) / 2;
+    case PS_COV_TETE: {  // src/covariance.jl:292-297; TTip, EEjq, TEiq, TEjp; r_TT, r_PP
+        const double rT = Ra[0] * Rb[0], rP = Ra[1] * Rb[1];
+        return g[0] * g[1] * X[0] + 0.5 * (Sa[2] * Sb[3] + Sa[3] * Sb[2]) * X[1] + g[0] * X[2] * rP + g[1] * X[3] * rT +
+               X[4] * (rT * rP);
     }
     case PS_COV_TEEE:
-    case PS_COV_TEEE_PLANCK: {  // src/covariance.jl:362-367 and :392-397
-        const double *EEjq = S[0], *EEjp = S[1], *TEip = S[2], *TEiq = S[3];
-        const double *rjq = R[0], *rjp = R[1];
-        return (sqrt(EEjq[a] * EEjq[b]) * (TEip[a] + TEip[b]) * X[0] +
-                sqrt(EEjp[a] * EEjp[b]) * (TEiq[a] + TEiq[b]) * X[1] + (TEip[a] + TEip[b]) * X[2] * rjq[a] * rjq[b] +
-                (TEiq[a] + TEiq[b]) * X[3] * rjp[a] * rjp[b]) /
-               2;
+    case PS_COV_TEEE_PLANCK:  // src/covariance.jl:362-367 and :392-397; EEjq, EEjp, TEip, TEiq; r_jq, r_jp
+        return (g[0] * (Sa[2] + Sb[2]) * X[0] + g[1] * (Sa[3] + Sb[3]) * X[1] + (Sa[2] + Sb[2]) * X[2] * Ra[0] * Rb[0] +
+                (Sa[3] + Sb[3]) * X[3] * Ra[1] * Rb[1]) / 2;
+    default:  // PS_COV_TTEE, src/covariance.jl:438-441; TEip, TEiq, TEjq, TEjp
+        return ((Sa[0] * Sb[2] + Sa[2] * Sb[0]) * X[0] + (Sa[1] * Sb[3] + Sa[3] * Sb[1]) * X[1]) / 2;
     }
-    default: {  // PS_COV_TTEE, src/covariance.jl:438-441
-        const double *TEip = S[0], *TEiq = S[1], *TEjq = S[2], *TEjp = S[3];
-        return ((TEip[a] * TEjq[b] + TEjq[a] * TEip[b]) * X[0] + (TEiq[a] * TEjp[b] + TEjp[a] * TEiq[b]) * X[1]) / 2;
+}
+
+// How many spectra of a kind enter through sqrt(Sa Sb): the first ones.
+__host__ __device__ constexpr int cov_roots(int kind)
+{
+    return kind == PS_COV_TTTT || kind == PS_COV_EEEE ? 4 : (kind == PS_COV_TTEE ? 0 : 2);
+}
+// ... and how many noise ratios it has.
+__host__ __device__ constexpr int cov_ratios(int kind)
+{
+    return kind == PS_COV_TTTT || kind == PS_COV_EEEE ? 4 : (kind == PS_COV_TTEE ? 0 : 2);
+}
+
+// The element of one pair (l1 = a, l2 = b), a <= b.
+__device__ __forceinline__ double cov_combine(int kind, const double* const* S, const double* const* R,
+                                              const double* X, int a, int b)
+{
+    double Sa[4], Sb[4], g[4], Ra[4], Rb[4];
+    const int ng = cov_roots(kind), nr = cov_ratios(kind);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        Sa[i] = S[i][a];
+        Sb[i] = S[i][b];
+        g[i] = i < ng ? sqrt(Sa[i] * Sb[i]) : 0.0;
+        Ra[i] = i < nr ? R[i][a] : 0.0;
+        Rb[i] = i < nr ? R[i][b] : 0.0;
     }
-    }
+    return cov_form(kind, Sa, Sb, g, Ra, Rb, X);
 }
 
 }  // namespace ps
