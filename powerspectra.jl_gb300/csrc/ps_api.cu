@@ -1615,8 +1615,8 @@ static int window_run(ps_ctx* c, const double* const* dA, const double* const* d
     p.lmax = lmax;
     p.mmax = mmax;
     p.lout = lout;
-    p.mchunk = ps::kAlmChunk;
-    p.nmchunks = ps::alm2cl_chunks(mmax);
+    p.mchunk = ps::alm2cl_chunk(mmax, lout);
+    p.nmchunks = mmax / p.mchunk + 1;
     for (int t = 0; t < nterms; ++t) {
         p.a[t] = (const double2*)dA[t];
         p.b[t] = (const double2*)dB[t];

@@ -111,7 +111,7 @@ cudaError_t launch_quickpol_ff(const double* W, long long nW, int lmax, int bl, 
 // alm2cl reduction (ps_window.cu).  Term t pairs coefficient sets a[t], b[t]
 // (HEALPix m-major order, lmax / mmax); a null set stands for all zeros.
 constexpr int kAlmMaxTerms = 16;
-constexpr int kAlmChunk = 64;  // m values per block of the partial-sum kernel
+constexpr int kAlmChunk = 64;  // most m values per block of the partial-sum kernel
 struct AlmParams {
     const double2* a[kAlmMaxTerms];
     const double2* b[kAlmMaxTerms];
@@ -120,7 +120,7 @@ struct AlmParams {
     int mchunk, nmchunks;
     double* partial;  // nterms * nmchunks * (lout + 1)
 };
-int alm2cl_chunks(int mmax);
+int alm2cl_chunk(int mmax, int lout);  // m values per chunk
 // after_partial, when given, is recorded between the partial-sum kernel and the reduction.
 cudaError_t launch_alm2cl(const AlmParams& p, double scale, bool per_l, double* W, cudaStream_t s,
                           cudaEvent_t after_partial = nullptr);
