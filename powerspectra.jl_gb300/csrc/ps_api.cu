@@ -427,26 +427,22 @@ static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* 
         st = ensure(c, &c->d_raw, &c->raw_cap, (size_t)K * nuse);
         if (st) return st;
     }
+    const bool split = mode == PS_MODE_CHOSEN;
+    if (split && (st = ensure_int2(c, &c->d_bf, &c->bf_cap, (size_t)K * wlen))) return st;
+    const double* src[ps::kMaxWin];
     for (int k = 0; k < K; ++k) {
         if (!W[k]) return set_err(c, PS_ERR_ARG, "window %d is NULL", k);
-        const double* src = W[k];
+        src[k] = W[k];
         if (host) {
             PS_CUDA(c, cudaMemcpyAsync(c->d_raw + (size_t)k * nuse, W[k], nuse * sizeof(double),
                                        cudaMemcpyHostToDevice, c->stream));
-            src = c->d_raw + (size_t)k * nuse;
+            src[k] = c->d_raw + (size_t)k * nuse;
         }
-        PS_CUDA(c, ps::launch_pad_windows(c->d_win + (size_t)k * wlen, src, nuse, wlen, c->stream));
-        c->launches++;
         p.win[k].wW = c->d_win + (size_t)k * wlen;
+        if (split) p.win[k].bf = c->d_bf + (size_t)k * wlen;
     }
-    if (mode == PS_MODE_CHOSEN) {
-        if ((st = ensure_int2(c, &c->d_bf, &c->bf_cap, (size_t)K * wlen))) return st;
-        for (int k = 0; k < K; ++k) {
-            PS_CUDA(c, ps::launch_split_windows(c->d_bf + (size_t)k * wlen, p.win[k].wW, wlen, c->stream));
-            c->launches++;
-            p.win[k].bf = c->d_bf + (size_t)k * wlen;
-        }
-    }
+    PS_CUDA(c, ps::launch_prep_set(src, K, nuse, wlen, c->d_win, split ? c->d_bf : nullptr, c->stream));
+    c->launches += ps::set_launches(K);
     return PS_OK;
 }
 
@@ -958,11 +954,10 @@ int ps_coupledcov_set_device(ps_ctx* c, int nblk, const int* kinds, const double
         (st = ensure_int2(c, &c->d_cbf, &c->cbf_cap, (size_t)nx * wlen)) ||
         (st = ensure(c, &c->d_xi, &c->xi_cap, (size_t)nx * n * n)))
         return st;
-    for (int j = 0; j < nx; ++j) {
-        PS_CUDA(c, ps::launch_pad_windows(c->d_cwin + (size_t)j * wlen, dW[xw[j].b][xw[j].k], nuse, wlen, c->stream));
-        PS_CUDA(c, ps::launch_split_windows(c->d_cbf + (size_t)j * wlen, c->d_cwin + (size_t)j * wlen, wlen, c->stream));
-        c->launches += 2;
-    }
+    std::vector<const double*> xsrc(nx);
+    for (int j = 0; j < nx; ++j) xsrc[j] = dW[xw[j].b][xw[j].k];
+    PS_CUDA(c, ps::launch_prep_set(xsrc.data(), nx, nuse, wlen, c->d_cwin, c->d_cbf, c->stream));
+    c->launches += ps::set_launches(nx);
     const int classes[4][2] = {{ps::PROD_00_00, ps::PAR_ALL}, {ps::PROD_22_22, ps::PAR_EVEN},
                                {ps::PROD_22_22, ps::PAR_ODD}, {ps::PROD_00_22, ps::PAR_EVEN}};
     for (const auto& cl : classes) {
@@ -1071,15 +1066,12 @@ int ps_mcm_set_device(ps_ctx* c, unsigned cases, const double* const* dW, int K,
         long long nuse = nW < (int64_t)(2 * lmax + 1) ? nW : (int64_t)(2 * lmax + 1);
         if ((st = ensure(c, &c->d_win, &c->win_cap, (size_t)K * wlen))) return st;
         if (mode == PS_MODE_CHOSEN && (st = ensure_int2(c, &c->d_bf, &c->bf_cap, (size_t)K * wlen))) return st;
+        const bool split = mode == PS_MODE_CHOSEN;
+        PS_CUDA(c, ps::launch_prep_set(dW, K, nuse, wlen, c->d_win, split ? c->d_bf : nullptr, c->stream));
+        c->launches += ps::set_launches(K);
         for (int k = 0; k < K; ++k) {
-            PS_CUDA(c, ps::launch_pad_windows(c->d_win + (size_t)k * wlen, dW[k], nuse, wlen, c->stream));
-            c->launches++;
             descs[k].wW = c->d_win + (size_t)k * wlen;
-            if (mode == PS_MODE_CHOSEN) {
-                PS_CUDA(c, ps::launch_split_windows(c->d_bf + (size_t)k * wlen, descs[k].wW, wlen, c->stream));
-                c->launches++;
-                descs[k].bf = c->d_bf + (size_t)k * wlen;
-            }
+            if (split) descs[k].bf = c->d_bf + (size_t)k * wlen;
         }
         base.wlen = wlen;
         base.nw = (int)nuse;

@@ -37,28 +37,60 @@ cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s)
     return launch_chosen8(p, spec, n00, n22, s);
 }
 
-// (2 l3 + 1) W[l3] in FP64 -> (float mantissa in [0.5, 1), exponent); zeros -> (0, kZeroExp)
-__global__ void k_split_windows(int2* __restrict__ dst, const double* __restrict__ wW, int wlen)
+// Entry j of a window: (2 l3 + 1) W[l3] in FP64, zero for j >= nW, and split into (float mantissa in
+// [0.5, 1), exponent), zeros as (0, kZeroExp).
+__device__ __forceinline__ void prep_entry(const double* __restrict__ src, long long nW, int j, double* wW, int2* bf)
 {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < wlen; j += gridDim.x * blockDim.x) {
-        double v = wW[j];
-        int e = 0;
-        double m = (v == 0.0) ? 0.0 : frexp(v, &e);
-        dst[j] = (v == 0.0) ? make_int2(0, kZeroExp) : make_int2(__float_as_int((float)m), e);
-    }
+    const double v = j < nW ? (2.0 * j + 1.0) * src[j] : 0.0;
+    wW[j] = v;
+    if (!bf) return;
+    int e = 0;
+    const double m = v == 0.0 ? 0.0 : frexp(v, &e);
+    bf[j] = v == 0.0 ? make_int2(0, kZeroExp) : make_int2(__float_as_int((float)m), e);
 }
 
 // All windows of a batch in one launch: pad + premultiply + split.
 __global__ void k_prep_windows(const WinPrep* __restrict__ list, int n)
 {
     const WinPrep w = list[blockIdx.y];
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < w.wlen; j += gridDim.x * blockDim.x) {
-        double v = (j < w.nW) ? (2.0 * j + 1.0) * w.src[j] : 0.0;
-        w.wW[j] = v;
-        int e = 0;
-        double m = (v == 0.0) ? 0.0 : frexp(v, &e);
-        w.bf[j] = (v == 0.0) ? make_int2(0, kZeroExp) : make_int2(__float_as_int((float)m), e);
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < w.wlen; j += gridDim.x * blockDim.x)
+        prep_entry(w.src, w.nW, j, w.wW, w.bf);
+}
+
+// The windows of one call: window blockIdx.y.  One launch instead of one or two per window, which cost
+// about 2.5 us each (31 windows of a covariance set: 62 launches).
+struct SetPrep {
+    const double* src[kSetWindows];
+    long long nW;
+    double* wW;
+    int2* bf;
+    int wlen;
+};
+__global__ void k_prep_set(const SetPrep p)
+{
+    const int k = blockIdx.y;
+    int2* bf = p.bf ? p.bf + (size_t)k * p.wlen : nullptr;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p.wlen; j += gridDim.x * blockDim.x)
+        prep_entry(p.src[k], p.nW, j, p.wW + (size_t)k * p.wlen, bf);
+}
+
+cudaError_t launch_prep_set(const double* const* src, int K, long long nW, int wlen, double* wW, int2* bf,
+                            cudaStream_t s)
+{
+    for (int k0 = 0; k0 < K; k0 += kSetWindows) {
+        const int n = K - k0 < kSetWindows ? K - k0 : kSetWindows;
+        SetPrep p;
+        for (int k = 0; k < n; ++k) p.src[k] = src[k0 + k];
+        p.nW = nW;
+        p.wW = wW + (size_t)k0 * wlen;
+        p.bf = bf ? bf + (size_t)k0 * wlen : nullptr;
+        p.wlen = wlen;
+        int bx = (wlen + 255) / 256;
+        if (bx > 64) bx = 64;
+        k_prep_set<<<dim3(bx, n), 256, 0, s>>>(p);
+        if (cudaError_t e = cudaGetLastError()) return e;
     }
+    return cudaSuccess;
 }
 
 cudaError_t launch_prep_windows(const WinPrep* list, int n, int max_wlen, cudaStream_t s)
@@ -68,15 +100,6 @@ cudaError_t launch_prep_windows(const WinPrep* list, int n, int max_wlen, cudaSt
     int bx = (max_wlen + threads - 1) / threads;
     if (bx > 64) bx = 64;
     k_prep_windows<<<dim3(bx, n), threads, 0, s>>>(list, n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_split_windows(int2* dst, const double* wW, int wlen, cudaStream_t s)
-{
-    int threads = 256;
-    int blocks = (wlen + threads - 1) / threads;
-    if (blocks > 1024) blocks = 1024;
-    k_split_windows<<<blocks, threads, 0, s>>>(dst, wW, wlen);
     return cudaGetLastError();
 }
 

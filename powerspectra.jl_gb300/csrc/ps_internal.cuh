@@ -93,8 +93,12 @@ int chosen_batch_template(const CouplingParams& p, int nwin);  // compile-time s
 cudaError_t launch_prep_windows(const WinPrep* list, int n, int max_wlen, cudaStream_t s);
 cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s);
 cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s);
-cudaError_t launch_pad_windows(double* dst, const double* src, long long nW, int wlen, cudaStream_t s);
-cudaError_t launch_split_windows(int2* dst, const double* wW, int wlen, cudaStream_t s);
+// K windows of nW entries (device pointers in a host array) into padded rows wW + k wlen of (2l+1) W[l]
+// and, when bf is given, their split copies bf + k wlen, one launch per kSetWindows windows.
+constexpr int kSetWindows = 64;
+inline int set_launches(int K) { return (K + kSetWindows - 1) / kSetWindows; }
+cudaError_t launch_prep_set(const double* const* src, int K, long long nW, int wlen, double* wW, int2* bf,
+                            cudaStream_t s);
 
 // Exponent marking an exact zero in the split window arrays.
 constexpr int kZeroExp = -100000;

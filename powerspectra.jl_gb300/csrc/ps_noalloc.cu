@@ -119,12 +119,12 @@ extern "C" int ps_mcm_multi_device_noalloc(unsigned cases, const double* const d
     const long long nuse = nW < (int64_t)(2 * lmax + 1) ? nW : (int64_t)(2 * lmax + 1);
     p.nw = (int)nuse;
     int K = 0;
+    const double* src[4];
     for (int sp = 0; sp < 4; ++sp) {
         if (!(cases & (1u << sp))) continue;
         double* w = win + (size_t)K * p.wlen;
         int2* b = bf + (size_t)K * p.wlen;
-        if (ps::launch_pad_windows(w, dW[sp], nuse, p.wlen, s) != cudaSuccess) return PS_ERR_CUDA;
-        if (ps::launch_split_windows(b, w, p.wlen, s) != cudaSuccess) return PS_ERR_CUDA;
+        src[K] = dW[sp];
         p.win[K].wW = w;
         p.win[K].bf = b;
         switch (sp) {
@@ -137,6 +137,7 @@ extern "C" int ps_mcm_multi_device_noalloc(unsigned cases, const double* const d
         ++K;
     }
     p.nwin = K;
+    if (ps::launch_prep_set(src, K, nuse, p.wlen, win, bf, s) != cudaSuccess) return PS_ERR_CUDA;
     const ps_tiles::Geometry G = ps_tiles::geometry(lmin, lmax);
     const int groups = 8 * G.nb - G.glo;
     k_fill_tiles<<<(groups + 255) / 256, 256, 0, s>>>(tasks, lmin, lmax);

@@ -307,23 +307,6 @@ cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------
-// window padding: dst[j] = (2j+1) src[j] for j < nW, 0 for nW <= j < wlen
-__global__ void k_pad_windows(double* __restrict__ dst, const double* __restrict__ src, long long nW, int wlen)
-{
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < wlen; j += gridDim.x * blockDim.x)
-        dst[j] = (j < nW) ? (2.0 * j + 1.0) * src[j] : 0.0;
-}
-
-cudaError_t launch_pad_windows(double* dst, const double* src, long long nW, int wlen, cudaStream_t s)
-{
-    int threads = 256;
-    int blocks = (wlen + threads - 1) / threads;
-    if (blocks > 1024) blocks = 1024;
-    k_pad_windows<<<blocks, threads, 0, s>>>(dst, src, nW, wlen);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
 // FMA-pipe probe: 8 independent FMA chains per thread, FMA counted as 2 flops.
 template <typename T>
 __global__ void __launch_bounds__(256) k_fma_probe(T* sink, int iters)
