@@ -103,6 +103,15 @@ cudaError_t launch_prep_set(const double* const* src, int K, long long nW, int w
 // Exponent marking an exact zero in the split window arrays.
 constexpr int kZeroExp = -100000;
 cudaError_t launch_fma_probe(int fp64, double* sink, int blocks, int iters, cudaStream_t s);
+// LU solve of the decoupling step (ps_lu.cu).
+bool lu_fits(int n, int nrhs);
+struct LuWork {
+    cudaStream_t side;         // the panels' stream
+    cudaEvent_t panel, rest;
+    int* perm;                 // 128 ints
+    int* info;
+};
+cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s);
 cudaError_t launch_transpose(double* dst, const double* src, int n, cudaStream_t s);
 // scratch: quickpol_scratch(lmax) doubles; half: for lmax
 size_t quickpol_scratch(int lmax);

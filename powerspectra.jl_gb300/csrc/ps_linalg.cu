@@ -7,9 +7,11 @@
 //       the decoupling `M \ pCl` of master (src/modecoupling.jl:358,
 //       src/blockspectralmatrix.jl:124-129).
 //
-// Both use cuSOLVER's FP64 getrf/getrs; a singular matrix is reported as
+// The first, and the second beyond ps::lu_fits, use cuSOLVER's FP64 getrf/getrs; the
+// second's usual sizes are solved by ps_lu.cu.  A singular matrix is reported as
 // PS_ERR_ARG (no device assert).  Matrices are column-major, as everywhere.
 #include <cusolverDn.h>
+#include <limits.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -55,6 +57,8 @@ struct ps_linalg {
     double* x = nullptr;  // right-hand sides / result
     double* t = nullptr;  // transpose scratch
     size_t cap = 0;       // elements of a / x / t
+    cudaStream_t side = nullptr;  // ps_lu.cu's panels
+    cudaEvent_t ev_panel = nullptr, ev_rest = nullptr;
 };
 
 static int la_err(char* err, size_t n, int code, const char* fmt, ...)
@@ -79,12 +83,10 @@ static int la_err(char* err, size_t n, int code, const char* fmt, ...)
         if (s_ != CUSOLVER_STATUS_SUCCESS) return la_err(err, errn, PS_ERR_CUDA, "%s: status %d", #call, (int)s_); \
     } while (0)
 
-static int la_reserve(ps_linalg* L, size_t n2, int n, cudaStream_t s, char* err, size_t errn)
+// Device buffers for n x n matrices (n2 elements each) and n pivots; with `solver`, cuSOLVER's handle
+// and workspace too, without it the stream and events of ps_lu.cu.
+static int la_reserve(ps_linalg* L, size_t n2, int n, bool solver, cudaStream_t s, char* err, size_t errn)
 {
-    if (!L->h) {
-        LA_SOLVER(cusolverDnCreate(&L->h));
-    }
-    LA_SOLVER(cusolverDnSetStream(L->h, s));
     if (n2 > L->cap) {
         cudaFree(L->a);
         cudaFree(L->x);
@@ -96,14 +98,29 @@ static int la_reserve(ps_linalg* L, size_t n2, int n, cudaStream_t s, char* err,
         LA_CUDA(cudaMalloc((void**)&L->t, n2 * sizeof(double)));
         L->cap = n2;
     }
-    if (n > L->ipiv_n) {
+    const int npiv = n < 128 ? 128 : n;  // pivots, or the row permutations of two panels
+    if (npiv > L->ipiv_n) {
         cudaFree(L->ipiv);
         L->ipiv = nullptr;
         L->ipiv_n = 0;
-        LA_CUDA(cudaMalloc((void**)&L->ipiv, (size_t)n * sizeof(int)));
-        L->ipiv_n = n;
+        LA_CUDA(cudaMalloc((void**)&L->ipiv, (size_t)npiv * sizeof(int)));
+        L->ipiv_n = npiv;
     }
     if (!L->info) LA_CUDA(cudaMalloc((void**)&L->info, sizeof(int)));
+    if (!solver) {
+        if (!L->side) {
+            int least = 0, greatest = 0;
+            LA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            LA_CUDA(cudaStreamCreateWithPriority(&L->side, cudaStreamNonBlocking, greatest));
+        }
+        if (!L->ev_panel) LA_CUDA(cudaEventCreateWithFlags(&L->ev_panel, cudaEventDisableTiming));
+        if (!L->ev_rest) LA_CUDA(cudaEventCreateWithFlags(&L->ev_rest, cudaEventDisableTiming));
+        return PS_OK;
+    }
+    if (!L->h) {
+        LA_SOLVER(cusolverDnCreate(&L->h));
+    }
+    LA_SOLVER(cusolverDnSetStream(L->h, s));
     int lw = 0;
     LA_SOLVER(cusolverDnDgetrf_bufferSize(L->h, n, n, L->a, n, &lw));
     if (lw > L->lwork) {
@@ -136,6 +153,9 @@ void ps_linalg_free(ps_linalg* L)
 {
     if (!L) return;
     if (L->h) cusolverDnDestroy(L->h);
+    if (L->side) cudaStreamDestroy(L->side);
+    if (L->ev_panel) cudaEventDestroy(L->ev_panel);
+    if (L->ev_rest) cudaEventDestroy(L->ev_rest);
     cudaFree(L->work);
     cudaFree(L->ipiv);
     cudaFree(L->info);
@@ -158,7 +178,7 @@ static int la_in(double* dst, const double* src, int rows, int cols, int64_t ld,
 int ps_linalg_decouple(ps_linalg* L, const double* Y, const double* B1, const double* B2, int n, int64_t ldin,
                        double* out, int64_t ldout, cudaStream_t s, char* err, size_t errn, bool on_device)
 {
-    int st = la_reserve(L, (size_t)n * n, n, s, err, errn);
+    int st = la_reserve(L, (size_t)n * n, n, true, s, err, errn);
     if (st) return st;
     if ((st = la_in(L->x, Y, n, n, ldin, s, err, errn, on_device))) return st;
     if ((st = la_in(L->a, B1, n, n, ldin, s, err, errn, on_device))) return st;
@@ -178,12 +198,25 @@ int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const dou
                     double* x, int64_t ldx, cudaStream_t s, char* err, size_t errn)
 {
     size_t need = (size_t)n * (size_t)(n > nrhs ? n : nrhs);
-    int st = la_reserve(L, need, n, s, err, errn);
+    const bool own = ps::lu_fits(n, nrhs);
+    int st = la_reserve(L, need, n, !own, s, err, errn);
     if (st) return st;
     if ((st = la_in(L->a, M, n, n, ldm, s, err, errn))) return st;
     if ((st = la_in(L->x, b, n, nrhs, ldb, s, err, errn))) return st;
-    if ((st = la_lu_solve(L, n, nrhs, L->x, s, "M", err, errn))) return st;
-    LA_CUDA(cudaMemcpy2DAsync(x, (size_t)ldx * sizeof(double), L->x, (size_t)n * sizeof(double),
+    const double* res = L->x;
+    if (own) {
+        const ps::LuWork wk = {L->side, L->ev_panel, L->ev_rest, L->ipiv, L->info};
+        LA_CUDA(ps::launch_lu_solve(L->a, n, L->x, nrhs, L->t, wk, s));
+        int info = 0;
+        LA_CUDA(cudaMemcpyAsync(&info, L->info, sizeof(int), cudaMemcpyDeviceToHost, s));
+        LA_CUDA(cudaStreamSynchronize(s));
+        if (info < 0) return la_err(err, errn, PS_ERR_TIMEOUT, "the LU panel kernel gave up waiting for its cluster");
+        if (info != INT_MAX) return la_err(err, errn, PS_ERR_ARG, "M is singular (zero pivot %d)", info);
+        res = L->t;
+    } else if ((st = la_lu_solve(L, n, nrhs, L->x, s, "M", err, errn))) {
+        return st;
+    }
+    LA_CUDA(cudaMemcpy2DAsync(x, (size_t)ldx * sizeof(double), res, (size_t)n * sizeof(double),
                               (size_t)n * sizeof(double), (size_t)nrhs, cudaMemcpyDeviceToHost, s));
     LA_CUDA(cudaStreamSynchronize(s));
     return PS_OK;
