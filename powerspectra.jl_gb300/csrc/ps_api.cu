@@ -54,6 +54,8 @@ struct ps_ctx {
     double* d_probe = nullptr;
     int2* d_bf = nullptr;  // split (mantissa, exponent) windows for the chosen kernel
     size_t bf_cap = 0;
+    unsigned char* d_slices = nullptr;  // its table of window slices, one launch at a time
+    size_t slices_cap = 0;
     double* d_alm = nullptr;  // harmonic coefficients copied in by ps_window_W (2 doubles each)
     size_t alm_cap = 0;
     double* d_part = nullptr;  // alm2cl partial sums
@@ -85,6 +87,8 @@ struct ps_ctx {
         bool launches = false;
         std::vector<ps::CouplingParams> host_groups;
         int2* d_tasks = nullptr;
+        unsigned char* d_slices = nullptr;  // the groups' tables of window slices
+        int ngroups = 0, max_slice_lmax = 0;  // the largest lmax with a table (0: no tables)
         // tensor-core launches (the problems' TT slots and ++/-- slots when there are
         // mma_min_slots of them), enqueued before the CUDA-core part,
         // with the block lists of every distinct (lmin, lmax) in d_mtiles
@@ -366,13 +370,18 @@ static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first =
     if (st) return st;
     p.tasks = c->d_tiles;
     p.ntasks = c->ntiles;
-    if (mode != PS_MODE_CHOSEN && (st = ensure_half(c, p.lmax, &p.half))) return st;
+    if (mode == PS_MODE_CHOSEN) {
+        if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, ps::slice_table_bytes(p)))) return st;
+        p.slices = c->d_slices;
+    } else if ((st = ensure_half(c, p.lmax, &p.half))) {
+        return st;
+    }
     if (first) PS_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     if (mode == PS_MODE_CHOSEN)
         PS_CUDA(c, ps::launch_chosen(p, c->stream));
     else
         PS_CUDA(c, ps::launch_plain_fp64(p, c->stream));
-    c->launches++;
+    c->launches += mode == PS_MODE_CHOSEN ? 2 : 1;
     if (last) {
         PS_CUDA(c, cudaEventRecord(c->ev1, c->stream));
         c->timed = true;
@@ -412,8 +421,8 @@ static int ensure_int2(ps_ctx* c, int2** p, size_t* cap, size_t need)
     return PS_OK;
 }
 
-// Upload (if host) and pad K windows into ctx->d_win; fills p.win[k].wW (and,
-// for the chosen kernel, the split copies p.win[k].bf).
+// Upload (if host) K windows and pad them into ctx->d_win, p.win[k].wW; for the chosen kernel its own
+// preparation does the padding (p.src), so p is good for one launch.
 static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* W, int K, int64_t nW, int lmax,
                          bool host, int mode)
 {
@@ -427,8 +436,6 @@ static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* 
         st = ensure(c, &c->d_raw, &c->raw_cap, (size_t)K * nuse);
         if (st) return st;
     }
-    const bool split = mode == PS_MODE_CHOSEN;
-    if (split && (st = ensure_int2(c, &c->d_bf, &c->bf_cap, (size_t)K * wlen))) return st;
     const double* src[ps::kMaxWin];
     for (int k = 0; k < K; ++k) {
         if (!W[k]) return set_err(c, PS_ERR_ARG, "window %d is NULL", k);
@@ -439,10 +446,12 @@ static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* 
             src[k] = c->d_raw + (size_t)k * nuse;
         }
         p.win[k].wW = c->d_win + (size_t)k * wlen;
-        if (split) p.win[k].bf = c->d_bf + (size_t)k * wlen;
+        if (mode == PS_MODE_CHOSEN) p.src[k] = src[k];
     }
-    PS_CUDA(c, ps::launch_prep_set(src, K, nuse, wlen, c->d_win, split ? c->d_bf : nullptr, c->stream));
-    c->launches += ps::set_launches(K);
+    if (mode != PS_MODE_CHOSEN) {
+        PS_CUDA(c, ps::launch_prep_set(src, K, nuse, wlen, c->d_win, nullptr, c->stream));
+        c->launches += ps::set_launches(K);
+    }
     return PS_OK;
 }
 
@@ -457,6 +466,7 @@ static void batch_release(ps_ctx* c)
     cudaFree(b.d_win);
     cudaFree(b.d_bf);
     cudaFree(b.d_tasks);
+    cudaFree(b.d_slices);
     cudaFree(b.d_mtiles);
     cudaFree(b.d_btab);
     b = ps_ctx::Batch();
@@ -622,6 +632,7 @@ void ps_destroy(ps_ctx* c)
     cudaFree(c->d_out);
     cudaFree(c->d_probe);
     cudaFree(c->d_bf);
+    cudaFree(c->d_slices);
     cudaFree(c->d_alm);
     cudaFree(c->d_part);
     cudaFree(c->d_qp);
@@ -1185,6 +1196,10 @@ int ps_mcm_set(ps_ctx* c, unsigned cases, const double* const* W, int K, int64_t
     return check_status(c);
 }
 
+// What the groups' slice tables of a batch may take together: 256 problems up to lmax 1023 need 1 GB.
+// Groups past it have none.
+static const size_t kBatchSliceBytes = (size_t)2 << 30, kNone = ~(size_t)0;
+
 int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int bps)
 {
     if (!c) return PS_ERR_ARG;
@@ -1194,6 +1209,7 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         if ((st = check_problem(c, probs[i], i))) return st;
     if (gs == 0) gs = c->tuned_group_slots ? c->tuned_group_slots : 4;
     if (gs != 2 && gs != 4 && gs != 8) return set_err(c, PS_ERR_ARG, "group_slots must be 2, 4 or 8 (got %d)", gs);
+    if (bps == 0) bps = c->tuned_blocks_per_sm;
     PS_CUDA(c, cudaSetDevice(c->device));
     batch_release(c);
     ps_ctx::Batch& b = c->batch;
@@ -1324,6 +1340,30 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
             }
         }
     }
+    // the groups' tables of window slices: one for the launches in turn; one each for the persistent
+    // kernel, whose groups run side by side (none for small lmax, or where there is no room)
+    size_t slice_bytes = 0, slice_cap = 0;
+    std::vector<size_t> slice_at(groups.size(), 0);
+    for (size_t g = 0; g < groups.size(); ++g) {
+        if (bps < 0) {
+            slice_bytes = std::max(slice_bytes, ps::slice_table_bytes(groups[g]));
+            continue;
+        }
+        const size_t need = (ps::batch_slice_bytes(groups[g].lmax, gs) + 255) / 256 * 256;
+        const bool has = groups[g].lmax >= ps::kSliceMinLmax && slice_bytes + need <= kBatchSliceBytes;
+        slice_at[g] = has ? slice_bytes : kNone;
+        if (has) slice_bytes += need;
+    }
+    if (slice_bytes && (st = ensure_bytes(c, &b.d_slices, &slice_cap, slice_bytes)) && bps < 0) {
+        batch_release(c);
+        return st;
+    }
+    for (size_t g = 0; g < groups.size() && b.d_slices; ++g) {
+        if (slice_at[g] == kNone) continue;
+        groups[g].slices = b.d_slices + slice_at[g];
+        b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
+    }
+    b.ngroups = (int)groups.size();
     // items of one kernel body together (warps of an SM then share their
     // instruction stream), longest first within each body
     std::vector<int> order(items.size());
@@ -1385,7 +1425,7 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
     int nsm = 0;
     PS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     int occ = ps::batch_blocks_per_sm(gs);
-    if (bps == 0) bps = c->tuned_blocks_per_sm ? c->tuned_blocks_per_sm : occ;
+    if (bps == 0) bps = occ;
     b.launches = bps < 0;
     if (!b.launches && (bps < 1 || bps > occ)) bps = occ;
     b.nitems = (int)sorted.size();
@@ -1415,6 +1455,8 @@ static int batch_enqueue(ps_ctx* c, cudaStream_t s)
         bp.items = b.d_items;
         bp.nitems = b.nitems;
         bp.counter = b.d_counter;
+        if (b.max_slice_lmax)
+            PS_CUDA(c, ps::launch_batch_slices(b.d_groups, b.ngroups, b.max_slice_lmax, b.group_slots, s));
         PS_CUDA(c, ps::launch_batch_chosen(bp, b.blocks, b.group_slots, s));
     }
     PS_CUDA(c, cudaEventRecord(c->ev1, s));
@@ -1424,7 +1466,8 @@ static int batch_enqueue(ps_ctx* c, cudaStream_t s)
 // kernels one run of the batch launches (window preparation included)
 static size_t batch_kernel_count(const ps_ctx::Batch& b)
 {
-    return 1 + 2 * b.host_mma.size() + (b.launches ? b.host_groups.size() : (b.nitems > 0 ? 1 : 0));
+    const size_t one = b.nitems > 0 ? 1 + (b.max_slice_lmax != 0) : 0;  // the persistent kernel and its tables
+    return 1 + 2 * b.host_mma.size() + (b.launches ? 2 * b.host_groups.size() : one);
 }
 
 int ps_batch_run(ps_ctx* c)

@@ -27,16 +27,13 @@ struct BatchSets<8> {
 template <int NWIN>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 3) k_batch_chosen(const BatchParams bp)
 {
-    __shared__ __align__(16) float sW[kWarpsPerBlock][2][NWIN][kSlots];  // 16-byte slot reads (4-slot bodies)
+    __shared__ Slice<NWIN> sS[kWarpsPerBlock][2][2];
     // each warp's copy of its current group's parameters: read in the inner
     // loops, so they live in shared memory rather than behind global loads
     __shared__ CouplingParams sG[kWarpsPerBlock];
-    __shared__ int2 sR[kWarpsPerBlock][2][NWIN][kSlots];
     __shared__ CoefTab sT[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    float* sF = &sW[warp][0][0][0];
-    float* sB = &sW[warp][1][0][0];
     int cur = -1;
     for (;;) {
         int it = 0;
@@ -56,17 +53,49 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 3) k_batc
         for (int q = 0; q < ntask; ++q) {
             const int l2_0 = item.z + 32 * q;
             switch (tmpl) {  // the group's compile-time slot set (prepare never emits others)
-            case 1: chosen_task<NWIN, true, false, BatchSets<NWIN>::s[0]>(g, item.y, l2_0, sF, sB, &sR[warp][0][0][0], sT[warp], lane); break;
-            case 2: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[1]>(g, item.y, l2_0, sF, sB, &sR[warp][0][0][0], sT[warp], lane); break;
-            case 3: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[2]>(g, item.y, l2_0, sF, sB, &sR[warp][0][0][0], sT[warp], lane); break;
-            case 4: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[3]>(g, item.y, l2_0, sF, sB, &sR[warp][0][0][0], sT[warp], lane); break;
-            case 5: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[4]>(g, item.y, l2_0, sF, sB, &sR[warp][0][0][0], sT[warp], lane); break;
-            case 6: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[5]>(g, item.y, l2_0, sF, sB, &sR[warp][0][0][0], sT[warp], lane); break;
+            case 1: chosen_task<NWIN, true, false, BatchSets<NWIN>::s[0]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
+            case 2: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[1]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
+            case 3: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[2]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
+            case 4: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[3]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
+            case 5: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[4]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
+            case 6: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[5]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
             default: break;  // prepare rejects groups without a body
             }
             __syncwarp();
         }
     }
+}
+
+// The slice tables of every group (blockIdx.z); window blockIdx.y.
+template <int NWIN>
+__global__ void __launch_bounds__(256) k_batch_slices(const CouplingParams* __restrict__ groups)
+{
+    const CouplingParams& p = groups[blockIdx.z];
+    const int k = blockIdx.y, lane = threadIdx.x & 31;
+    if (k >= p.nwin || !p.slices) return;
+    const int2* bf = p.win[k].bf;
+    const int n = slice_count(p.lmax), wlen = p.wlen;
+    Slice<NWIN>* table = reinterpret_cast<Slice<NWIN>*>(p.slices);
+    for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += gridDim.x * 8)
+        put_slice<NWIN>(table[i], i, k, wlen, lane, [&](int j) { return __ldg(bf + j); });
+}
+
+size_t batch_slice_bytes(int lmax, int nwin)
+{
+    return slice_bytes(nwin > 4 ? 8 : 4) * (size_t)slice_count(lmax);
+}
+
+cudaError_t launch_batch_slices(const CouplingParams* groups, int ngroups, int max_lmax, int nwin, cudaStream_t s)
+{
+    int bx = (slice_count(max_lmax) + 63) / 64;
+    if (bx > 32) bx = 32;  // the groups are many and uneven: few blocks each, several entries per warp
+    for (int g0 = 0; g0 < ngroups; g0 += 65535) {
+        const dim3 grid((unsigned)bx, nwin > 4 ? 8 : 4, (unsigned)(ngroups - g0 < 65535 ? ngroups - g0 : 65535));
+        if (nwin > 4) k_batch_slices<8><<<grid, 256, 0, s>>>(groups + g0);
+        else k_batch_slices<4><<<grid, 256, 0, s>>>(groups + g0);
+        if (cudaError_t e = cudaGetLastError()) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_batch_chosen(const BatchParams& bp, int blocks, int nwin, cudaStream_t s)

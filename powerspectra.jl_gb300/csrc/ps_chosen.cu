@@ -8,45 +8,61 @@ namespace ps {
 
 cudaError_t launch_chosen8(const CouplingParams& p, uint32_t spec, bool n00, bool n22, cudaStream_t s);
 
+namespace {
+
+// The instantiations: a launch takes the first whose slot list starts with its configuration, or the one
+// of its number of slots that reads the configuration from the parameters.
+struct Inst {
+    uint32_t spec;
+    int n;  // slots
+    cudaError_t (*launch)(const CouplingParams&, bool, bool, cudaStream_t);
+};
+#define PS_INST(n, spec) Inst{spec, n, launch_cfg<n, spec>}
+const Inst kInst[] = {
+    PS_INST(1, W00),          PS_INST(1, W02),          PS_INST(1, WPP),          PS_INST(1, WMM),
+    PS_INST(2, S_PPMM),       PS_INST(4, rep(W00, 4)),  PS_INST(4, S_PPMM2),      PS_INST(4, S_MCM4),
+    PS_INST(4, rep(W02, 4)),  PS_INST(4, rep(WPP, 4)),  PS_INST(4, rep(WMM, 4)),  PS_INST(5, S_TETE),
+};
+const Inst kAny[] = {PS_INST(1, 0), PS_INST(2, 0), PS_INST(4, 0)};
+#undef PS_INST
+
+const Inst* find_inst(const CouplingParams& p, uint32_t spec)  // null: launch_chosen8
+{
+    for (const Inst& i : kInst)
+        if (spec_fits(spec, p.nwin, i.spec, i.n)) return &i;
+    for (const Inst& i : kAny)
+        if (p.nwin <= i.n) return &i;
+    return nullptr;
+}
+
+}  // namespace
+
+size_t slice_table_bytes(const CouplingParams& p)
+{
+    const Inst* i = find_inst(p, spec_of(p));
+    return slice_bytes(i ? i->n : 8) * (size_t)slice_count(p.lmax);
+}
+
 cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s)
 {
+    if (p.ntasks <= 0) return cudaSuccess;
+    if (!p.slices || ((uintptr_t)p.slices & 15u)) return cudaErrorInvalidValue;
     bool n00 = false, n22 = false;
     for (int k = 0; k < p.nwin; ++k) {
         if (p.win[k].product != PROD_22_22) n00 = true;
         if (p.win[k].product != PROD_00_00) n22 = true;
     }
     const uint32_t spec = spec_of(p);
-    const int nw = p.nwin;
-    if (p.ntasks <= 0) return cudaSuccess;
-    // the smallest instantiation whose slot list starts with this configuration
-    if (spec_fits(spec, nw, W00, 1)) return launch_cfg<1, W00>(p, n00, n22, s);
-    if (spec_fits(spec, nw, W02, 1)) return launch_cfg<1, W02>(p, n00, n22, s);
-    if (spec_fits(spec, nw, WPP, 1)) return launch_cfg<1, WPP>(p, n00, n22, s);
-    if (spec_fits(spec, nw, WMM, 1)) return launch_cfg<1, WMM>(p, n00, n22, s);
-    if (spec_fits(spec, nw, S_PPMM, 2)) return launch_cfg<2, S_PPMM>(p, n00, n22, s);
-    if (spec_fits(spec, nw, rep(W00, 4), 4)) return launch_cfg<4, rep(W00, 4)>(p, n00, n22, s);
-    if (spec_fits(spec, nw, S_PPMM2, 4)) return launch_cfg<4, S_PPMM2>(p, n00, n22, s);
-    if (spec_fits(spec, nw, S_MCM4, 4)) return launch_cfg<4, S_MCM4>(p, n00, n22, s);
-    if (spec_fits(spec, nw, rep(W02, 4), 4)) return launch_cfg<4, rep(W02, 4)>(p, n00, n22, s);
-    if (spec_fits(spec, nw, rep(WPP, 4), 4)) return launch_cfg<4, rep(WPP, 4)>(p, n00, n22, s);
-    if (spec_fits(spec, nw, rep(WMM, 4), 4)) return launch_cfg<4, rep(WMM, 4)>(p, n00, n22, s);
-    if (spec_fits(spec, nw, S_TETE, 5)) return launch_cfg<5, S_TETE>(p, n00, n22, s);
-    if (nw <= 1) return launch_cfg<1, 0>(p, n00, n22, s);
-    if (nw <= 2) return launch_cfg<2, 0>(p, n00, n22, s);
-    if (nw <= 4) return launch_cfg<4, 0>(p, n00, n22, s);
-    return launch_chosen8(p, spec, n00, n22, s);
+    const Inst* i = find_inst(p, spec);
+    return i ? i->launch(p, n00, n22, s) : launch_chosen8(p, spec, n00, n22, s);
 }
 
-// Entry j of a window: (2 l3 + 1) W[l3] in FP64, zero for j >= nW, and split into (float mantissa in
-// [0.5, 1), exponent), zeros as (0, kZeroExp).
+// Entry j of a window: (2 l3 + 1) W[l3] in FP64, zero for j >= nW, and split.
 __device__ __forceinline__ void prep_entry(const double* __restrict__ src, long long nW, int j, double* wW, int2* bf)
 {
     const double v = j < nW ? (2.0 * j + 1.0) * src[j] : 0.0;
     wW[j] = v;
-    if (!bf) return;
-    int e = 0;
-    const double m = v == 0.0 ? 0.0 : frexp(v, &e);
-    bf[j] = v == 0.0 ? make_int2(0, kZeroExp) : make_int2(__float_as_int((float)m), e);
+    if (bf) bf[j] = split_entry(v);
 }
 
 // All windows of a batch in one launch: pad + premultiply + split.

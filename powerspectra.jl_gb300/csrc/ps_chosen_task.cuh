@@ -18,11 +18,13 @@
 //  * the forward (from jmin) and backward (from jmax) sweeps run interleaved
 //    in one loop: two independent dependency chains per lane;
 //  * windows are stored as (mantissa, exponent) pairs.  Every 32 steps each
-//    warp stages the slice of every window it is about to read into shared
+//    warp takes the slices of the windows it is about to read into shared
 //    memory, scaled by 2^-E with E the largest exponent of the slice, so FP32
 //    keeps full relative precision whatever the windows' dynamic range
 //    (mask spectra span > 1e-45 at l ~ 8000).  The 32-step FP32 partial sums
-//    are added into FP64 totals with the factor 2^E;
+//    are added into FP64 totals with the factor 2^E.  A slice depends on its
+//    first l3 alone, so a table of all of them is built once per launch (k_slices)
+//    and a warp copies its two per 32 steps;
 //  * FP64 is kept where stability and range need it: the last forward point,
 //    the least-squares match of the two sweeps, the normalisation, the sign and
 //    the totals;
@@ -106,44 +108,6 @@ struct ChunkSum<true> {
 template <int NWIN, bool N22>
 constexpr bool chunk_sums_ff() { return NWIN >= 8 && !N22; }
 
-// Window slices move in two stages.  fetch_slice issues asynchronous copies
-// (cp.async, 8 bytes per lane and slot) of the raw (mantissa, exponent) slots
-// [base, base + kSlots) into shared memory; they land while the previous chunk
-// computes.  scale_slice then rescales the raw slice by 2^-E, with E the
-// slice's largest exponent, into the FP32 slots the steps read, and returns E.
-__device__ __forceinline__ void fetch_slice(int2* raw, const int2* __restrict__ bf, int base, int wlen, int lane)
-{
-#pragma unroll
-    for (int q = 0; q < kStagePerLane; ++q) {
-        const int j = base + lane + 32 * q;
-        int2* d = raw + lane + 32 * q;
-        if (j >= 0 && j < wlen) {
-            const unsigned sa = (unsigned)__cvta_generic_to_shared(d);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(bf + j) : "memory");
-        } else {
-            *d = make_int2(0, kZeroExp);
-        }
-    }
-}
-__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void fetch_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-__device__ __forceinline__ int scale_slice(float* dst, const int2* raw, int lane, int stride = 1)
-{
-    int2 v[kStagePerLane];
-    int emax = kZeroExp;
-#pragma unroll
-    for (int q = 0; q < kStagePerLane; ++q) {
-        v[q] = raw[lane + 32 * q];
-        emax = max(emax, v[q].y);
-    }
-    emax = __reduce_max_sync(0xffffffffu, emax);
-#pragma unroll
-    for (int q = 0; q < kStagePerLane; ++q)
-        dst[(lane + 32 * q) * stride] = __int_as_float(v[q].x) * pow2f_or_zero(v[q].y - emax);
-    return emax;
-}
-
 // The scaled slices of a 4-slot kernel are interleaved as [slot][window], so
 // that a step reads the values of all its windows with one 16-byte load; other
 // kernels keep [window][slot].  Measured: the interleaving makes the 4-slot
@@ -151,6 +115,108 @@ __device__ __forceinline__ int scale_slice(float* dst, const int2* raw, int lane
 // to 16 % slower.
 template <int NWIN>
 constexpr bool slots_interleaved() { return NWIN == 4; }
+
+// One slice: the 64 values from some l3 of every window of a launch, each window in units of 2^E.
+template <int NWIN>
+struct __align__(16) Slice {
+    float v[NWIN * kSlots];
+    int E[(NWIN + 3) / 4 * 4];
+};
+constexpr size_t slice_bytes(int nwin) { return (size_t)nwin * kSlots * sizeof(float) + (size_t)(nwin + 3) / 4 * 16; }
+static_assert(sizeof(Slice<1>) == slice_bytes(1) && sizeof(Slice<4>) == slice_bytes(4) &&
+                  sizeof(Slice<5>) == slice_bytes(5) && slice_bytes(8) == 2080,
+              "whole 16-byte units");
+
+// The table: entry i is the slice from l3 = i + kSlice0.  A forward slice starts at l2_0 - l1 + t0, a
+// backward one at l1 + l2_0 - t0 - 31, with -31 <= l2_0 <= lmax, l2_0 + 31 >= l1 and 0 <= t0 < l1: from
+// -61 to 2 lmax - 31.
+constexpr int kSlice0 = -64;
+__host__ __device__ constexpr int slice_count(int lmax) { return 2 * lmax - 31 - kSlice0 + 1; }
+
+// (2 l3 + 1) W[l3] split into (float mantissa in [0.5, 1), exponent), zeros as (0, kZeroExp)
+__device__ __forceinline__ int2 split_entry(double v)
+{
+    int e = 0;
+    const double m = v == 0.0 ? 0.0 : frexp(v, &e);
+    return v == 0.0 ? make_int2(0, kZeroExp) : make_int2(__float_as_int((float)m), e);
+}
+
+// One warp per entry and window: entry `i`, window `k`, at(j) its split value at l3 = j (inside 0 .. wlen - 1).
+template <int NWIN, class At>
+__device__ __forceinline__ void put_slice(Slice<NWIN>& s, int i, int k, int wlen, int lane, At at)
+{
+    int2 v[kStagePerLane];
+    int emax = kZeroExp;
+#pragma unroll
+    for (int q = 0; q < kStagePerLane; ++q) {
+        const int j = i + kSlice0 + lane + 32 * q;
+        v[q] = j >= 0 && j < wlen ? at(j) : make_int2(0, kZeroExp);
+        emax = max(emax, v[q].y);
+    }
+    emax = __reduce_max_sync(0xffffffffu, emax);
+#pragma unroll
+    for (int q = 0; q < kStagePerLane; ++q) {
+        const int slot = lane + 32 * q;
+        s.v[slots_interleaved<NWIN>() ? slot * NWIN + k : k * kSlots + slot] =
+            __int_as_float(v[q].x) * pow2f_or_zero(v[q].y - emax);
+    }
+    if (lane == 0) s.E[k] = emax;
+}
+// The table of one launch's windows (blockIdx.y).  Staging each warp's slices from (mantissa, exponent)
+// pairs in the coupling kernel itself, a copy, a maximum and a scaling of 64 values per window and
+// sweep, took 17.75 ms for all spin cases at lmax 3071 where this takes 16.98, and 20.4 against 18.7 ms for
+// 256 small problems.  RAW: from the windows themselves (p.src), writing the padded rows too: a call
+// with one coupling launch then has no other preparation (TT at lmax 767 107.0 -> 105.0 us).
+template <int NWIN, bool RAW>
+__global__ void __launch_bounds__(256) k_slices(const CouplingParams p)
+{
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), k = blockIdx.y, lane = threadIdx.x & 31;
+    if (i >= slice_count(p.lmax)) return;
+    Slice<NWIN>& s = reinterpret_cast<Slice<NWIN>*>(p.slices)[i];
+    if (RAW) {
+        const double* __restrict__ W = p.src[k];
+        auto value = [&](int j) { return j < p.nw ? (2.0 * j + 1.0) * __ldg(W + j) : 0.0; };
+        put_slice<NWIN>(s, i, k, p.wlen, lane, [&](int j) { return split_entry(value(j)); });
+        // entry i writes the row's value at its first l3, the last entry those that follow
+        const int end = i + 1 == slice_count(p.lmax) ? p.wlen : i + kSlice0 + 1;
+        for (int j = i + kSlice0 + lane; j < end; j += 32)
+            if (j >= 0) const_cast<double*>(p.win[k].wW)[j] = value(j);
+    } else {
+        const int2* __restrict__ bf = p.win[k].bf;
+        put_slice<NWIN>(s, i, k, p.wlen, lane, [&](int j) { return __ldg(bf + j); });
+    }
+}
+
+// A slice into shared memory, asynchronously (it lands while the previous chunk computes).
+template <int NWIN>
+__device__ __forceinline__ void fetch_slice(Slice<NWIN>& dst, const unsigned char* table, int l3, int lane)
+{
+    const char* src = reinterpret_cast<const char*>(reinterpret_cast<const Slice<NWIN>*>(table) + (l3 - kSlice0));
+    const unsigned d = (unsigned)__cvta_generic_to_shared(&dst);
+#pragma unroll
+    for (int q = 0; q < ((int)sizeof(Slice<NWIN>) + 511) / 512; ++q) {
+        const int o = 16 * lane + 512 * q;
+        if (o < (int)sizeof(Slice<NWIN>))
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o), "l"(src + o) : "memory");
+    }
+}
+// A slice from the table or, with OWN, made here for a group that has none.  A compile-time choice, as the
+// launches always have a table; the branch moves their kernels by -2 % (all spin cases) to +3 % (TT, 02).
+template <int NWIN, bool OWN>
+__device__ __forceinline__ void get_slice(const CouplingParams& p, Slice<NWIN>& dst, int l3, int lane)
+{
+    if (!OWN || p.slices) {
+        fetch_slice<NWIN>(dst, p.slices, l3, lane);
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < p.nwin; ++k) {
+            const int2* __restrict__ bf = p.win[k].bf;
+            put_slice<NWIN>(dst, l3 - kSlice0, k, p.wlen, lane, [&](int j) { return __ldg(bf + j); });
+        }
+    }
+}
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void fetch_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // Window configuration: 4 bits per window, product + 1 in bits 0-1 (so a used
 // window is never 0) and parity in bits 2-3.  A non-zero SPEC fixes the
@@ -251,8 +317,8 @@ __device__ __forceinline__ void sweep_acc(const WinCfg<NWIN>& p, const Sweep& s,
     }
 }
 
-// One warp task: 32 consecutive l2 from l2_0 of row l1.  sF / sB are the
-// warp's shared-memory staging areas ([NWIN][kSlots] floats each).
+// One warp task: 32 consecutive l2 from l2_0 of row l1.  sl: the warp's slices in shared memory, two
+// per sweep (forward, backward), alternating from chunk to chunk.
 // ---- coefficient tables ----------------------------------------------------
 // For lane i of a warp task (l1, l2_0 + i) the recurrence coefficient at
 // forward step t factorises as P = G(t) F(u), u = 2i + t, with
@@ -434,9 +500,9 @@ __device__ __forceinline__ void tab_bwd(Sweep& s, const CoefTab& tb, int st, int
 // The Xi of pair (l1, l2_0 + lane) into Xi[]; returns whether the lane holds a
 // pair to write (l1 <= l2 <= lmax).  Lanes outside clamp l2 into [l1, lmax] and
 // compute values nobody writes.
-template <int NWIN, bool N00, bool N22, uint32_t SPEC>
-__device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1, const int l2_0, float* sF,
-                                          float* sB, int2* raw, CoefTab& tb, const int lane, double* Xi)
+template <int NWIN, bool N00, bool N22, uint32_t SPEC, bool OWN = false>
+__device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1, const int l2_0, Slice<NWIN> (*sl)[2],
+                                          CoefTab& tb, const int lane, double* Xi)
 {
     const int l2raw = l2_0 + lane;
     const bool active = l2raw >= l1 && l2raw <= p.lmax;
@@ -472,45 +538,19 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
     SBN0.zero();
     SBN2.zero();
 
-    int2* rF = raw;                  // raw forward slices, [NWIN][kSlots]
-    int2* rB = raw + NWIN * kSlots;  // raw backward slices
-#pragma unroll
-    for (int k = 0; k < NWIN; ++k) {
-        if (k < p.nwin) {
-            fetch_slice(rF + k * kSlots, p.win[k].bf, jmin0, p.wlen, lane);
-            fetch_slice(rB + k * kSlots, p.win[k].bf, jmax0 - kChunk + 1, p.wlen, lane);
-        }
-    }
+    get_slice<NWIN, OWN>(p, sl[0][0], jmin0, lane);
+    get_slice<NWIN, OWN>(p, sl[0][1], jmax0 - kChunk + 1, lane);
     fetch_commit();
     init_f_tables<N22>(tb, l1, l2_0, lane);
     for (int t0 = 0; t0 < T; t0 += kChunk) {
-        int eF[NWIN], eB[NWIN];
+        const int cur = (t0 / kChunk) & 1;
+        const float *sF = sl[cur][0].v, *sB = sl[cur][1].v;
         fetch_wait_all();
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < NWIN; ++k) {
-            if (k < p.nwin) {
-                if constexpr (slots_interleaved<NWIN>()) {
-                    eF[k] = scale_slice(sF + k, rF + k * kSlots, lane, NWIN);
-                    eB[k] = scale_slice(sB + k, rB + k * kSlots, lane, NWIN);
-                } else {
-                    eF[k] = scale_slice(sF + k * kSlots, rF + k * kSlots, lane);
-                    eB[k] = scale_slice(sB + k * kSlots, rB + k * kSlots, lane);
-                }
-            } else {
-                eF[k] = eB[k] = kZeroExp;
-            }
-        }
         build_tables<N22>(tb, t0, T, l1, l2_0, lane);
         __syncwarp();
         if (t0 + kChunk < T) {  // the next chunk's slices land while this one computes
-#pragma unroll
-            for (int k = 0; k < NWIN; ++k) {
-                if (k < p.nwin) {
-                    fetch_slice(rF + k * kSlots, p.win[k].bf, jmin0 + t0 + kChunk, p.wlen, lane);
-                    fetch_slice(rB + k * kSlots, p.win[k].bf, jmax0 - t0 - 2 * kChunk + 1, p.wlen, lane);
-                }
-            }
+            get_slice<NWIN, OWN>(p, sl[cur ^ 1][0], jmin0 + t0 + kChunk, lane);
+            get_slice<NWIN, OWN>(p, sl[cur ^ 1][1], jmax0 - t0 - 2 * kChunk + 1, lane);
         }
         fetch_commit();
         float cF[NWIN], cB[NWIN];
@@ -568,8 +608,8 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
         // ---- flush of the chunk sums (the norm sums carry the weight factor ws = 2^(WS4 ? 2 : 0)) ----
 #pragma unroll
         for (int k = 0; k < NWIN; ++k) {
-            SFW[k].add(cF[k], eF[k]);
-            SBW[k].add(cB[k], eB[k]);
+            SFW[k].add(cF[k], k < p.nwin ? sl[cur][0].E[k] : kZeroExp);
+            SBW[k].add(cB[k], k < p.nwin ? sl[cur][1].E[k] : kZeroExp);
         }
         if (N00) {
             SFN0.add(n0F, WS4 ? -2 : 0);
@@ -662,19 +702,18 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
 // One warp task with its own writes (the persistent batch kernel, whose items
 // hold l2_0 >= l1).
 template <int NWIN, bool N00, bool N22, uint32_t SPEC>
-__device__ __forceinline__ void chosen_task(const CouplingParams& p, const int l1, const int l2_0, float* sF,
-                                            float* sB, int2* raw, CoefTab& tb, const int lane)
+__device__ __forceinline__ void chosen_task(const CouplingParams& p, const int l1, const int l2_0, Slice<NWIN> (*sl)[2],
+                                            CoefTab& tb, const int lane)
 {
     double Xi[kMaxWin];
-    if (chosen_xi<NWIN, N00, N22, SPEC>(p, l1, l2_0, sF, sB, raw, tb, lane, Xi)) write_pair(p, l1, l2_0 + lane, Xi);
+    if (chosen_xi<NWIN, N00, N22, SPEC, true>(p, l1, l2_0, sl, tb, lane, Xi)) write_pair(p, l1, l2_0 + lane, Xi);
 }
 
 
 template <int NWIN, bool N00, bool N22, uint32_t SPEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 4) k_coupling_chosen(const CouplingParams p)
 {
-    __shared__ __align__(16) float sW[kWarpsPerBlock][2][NWIN][kSlots];
-    __shared__ int2 sR[kWarpsPerBlock][2][NWIN][kSlots];
+    __shared__ Slice<NWIN> sS[kWarpsPerBlock][2][2];
     __shared__ CoefTab sT[kWarpsPerBlock];
     __shared__ TileRows rows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -684,12 +723,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 4) k_coup
     double Xi[kMaxWin];
     bool active = false;
     if (task.x >= 0)  // warp-uniform
-        active = chosen_xi<NWIN, N00, N22, SPEC>(p, task.x, task.y, &sW[warp][0][0][0], &sW[warp][1][0][0],
-                                                 &sR[warp][0][0][0], sT[warp], lane, Xi);
-    // each warp's slice staging area (2 NWIN kSlots floats) holds its [NWIN][32] row-half doubles
-    static_assert(2 * NWIN * kSlots >= 2 * NWIN * 32, "row-half staging fits the slice area");
-    write_tile<NWIN>(p, task.x, task.y, active, Xi, reinterpret_cast<double*>(&sW[0][0][0][0]), NWIN * kSlots, rows,
-                     warp, lane);
+        active = chosen_xi<NWIN, N00, N22, SPEC>(p, task.x, task.y, sS[warp], sT[warp], lane, Xi);
+    // each warp's slices hold its [NWIN][32] row-half doubles
+    static_assert(sizeof(sS[0]) >= NWIN * 32 * sizeof(double) && sizeof(sS[0]) % sizeof(double) == 0, "they fit");
+    write_tile<NWIN>(p, task.x, task.y, active, Xi, reinterpret_cast<double*>(sS), (int)(sizeof(sS[0]) / sizeof(double)),
+                     rows, warp, lane);
 }
 
 // families a compile-time window set needs
@@ -708,6 +746,10 @@ inline cudaError_t launch_cfg(const CouplingParams& p, bool n00, bool n22, cudaS
 {
     const int threads = kWarpsPerBlock * 32;
     const unsigned blocks = (unsigned)((p.ntasks + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    const dim3 sgrid((unsigned)((slice_count(p.lmax) + 7) / 8), (unsigned)p.nwin);
+    if (p.src[0]) k_slices<NWIN, true><<<sgrid, 256, 0, s>>>(p);
+    else k_slices<NWIN, false><<<sgrid, 256, 0, s>>>(p);
+    if (cudaError_t e = cudaGetLastError()) return e;
     if constexpr (SPEC != 0) {
         constexpr bool a = spec_needs(SPEC, NWIN, true), b = spec_needs(SPEC, NWIN, false);
         (void)n00;

@@ -36,7 +36,7 @@ enum Epilogue : int { EPI_MCM = 0, EPI_XI = 1, EPI_COV = 2 };
 
 struct WinDesc {
     const double* wW;  // padded (2 l3 + 1) W[l3], length wlen >= 2 lmax + 2
-    const int2* bf;    // the same values split as (float mantissa bits, int exponent) for the chosen kernel
+    const int2* bf;    // the same values split as (float mantissa bits, int exponent): what slices are made of
     int product;
     int parity;
 };
@@ -60,10 +60,14 @@ struct CouplingParams {
     long long ldo;
     int wlen;  // length of the padded window arrays
     int nw;    // their entries at l3 >= nw are zero
+    // chosen kernel: the windows themselves (device pointers, nw entries), for launches that prepare the
+    // rows win[k].wW with their slices and leave win[k].bf unset; src[0] null otherwise
+    const double* src[kMaxWin];
     int cov_kind;
     const double* S[4];  // covariance signal spectra (length >= lmax + 1), reference argument order
     const double* R[4];  // covariance noise ratios
     HalfTable half;      // the plain kernel's factors (unset for the chosen kernel)
+    unsigned char* slices;  // the chosen kernel's table of window slices (slice_table_bytes of scratch)
 };
 
 // One window of a batch: user spectrum -> padded (2l+1)W row and its split copy.
@@ -92,7 +96,17 @@ int batch_blocks_per_sm(int nwin);
 int chosen_batch_template(const CouplingParams& p, int nwin);  // compile-time slot set of a batch group (0: none fits)
 cudaError_t launch_prep_windows(const WinPrep* list, int n, int max_wlen, cudaStream_t s);
 cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s);
+// Two launches: the table of window slices into p.slices (16-byte aligned), then the coupling kernel.
 cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s);
+size_t slice_table_bytes(const CouplingParams& p);
+// Smaller lmax in a batch: no table, each warp makes its few slices itself.  Then a table holds more slices than are
+// read: 2000 problems up to lmax 32 took 158 us without and 224 with tables, 64 of lmax 96-128 167 and 169,
+// 256 of lmax 128-200 1252 and 1232.
+constexpr int kSliceMinLmax = 128;
+// The slice tables of a batch's groups (NWIN = 4 or 8 as for launch_batch_chosen), each into its group's
+// own p.slices of batch_slice_bytes(lmax, nwin).
+cudaError_t launch_batch_slices(const CouplingParams* groups, int ngroups, int max_lmax, int nwin, cudaStream_t s);
+size_t batch_slice_bytes(int lmax, int nwin);
 // K windows of nW entries (device pointers in a host array) into padded rows wW + k wlen of (2l+1) W[l]
 // and, when bf is given, their split copies bf + k wlen, one launch per kSetWindows windows.
 constexpr int kSetWindows = 64;

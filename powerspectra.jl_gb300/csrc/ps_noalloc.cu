@@ -9,8 +9,8 @@
 // runs with PS_MODE_CHOSEN) with its scratch memory taken from a fixed array
 // that lives in the library's device image instead of from cudaMalloc.
 //
-// The scratch holds the padded windows, their split (mantissa, exponent) copies
-// and the warp task list.  Every call rewrites all of it before use, so nothing
+// The scratch holds the padded windows, the table of their slices and the warp
+// task list.  Every call rewrites all of it before use, so nothing
 // has to start at zero, but every call on a device shares this one array:
 // calls whose GPU work overlaps (on different streams or threads) race.
 #include "ps_internal.cuh"
@@ -29,12 +29,13 @@ constexpr int kNoAllocMaxWlen = 2 * kNoAllocMaxLmax + 2;
 constexpr long long kNoAllocMaxTasks = ps_tiles::task_count(0, kNoAllocMaxLmax);
 static_assert(kNoAllocMaxTasks == 264192, "4 tasks per tile, 66048 tiles at lmax 4095");
 
-// windows: 4 x wlen doubles, split copies: 4 x wlen int2, tasks: int2 each
+// windows: 4 x wlen doubles, tasks: int2 each, slices
 constexpr size_t kWinBytes = 4ull * kNoAllocMaxWlen * sizeof(double);
-constexpr size_t kBfBytes = 4ull * kNoAllocMaxWlen * sizeof(int2);
 constexpr size_t kTaskBytes = (size_t)kNoAllocMaxTasks * sizeof(int2);
-constexpr size_t kScratchBytes = kWinBytes + kBfBytes + kTaskBytes;  // 2.6 MB
-static_assert(kWinBytes % 256 == 0 && kBfBytes % 256 == 0, "each scratch region starts 256-byte aligned");
+constexpr size_t kSliceBytes = 1040ull * (2 * kNoAllocMaxLmax + 34);  // the slices of 4 windows (checked per call)
+constexpr size_t kScratchBytes = kWinBytes + kTaskBytes + kSliceBytes;  // 10.9 MB
+static_assert(kWinBytes % 256 == 0 && kTaskBytes % 256 == 0,
+              "each scratch region starts 256-byte aligned");
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -106,8 +107,7 @@ extern "C" int ps_mcm_multi_device_noalloc(unsigned cases, const double* const d
     unsigned char* base = (unsigned char*)scratch_address(dev, s);
     if (!base) return PS_ERR_CUDA;  // no lookup yet on this device (first call made during capture) or CUDA error
     double* win = (double*)base;
-    int2* bf = (int2*)(base + kWinBytes);
-    int2* tasks = (int2*)(base + kWinBytes + kBfBytes);
+    int2* tasks = (int2*)(base + kWinBytes);
 
     ps::CouplingParams p;
     memset(&p, 0, sizeof(p));
@@ -119,14 +119,11 @@ extern "C" int ps_mcm_multi_device_noalloc(unsigned cases, const double* const d
     const long long nuse = nW < (int64_t)(2 * lmax + 1) ? nW : (int64_t)(2 * lmax + 1);
     p.nw = (int)nuse;
     int K = 0;
-    const double* src[4];
     for (int sp = 0; sp < 4; ++sp) {
         if (!(cases & (1u << sp))) continue;
         double* w = win + (size_t)K * p.wlen;
-        int2* b = bf + (size_t)K * p.wlen;
-        src[K] = dW[sp];
+        p.src[K] = dW[sp];
         p.win[K].wW = w;
-        p.win[K].bf = b;
         switch (sp) {
         case PS_SPIN_00: p.win[K].product = ps::PROD_00_00; p.win[K].parity = ps::PAR_ALL; break;
         case PS_SPIN_02: p.win[K].product = ps::PROD_00_22; p.win[K].parity = ps::PAR_EVEN; break;
@@ -137,13 +134,14 @@ extern "C" int ps_mcm_multi_device_noalloc(unsigned cases, const double* const d
         ++K;
     }
     p.nwin = K;
-    if (ps::launch_prep_set(src, K, nuse, p.wlen, win, bf, s) != cudaSuccess) return PS_ERR_CUDA;
     const ps_tiles::Geometry G = ps_tiles::geometry(lmin, lmax);
     const int groups = 8 * G.nb - G.glo;
     k_fill_tiles<<<(groups + 255) / 256, 256, 0, s>>>(tasks, lmin, lmax);
     if (cudaGetLastError() != cudaSuccess) return PS_ERR_CUDA;
     p.tasks = tasks;
     p.ntasks = (int)ntasks;
+    if (ps::slice_table_bytes(p) > kSliceBytes) return PS_ERR_ARG;  // 4 windows at lmax 4095 fill it
+    p.slices = base + kWinBytes + kTaskBytes;
     if (ps::launch_chosen(p, s) != cudaSuccess) return PS_ERR_CUDA;
     return PS_OK;
 }
