@@ -97,7 +97,12 @@ int ps_mcm(ps_ctx *ctx, int spin, const double *W, int64_t nW, int lmin, int lma
  * separately for :EE_BB / :EB_BE, src/modecoupling.jl:210-223). */
 int ps_mcm_multi(ps_ctx *ctx, unsigned cases, const double *const W[4], int64_t nW, int lmin, int lmax, int mode,
                  double *const M[4], int64_t ldm);
-/* Same with device pointers, enqueued on the context stream (no host copies). */
+/* The 2 x 2 block matrices of the spin-2 pairs (src/modecoupling.jl:210-245) from one ++/-- pass, written
+ * whole: EE_BB = [++ --; -- ++] and EB_BE = [++ -(--); -(--) ++], host, column-major, 2 n x 2 n with
+ * n = lmax - lmin + 1 and leading dimension ld >= 2 n.  Either may be NULL, not both. */
+int ps_mcm_blocks(ps_ctx *ctx, const double *W, int64_t nW, int lmin, int lmax, int mode, double *EE_BB,
+                  double *EB_BE, int64_t ld);
+/* ps_mcm_multi with device pointers, enqueued on the context stream (no host copies). */
 int ps_mcm_multi_device(ps_ctx *ctx, unsigned cases, const double *const dW[4], int64_t nW, int lmin, int lmax,
                         int mode, double *const dM[4], int64_t ldm);
 

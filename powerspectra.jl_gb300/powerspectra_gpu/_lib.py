@@ -24,7 +24,7 @@ COV_NRATIOS = {0: 4, 1: 4, 2: 2, 3: 2, 4: 2, 5: 2, 6: 0}
 MODES = {"plain": PS_MODE_PLAIN_FP64, "fp64": PS_MODE_PLAIN_FP64, "chosen": PS_MODE_CHOSEN}
 
 # every symbol declared in include/powerspectra_gpu.h
-EXPORTS = ("ps_create", "ps_destroy", "ps_last_error", "ps_set_stream", "ps_synchronize", "ps_mcm", "ps_mcm_multi",
+EXPORTS = ("ps_create", "ps_destroy", "ps_last_error", "ps_set_stream", "ps_synchronize", "ps_mcm", "ps_mcm_multi", "ps_mcm_blocks",
            "ps_mcm_multi_device", "ps_xi", "ps_coupledcov", "ps_coupledcov_device", "ps_coupledcov_set_device", "ps_mcm_set_device",
            "ps_batch_prepare", "ps_batch_run", "ps_batch_graph_launch", "ps_batch_autotune", "ps_last_kernel_ms",
            "ps_launch_count", "ps_probe_fma_peak", "ps_mcm_multi_device_noalloc", "ps_decouple_covmat", "ps_solve",
@@ -93,6 +93,8 @@ def load(path=None):
         lib.ps_mcm.restype = ci
         lib.ps_mcm_multi.argtypes = [vp, ctypes.c_uint, _DPP, i64, ci, ci, ci, _DPP, i64]
         lib.ps_mcm_multi.restype = ci
+        lib.ps_mcm_blocks.argtypes = [vp, _DP, i64, ci, ci, ci, _DP, _DP, i64]
+        lib.ps_mcm_blocks.restype = ci
         lib.ps_mcm_multi_device.argtypes = [vp, ctypes.c_uint, _DPP, i64, ci, ci, ci, _DPP, i64]
         lib.ps_mcm_multi_device.restype = ci
         lib.ps_xi.argtypes = [vp, ci, ci, _DPP, ci, i64, ci, ci, ci, _DPP, i64]
@@ -242,6 +244,15 @@ class Context:
         self.check(self.lib.ps_mcm_multi(self.handle, cases, dptr_array(wl), nW or 1, lmin, lmax, mode_code(mode),
                                          dptr_array(ml), n))
         return {s: ml[s] for s in Ws}
+
+    def mcm_blocks(self, W, lmin, lmax, mode="plain", ee_bb=True, eb_be=False):
+        """The 2n x 2n matrices [++ --; -- ++] and [++ -(--); -(--) ++] (None where not asked for)."""
+        W = np.ascontiguousarray(W, dtype=np.float64)
+        n = 2 * max(lmax - lmin + 1, 0)
+        out = [np.empty((n, n), dtype=np.float64, order="F") if want else None for want in (ee_bb, eb_be)]
+        self.check(self.lib.ps_mcm_blocks(self.handle, dptr(W), len(W), lmin, lmax, mode_code(mode),
+                                          *(None if M is None else dptr(M) for M in out), n))
+        return out
 
     def mcm_multi_device(self, dWs, nW, lmin, lmax, dMs, ldm, mode="plain"):
         """Device-pointer variant: dWs / dMs map spin -> device address (int)."""

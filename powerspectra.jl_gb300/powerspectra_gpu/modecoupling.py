@@ -80,6 +80,13 @@ def _spectrum(W, lmax):
     return np.ascontiguousarray(W[:lmax + 1]), lmax  # Vij = alm2cl(...)[1:(lmax+1)], src/modecoupling.jl:197
 
 
+def _blocks(specs, V, lmin, lmax, mode, ctx):
+    """[++ --; -- ++] for EE_BB, [++ -(--); -(--) ++] for EB_BE, from one pass."""
+    ax = range(lmin, lmax + 1)
+    Ms = _ctx(ctx).mcm_blocks(V, lmin, lmax, mode=mode, ee_bb="EE_BB" in specs, eb_be="EB_BE" in specs)
+    return [BlockSpectralMatrix(M, (ax, ax), (ax, ax)) for M in Ms if M is not None]
+
+
 def mcm(spec, W, lmin=0, lmax=None, mode="plain", ctx=None):
     """Mode-coupling matrix for `spec` from the mask cross-spectrum W.
 
@@ -92,11 +99,7 @@ def mcm(spec, W, lmin=0, lmax=None, mode="plain", ctx=None):
         if tuple(spec) != ("EE_BB", "EB_BE"):
             return None  # the reference's tuple method returns nothing for other tuples
         V, lmax = _spectrum(W, lmax)
-        Mpp, Mmm = spectralzeros(range(lmin, lmax + 1), range(lmin, lmax + 1)), \
-            spectralzeros(range(lmin, lmax + 1), range(lmin, lmax + 1))
-        inner_mcmPPMM(Mpp, Mmm, V, mode, ctx)
-        return (BlockSpectralMatrix.hvcat([[Mpp, Mmm], [Mmm, Mpp]]),
-                BlockSpectralMatrix.hvcat([[Mpp, -Mmm], [-Mmm, Mpp]]))
+        return tuple(_blocks(spec, V, lmin, lmax, mode, ctx))
     V, lmax = _spectrum(W, lmax)
     ax = range(lmin, lmax + 1)
     if spec in SPEC_00:
@@ -108,9 +111,5 @@ def mcm(spec, W, lmin=0, lmax=None, mode="plain", ctx=None):
     if spec in SPEC_MM:
         return inner_mcmMM(spectralzeros(ax, ax), V, mode, ctx)
     if spec in ("EE_BB", "EB_BE"):
-        Mpp, Mmm = spectralzeros(ax, ax), spectralzeros(ax, ax)
-        inner_mcmPPMM(Mpp, Mmm, V, mode, ctx)
-        if spec == "EE_BB":
-            return BlockSpectralMatrix.hvcat([[Mpp, Mmm], [Mmm, Mpp]])
-        return BlockSpectralMatrix.hvcat([[Mpp, -Mmm], [-Mmm, Mpp]])
+        return _blocks((spec,), V, lmin, lmax, mode, ctx)[0]
     raise PowerSpectraArgumentError(_lib.PS_ERR_ARG, "%s not a valid spectrum." % (spec,))  # :225
