@@ -57,6 +57,10 @@ struct ps_ctx {
     int2* d_bf = nullptr;  // split (mantissa, exponent) windows for the chosen kernel
     size_t bf_cap = 0;
     unsigned char* d_slices = nullptr;  // its table of window slices, one launch at a time
+    // the chosen kernels' square-root ratios, for lmax up to coef_lmax
+    unsigned char* d_coef = nullptr;
+    size_t coef_cap = 0;
+    int coef_lmax = -1;
     size_t slices_cap = 0;
     double* d_alm = nullptr;  // harmonic coefficients copied in by ps_window_W (2 doubles each)
     size_t alm_cap = 0;
@@ -90,6 +94,7 @@ struct ps_ctx {
         std::vector<ps::CouplingParams> host_groups;
         int2* d_tasks = nullptr;
         unsigned char* d_slices = nullptr;  // the groups' tables of window slices
+        unsigned char* d_coef = nullptr;    // the square-root ratios of all of them
         int ngroups = 0, max_slice_lmax = 0;  // the largest lmax with a table (0: no tables)
         // tensor-core launches (the problems' TT slots and ++/-- slots when there are
         // mma_min_slots of them), enqueued before the CUDA-core part,
@@ -366,6 +371,27 @@ void cov_window_spec(int kind, int k, int* product, int* parity)
 // Launch the coupling kernel with event timing on the context stream.  A call
 // that launches several groups passes first/last so that the two events
 // bracket all of its coupling kernels (ps_last_kernel_ms).
+static int ensure_bytes(ps_ctx* c, unsigned char** p, size_t* cap, size_t need);
+
+// The chosen kernels' square-root ratios for rows up to lmax, kept by the context and replaced by larger ones.
+// None beyond kCoefMaxLmax or where there is no room: the kernels then make them chunk by chunk.
+static const int kCoefMaxLmax = 4096;
+static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
+{
+    *out = ps::CoefRows{};
+    if (lmax > kCoefMaxLmax) return PS_OK;
+    if (c->coef_lmax < lmax) {
+        c->coef_lmax = -1;
+        if (ensure_bytes(c, &c->d_coef, &c->coef_cap, ps::coef_bytes(lmax))) return PS_OK;
+        PS_CUDA(c, ps::launch_coef((float4*)c->d_coef, lmax, c->stream));
+        PS_CUDA(c, cudaStreamSynchronize(c->stream));  // later calls may be on other streams
+        c->launches++;
+        c->coef_lmax = lmax;
+    }
+    *out = ps::coef_rows((const float4*)c->d_coef, c->coef_lmax);
+    return PS_OK;
+}
+
 static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first = true, bool last = true)
 {
     int st = ensure_tiles(c, p.lmin, p.lmax);
@@ -375,6 +401,7 @@ static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first =
     if (mode == PS_MODE_CHOSEN) {
         if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, ps::slice_table_bytes(p)))) return st;
         p.slices = c->d_slices;
+        if (ps::reads_coef(p) && (st = ensure_coef(c, p.lmax, &p.coef))) return st;
     } else if ((st = ensure_half(c, p.lmax, &p.half))) {
         return st;
     }
@@ -469,6 +496,7 @@ static void batch_release(ps_ctx* c)
     cudaFree(b.d_bf);
     cudaFree(b.d_tasks);
     cudaFree(b.d_slices);
+    cudaFree(b.d_coef);
     cudaFree(b.d_mtiles);
     cudaFree(b.d_btab);
     b = ps_ctx::Batch();
@@ -635,6 +663,7 @@ void ps_destroy(ps_ctx* c)
     cudaFree(c->d_probe);
     cudaFree(c->d_bf);
     cudaFree(c->d_slices);
+    cudaFree(c->d_coef);
     cudaFree(c->d_alm);
     cudaFree(c->d_part);
     cudaFree(c->d_qp);
@@ -1447,6 +1476,16 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         groups[g].slices = b.d_slices + slice_at[g];
         b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
     }
+    // and one table of the square-root ratios (the batch's own: a context's may be replaced by a larger one)
+    int max_lmax = 0;
+    for (const auto& g : groups) max_lmax = std::max(max_lmax, g.lmax);
+    if (!groups.empty() && max_lmax <= kCoefMaxLmax) {
+        size_t cap = 0;
+        if (ensure_bytes(c, &b.d_coef, &cap, ps::coef_bytes(max_lmax)) == PS_OK) {
+            PS_CUDA(c, ps::launch_coef((float4*)b.d_coef, max_lmax, c->stream));
+            for (auto& g : groups) g.coef = ps::coef_rows((const float4*)b.d_coef, max_lmax);
+        }
+    }
     b.ngroups = (int)groups.size();
     // items of one kernel body together (warps of an SM then share their
     // instruction stream), longest first within each body
@@ -1538,6 +1577,7 @@ static int batch_enqueue(ps_ctx* c, cudaStream_t s)
         bp.groups = b.d_groups;
         bp.items = b.d_items;
         bp.nitems = b.nitems;
+        bp.coef = b.d_coef != nullptr;
         bp.counter = b.d_counter;
         if (b.max_slice_lmax)
             PS_CUDA(c, ps::launch_batch_slices(b.d_groups, b.ngroups, b.max_slice_lmax, b.group_slots, s));

@@ -24,7 +24,7 @@ struct BatchSets<8> {
     static constexpr uint32_t s[6] = {rep(W00, 8), S_PPMM4, S_MCM8, rep(WPP, 8), rep(WMM, 8), rep(W02, 8)};
 };
 
-template <int NWIN>
+template <int NWIN, bool TAB>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 3) k_batch_chosen(const BatchParams bp)
 {
     __shared__ Slice<NWIN> sS[kWarpsPerBlock][2][2];
@@ -32,8 +32,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 3) k_batc
     // loops, so they live in shared memory rather than behind global loads
     __shared__ CouplingParams sG[kWarpsPerBlock];
     __shared__ CoefTab sT[kWarpsPerBlock];
+    __shared__ CoefStageIf<TAB> sC[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+    CoefStage* const st = stage_of<TAB>(sC[warp]);
     int cur = -1;
     for (;;) {
         int it = 0;
@@ -53,12 +55,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 3) k_batc
         for (int q = 0; q < ntask; ++q) {
             const int l2_0 = item.z + 32 * q;
             switch (tmpl) {  // the group's compile-time slot set (prepare never emits others)
-            case 1: chosen_task<NWIN, true, false, BatchSets<NWIN>::s[0]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
-            case 2: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[1]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
-            case 3: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[2]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
-            case 4: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[3]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
-            case 5: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[4]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
-            case 6: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[5]>(g, item.y, l2_0, sS[warp], sT[warp], lane); break;
+            case 1: chosen_task<NWIN, true, false, BatchSets<NWIN>::s[0], false>(g, item.y, l2_0, sS[warp], sT[warp], st, lane); break;
+            case 2: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[1], TAB>(g, item.y, l2_0, sS[warp], sT[warp], st, lane); break;
+            case 3: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[2], TAB>(g, item.y, l2_0, sS[warp], sT[warp], st, lane); break;
+            case 4: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[3], TAB>(g, item.y, l2_0, sS[warp], sT[warp], st, lane); break;
+            case 5: chosen_task<NWIN, false, true, BatchSets<NWIN>::s[4], TAB>(g, item.y, l2_0, sS[warp], sT[warp], st, lane); break;
+            case 6: chosen_task<NWIN, true, true, BatchSets<NWIN>::s[5], TAB>(g, item.y, l2_0, sS[warp], sT[warp], st, lane); break;
             default: break;  // prepare rejects groups without a body
             }
             __syncwarp();
@@ -102,17 +104,19 @@ cudaError_t launch_batch_chosen(const BatchParams& bp, int blocks, int nwin, cud
 {
     if (bp.nitems <= 0) return cudaSuccess;
     if (nwin > 4)
-        k_batch_chosen<8><<<blocks, kWarpsPerBlock * 32, 0, s>>>(bp);
+        k_batch_chosen<8, false><<<blocks, kWarpsPerBlock * 32, 0, s>>>(bp);
+    else if (bp.coef)
+        k_batch_chosen<4, true><<<blocks, kWarpsPerBlock * 32, 0, s>>>(bp);
     else
-        k_batch_chosen<4><<<blocks, kWarpsPerBlock * 32, 0, s>>>(bp);
+        k_batch_chosen<4, false><<<blocks, kWarpsPerBlock * 32, 0, s>>>(bp);
     return cudaGetLastError();
 }
 
 int batch_blocks_per_sm(int nwin)
 {
     int n = 0;
-    cudaError_t e = nwin > 4 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_chosen<8>, kWarpsPerBlock * 32, 0)
-                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_chosen<4>, kWarpsPerBlock * 32, 0);
+    cudaError_t e = nwin > 4 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_chosen<8, false>, kWarpsPerBlock * 32, 0)
+                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_chosen<4, true>, kWarpsPerBlock * 32, 0);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return 1;

@@ -15,9 +15,10 @@ namespace {
 struct Inst {
     uint32_t spec;
     int n;  // slots
+    bool coef;  // reads the table of square-root ratios
     cudaError_t (*launch)(const CouplingParams&, bool, bool, cudaStream_t);
 };
-#define PS_INST(n, spec) Inst{spec, n, launch_cfg<n, spec>}
+#define PS_INST(n, spec) Inst{spec, n, kHasCoef<n, spec>, launch_cfg<n, spec>}
 const Inst kInst[] = {
     PS_INST(1, W00),          PS_INST(1, W02),          PS_INST(1, WPP),          PS_INST(1, WMM),
     PS_INST(2, S_PPMM),       PS_INST(4, rep(W00, 4)),  PS_INST(4, S_PPMM2),      PS_INST(4, S_MCM4),
@@ -37,10 +38,54 @@ const Inst* find_inst(const CouplingParams& p, uint32_t spec)  // null: launch_c
 
 }  // namespace
 
+// Below lmax 512 the copies of a warp's first chunk wait longer than its square roots take (TT, TE and ++/--
+// together, without and with the table: lmax 95 55.8 and 55.6 us, ++ alone 38.0 and 43.3; 383 83.7 and 84.8; 767
+// 268.0 and 258.5).
+bool reads_coef(const CouplingParams& p)
+{
+    const Inst* i = find_inst(p, spec_of(p));
+    return p.lmax >= 512 && i && i->coef;
+}
+
 size_t slice_table_bytes(const CouplingParams& p)
 {
     const Inst* i = find_inst(p, spec_of(p));
     return slice_bytes(i ? i->n : 8) * (size_t)slice_count(p.lmax);
+}
+
+namespace {
+
+// One row of the table per blockIdx.y.
+__global__ void __launch_bounds__(256) k_coef(float4* __restrict__ t, int lmax)
+{
+    const int l1 = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x;
+    const long long n = coef_row(lmax, lmax + 1), row = coef_row(lmax, l1);
+    const float h = (float)(2 * l1 + 1);
+    auto put = [](float4* at, ff rho, ff r) { *at = make_float4(rho.h, rho.l, r.h, r.l); };
+    if (i < 2 * lmax + 160 - l1) {
+        ff rho = ff_make(0.0f), r = rho;
+        const float a = (float)(i - 62);
+        if (a >= 0.0f) sqrt_ratio(two_prod(a, a + h), two_prod(a + 1.0f, a + h + 1.0f), rho, r);
+        put(t + row + i, ff_neg(rho), r);
+        const float b = (float)(i + l1 - 92);
+        rho = r = ff_make(0.0f);
+        if (b > 0.0f) sqrt_ratio(two_prod(b + 1.0f, b + h + 1.0f), two_prod(b, b + h), rho, r);
+        put(t + n + row + i, ff_neg(rho), r);
+    }
+    if (i < l1 || (l1 == lmax && i < l1 + 32)) {
+        ff rho = ff_make(0.0f), r = rho;
+        const float x = (float)i;
+        if (i < l1) sqrt_ratio(two_prod(x, h - x), two_prod(x + 1.0f, h - 1.0f - x), rho, r);
+        put(t + 2 * n + coef_row_g(l1) + i, rho, r);
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_coef(float4* t, int lmax, cudaStream_t s)
+{
+    k_coef<<<dim3((unsigned)((2 * lmax + 160 + 255) / 256), (unsigned)(lmax + 1)), 256, 0, s>>>(t, lmax);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s)

@@ -456,6 +456,64 @@ __device__ __forceinline__ void build_tables(CoefTab& tb, int t0, int T, int l1,
     }
 }
 
+// With a table of all rows (CoefRows) a chunk's entries come from there: those of lane i's steps depend on
+// l1 and on 2 (l2_0 - l1) + u or 2 l2_0 + v alone, so they are the same numbers.  A chunk then costs 3 copies and
+// the move instead of 5 square roots per lane: all spin cases at lmax 3071 16.98 -> 16.28 ms, 256 small problems
+// 18.70 -> 18.12.  The (0 0 0) family alone makes two roots per chunk only, and reads every other entry
+// (TT at lmax 767 120 us without and 125 with the table): it has none.
+struct CoefStage {  // what the next chunk adds
+    ffpair g[2][32];  // its G entries (two chunks alternate)
+    ffpair f[32], b[32];
+};
+template <bool TAB>
+struct CoefStageIf : CoefStage {};
+template <>
+struct CoefStageIf<false> {};
+template <bool TAB>
+__device__ __forceinline__ CoefStage* stage_of(CoefStageIf<TAB>& s)
+{
+    if constexpr (TAB) return &s;
+    else return nullptr;
+}
+__device__ __forceinline__ void copy_async(ffpair* dst, const float4* src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
+struct CoefSrc {
+    const float4 *f, *b, *g;  // entries u = 0, v = -31 and t = 0 of the task
+};
+__device__ __forceinline__ CoefSrc coef_src(const CoefRows& t, int l1, int l2_0)
+{
+    const long long row = coef_row(t.lmax, l1);
+    return CoefSrc{t.f + row + 62 + 2 * (l2_0 - l1), t.b + row + 92 - l1 + 2 * l2_0 - (kChunk - 1), t.g + coef_row_g(l1)};
+}
+__device__ __forceinline__ void fetch_first(CoefTab& tb, CoefStage& st, const CoefSrc& c, int lane)
+{
+#pragma unroll
+    for (int q = 0; q < 2 * kFEnt / 32; ++q) {
+        const int e = lane + 32 * q;
+        copy_async(&tb.fF[e & 1][e >> 1], c.f + e);
+        copy_async(&tb.fB[e & 1][e >> 1], c.b + e);
+    }
+    copy_async(&st.g[0][lane], c.g + lane);
+}
+__device__ __forceinline__ void fetch_next(CoefStage& st, const CoefSrc& c, int t0, int lane)  // for the chunk at t0
+{
+    copy_async(&st.f[lane], c.f + t0 + 64 + lane);
+    copy_async(&st.b[lane], c.b - t0 + lane);
+    copy_async(&st.g[(t0 / kChunk) & 1][lane], c.g + t0 + lane);
+}
+__device__ __forceinline__ void place_next(CoefTab& tb, const CoefStage& st, int lane)
+{
+    move_row(tb.fF[0], lane + 16, lane);
+    move_row(tb.fF[1], lane + 16, lane);
+    move_row(tb.fB[0], lane, lane + 16);
+    move_row(tb.fB[1], lane, lane + 16);
+    tb.fF[lane & 1][32 + (lane >> 1)] = st.f[lane];
+    tb.fB[lane & 1][lane >> 1] = st.b[lane];
+}
+
 // One table-driven step: g(next) = 4 (2j+1) r g(cur) - rho g(prev) for g(t) = (-1)^t f(t), with -rho
 // from the tables: no negations (measured against f itself, same bits: all spin cases at lmax 3071
 // 18.80 -> 18.47 ms, TT at lmax 767 109.3 -> 107.7 us).  With
@@ -500,9 +558,9 @@ __device__ __forceinline__ void tab_bwd(Sweep& s, const CoefTab& tb, int st, int
 // The Xi of pair (l1, l2_0 + lane) into Xi[]; returns whether the lane holds a
 // pair to write (l1 <= l2 <= lmax).  Lanes outside clamp l2 into [l1, lmax] and
 // compute values nobody writes.
-template <int NWIN, bool N00, bool N22, uint32_t SPEC, bool OWN = false>
+template <int NWIN, bool N00, bool N22, uint32_t SPEC, bool TAB, bool OWN = false>
 __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1, const int l2_0, Slice<NWIN> (*sl)[2],
-                                          CoefTab& tb, const int lane, double* Xi)
+                                          CoefTab& tb, CoefStage* st, const int lane, double* Xi)
 {
     const int l2raw = l2_0 + lane;
     const bool active = l2raw >= l1 && l2raw <= p.lmax;
@@ -513,6 +571,7 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
     const bool fam22 = N22 && (l1 >= 2);
     const int jmin0 = l2_0 - l1, jmax0 = l2_0 + l1;  // lane 0's ends: lane i reads slot i + step
     const WinCfg<NWIN> wc = win_cfg<NWIN, SPEC>(p);
+    static_assert(N22 || !TAB, "the (0 0 0) family alone has no table");
 
     if (T == 0) {
         xi_single_term(p, l2, Xi);
@@ -540,17 +599,21 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
 
     get_slice<NWIN, OWN>(p, sl[0][0], jmin0, lane);
     get_slice<NWIN, OWN>(p, sl[0][1], jmax0 - kChunk + 1, lane);
+    const CoefSrc cs = TAB ? coef_src(p.coef, l1, l2_0) : CoefSrc{};
+    if constexpr (TAB) fetch_first(tb, *st, cs, lane);
     fetch_commit();
-    init_f_tables<N22>(tb, l1, l2_0, lane);
+    if constexpr (!TAB) init_f_tables<N22>(tb, l1, l2_0, lane);
     for (int t0 = 0; t0 < T; t0 += kChunk) {
         const int cur = (t0 / kChunk) & 1;
         const float *sF = sl[cur][0].v, *sB = sl[cur][1].v;
         fetch_wait_all();
-        build_tables<N22>(tb, t0, T, l1, l2_0, lane);
+        if constexpr (!TAB) build_tables<N22>(tb, t0, T, l1, l2_0, lane);
+        else if (t0 > 0) place_next(tb, *st, lane);
         __syncwarp();
         if (t0 + kChunk < T) {  // the next chunk's slices land while this one computes
             get_slice<NWIN, OWN>(p, sl[cur ^ 1][0], jmin0 + t0 + kChunk, lane);
             get_slice<NWIN, OWN>(p, sl[cur ^ 1][1], jmax0 - t0 - 2 * kChunk + 1, lane);
+            if constexpr (TAB) fetch_next(*st, cs, t0 + kChunk, lane);
         }
         fetch_commit();
         float cF[NWIN], cB[NWIN];
@@ -566,7 +629,7 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
         int s = 0;
         if constexpr (N22) {
             constexpr float kDw = WS4 ? 8.0f : 2.0f;
-            const ffpair *pg = tb.g, *pf = tb.fF[0] + lane, *pb = tb.fB[0] + lane + (kChunk / 2 - 1);
+            const ffpair *pg = TAB ? st->g[cur] : tb.g, *pf = tb.fF[0] + lane, *pb = tb.fB[0] + lane + (kChunk / 2 - 1);
             const float *wF = sF + lane * kSlot, *wB = sB + (lane + kChunk - 1) * kSlot;
             for (; s + 1 < steps; s += 2) {
                 sweep_acc<NWIN, N00, N22, SPEC, true>(wc, F, wF, cF, n0F, n2F);
@@ -674,7 +737,8 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
 
     // match, normalise, sign (FP64)
     const double lam0 = N00 ? g0s / h0s : 0.0;
-    const double lam2 = fam22 ? (gm0 * hm0 + gm1 * hm1) / (hm0 * hm0 + hm1 * hm1) : 0.0;
+    // the sums in one order, so that every form of the kernel gives the same bits
+    const double lam2 = fam22 ? fma(gm1, hm1, gm0 * hm0) / fma(hm1, hm1, hm0 * hm0) : 0.0;
     const double N0 = fma(lam0 * lam0, BN0, FN0);
     const double N2 = fma(lam2 * lam2, BN2, FN2);
     const double inv0 = N00 ? kInv4Pi / N0 : 0.0;
@@ -701,20 +765,21 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
 
 // One warp task with its own writes (the persistent batch kernel, whose items
 // hold l2_0 >= l1).
-template <int NWIN, bool N00, bool N22, uint32_t SPEC>
+template <int NWIN, bool N00, bool N22, uint32_t SPEC, bool TAB>
 __device__ __forceinline__ void chosen_task(const CouplingParams& p, const int l1, const int l2_0, Slice<NWIN> (*sl)[2],
-                                            CoefTab& tb, const int lane)
+                                            CoefTab& tb, CoefStage* st, const int lane)
 {
     double Xi[kMaxWin];
-    if (chosen_xi<NWIN, N00, N22, SPEC, true>(p, l1, l2_0, sl, tb, lane, Xi)) write_pair(p, l1, l2_0 + lane, Xi);
+    if (chosen_xi<NWIN, N00, N22, SPEC, TAB, true>(p, l1, l2_0, sl, tb, st, lane, Xi)) write_pair(p, l1, l2_0 + lane, Xi);
 }
 
 
-template <int NWIN, bool N00, bool N22, uint32_t SPEC>
+template <int NWIN, bool N00, bool N22, uint32_t SPEC, bool TAB>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 4) k_coupling_chosen(const CouplingParams p)
 {
     __shared__ Slice<NWIN> sS[kWarpsPerBlock][2][2];
     __shared__ CoefTab sT[kWarpsPerBlock];
+    __shared__ CoefStageIf<TAB> sC[kWarpsPerBlock];
     __shared__ TileRows rows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the task list is tiled: kTileRows tasks per block, rows outside [lmin, lmax] as l1 = -1
@@ -723,7 +788,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 4) k_coup
     double Xi[kMaxWin];
     bool active = false;
     if (task.x >= 0)  // warp-uniform
-        active = chosen_xi<NWIN, N00, N22, SPEC>(p, task.x, task.y, sS[warp], sT[warp], lane, Xi);
+        active = chosen_xi<NWIN, N00, N22, SPEC, TAB>(p, task.x, task.y, sS[warp], sT[warp], stage_of<TAB>(sC[warp]), lane, Xi);
     // each warp's slices hold its [NWIN][32] row-half doubles
     static_assert(sizeof(sS[0]) >= NWIN * 32 * sizeof(double) && sizeof(sS[0]) % sizeof(double) == 0, "they fit");
     write_tile<NWIN>(p, task.x, task.y, active, Xi, reinterpret_cast<double*>(sS), (int)(sizeof(sS[0]) / sizeof(double)),
@@ -741,6 +806,10 @@ constexpr bool spec_needs(uint32_t spec, int nwin, bool fam00)
     return need;
 }
 
+// Lists with the (2 -2 0) family read the table of square-root ratios; with 8 slots the stage does not fit
+// beside the slices, and one TE window gains nothing (lmax 767 283 without and 287 us with it, 1500 1767 and 1762).
+template <int NWIN, uint32_t SPEC>
+constexpr bool kHasCoef = SPEC != 0 && NWIN <= 5 && spec_needs(SPEC, NWIN, false) && !(NWIN == 1 && SPEC == W02);
 template <int NWIN, uint32_t SPEC>
 inline cudaError_t launch_cfg(const CouplingParams& p, bool n00, bool n22, cudaStream_t s)
 {
@@ -754,14 +823,19 @@ inline cudaError_t launch_cfg(const CouplingParams& p, bool n00, bool n22, cudaS
         constexpr bool a = spec_needs(SPEC, NWIN, true), b = spec_needs(SPEC, NWIN, false);
         (void)n00;
         (void)n22;
-        k_coupling_chosen<NWIN, a, b, SPEC><<<blocks, threads, 0, s>>>(p);
+        if constexpr (kHasCoef<NWIN, SPEC>)
+            if (p.coef.f) {
+                k_coupling_chosen<NWIN, a, b, SPEC, true><<<blocks, threads, 0, s>>>(p);
+                return cudaGetLastError();
+            }
+        k_coupling_chosen<NWIN, a, b, SPEC, false><<<blocks, threads, 0, s>>>(p);
     } else {
         if (n00 && n22)
-            k_coupling_chosen<NWIN, true, true, 0><<<blocks, threads, 0, s>>>(p);
+            k_coupling_chosen<NWIN, true, true, 0, false><<<blocks, threads, 0, s>>>(p);
         else if (n22)
-            k_coupling_chosen<NWIN, false, true, 0><<<blocks, threads, 0, s>>>(p);
+            k_coupling_chosen<NWIN, false, true, 0, false><<<blocks, threads, 0, s>>>(p);
         else
-            k_coupling_chosen<NWIN, true, false, 0><<<blocks, threads, 0, s>>>(p);
+            k_coupling_chosen<NWIN, true, false, 0, false><<<blocks, threads, 0, s>>>(p);
     }
     return cudaGetLastError();
 }

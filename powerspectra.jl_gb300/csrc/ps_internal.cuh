@@ -49,6 +49,31 @@ struct HalfTable {
     int top;
 };
 
+// The square-root ratios of the chosen kernels' recurrences (chosen_xi), float-float pairs (rho, r) of 16
+// bytes, for every row l1 <= lmax.  With F(a) = a (a + 2 l1 + 1) and G(t) = t (2 l1 + 1 - t):
+//   f, entry a:  -sqrt(F(a) / F(a + 1)), 1 / sqrt(F(a + 1))   a = -62 .. 2 lmax - l1 + 94, zeros below a = 0
+//   b, entry a:  -sqrt(F(a + 1) / F(a)), 1 / sqrt(F(a))       a = l1 - 92 .. 2 lmax + 64, zeros up to a = 0
+//   g, entry t:   sqrt(G(t) / G(t + 1)), 1 / sqrt(G(t + 1))   t = 0 .. l1 - 1
+struct CoefRows {
+    const float4 *f, *b, *g;  // f null: no table
+    int lmax;                 // of the table: at least that of the launches that read it
+};
+__host__ __device__ constexpr long long coef_row(int lmax, int l1)  // first entry of row l1 in f and b
+{
+    return (long long)l1 * (2 * lmax + 160) - (long long)l1 * (l1 - 1) / 2;
+}
+__host__ __device__ constexpr long long coef_row_g(int l1) { return (long long)l1 * (l1 - 1) / 2; }
+// rows 0 .. lmax of f, then of b, then of g (a warp reads 32 entries at a time, past the last row's end)
+constexpr size_t coef_bytes(int lmax)
+{
+    return (size_t)(2 * coef_row(lmax, lmax + 1) + coef_row_g(lmax + 1) + 32) * sizeof(float4);
+}
+inline CoefRows coef_rows(const float4* t, int lmax)
+{
+    const long long n = coef_row(lmax, lmax + 1);
+    return CoefRows{t, t + n, t + 2 * n, lmax};
+}
+
 struct CouplingParams {
     int lmin, lmax;
     int nwin;
@@ -68,6 +93,7 @@ struct CouplingParams {
     const double* R[4];  // covariance noise ratios
     HalfTable half;      // the plain kernel's factors (unset for the chosen kernel)
     unsigned char* slices;  // the chosen kernel's table of window slices (slice_table_bytes of scratch)
+    CoefRows coef;          // the chosen kernel's square-root ratios, or none (it makes them itself)
 };
 
 // One window of a batch: user spectrum -> padded (2l+1)W row and its split copy.
@@ -86,6 +112,7 @@ struct BatchParams {
     const CouplingParams* groups;
     const int4* items;
     int nitems;
+    bool coef;  // the groups have a table of square-root ratios
     unsigned* counter;  // work-queue head, zeroed before every launch
 };
 
@@ -99,6 +126,9 @@ cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s);
 // Two launches: the table of window slices into p.slices (16-byte aligned), then the coupling kernel.
 cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s);
 size_t slice_table_bytes(const CouplingParams& p);
+// The table of square-root ratios (coef_bytes(lmax)), and whether launch_chosen reads one if p.coef has it.
+cudaError_t launch_coef(float4* t, int lmax, cudaStream_t s);
+bool reads_coef(const CouplingParams& p);
 // Smaller lmax in a batch: no table, each warp makes its few slices itself.  Then a table holds more slices than are
 // read: 2000 problems up to lmax 32 took 158 us without and 224 with tables, 64 of lmax 96-128 167 and 169,
 // 256 of lmax 128-200 1252 and 1232.
