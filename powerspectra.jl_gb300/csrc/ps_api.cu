@@ -408,8 +408,13 @@ static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first =
     if (first) PS_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     if (mode == PS_MODE_CHOSEN)
         PS_CUDA(c, ps::launch_chosen(p, c->stream));
-    else
+    else {
+        if (p.src[0]) {  // directly before the kernel, whose start it then hides
+            PS_CUDA(c, ps::launch_prep_set(p.src, p.nwin, p.nw, p.wlen, const_cast<double*>(p.win[0].wW), nullptr, c->stream));
+            c->launches += ps::set_launches(p.nwin);
+        }
         PS_CUDA(c, ps::launch_plain_fp64(p, c->stream));
+    }
     c->launches += mode == PS_MODE_CHOSEN ? 2 : 1;
     if (last) {
         PS_CUDA(c, cudaEventRecord(c->ev1, c->stream));
@@ -450,8 +455,8 @@ static int ensure_int2(ps_ctx* c, int2** p, size_t* cap, size_t need)
     return PS_OK;
 }
 
-// Upload (if host) K windows and pad them into ctx->d_win, p.win[k].wW; for the chosen kernel its own
-// preparation does the padding (p.src), so p is good for one launch.
+// Upload (if host) K windows (p.src); run_coupling pads them into ctx->d_win, p.win[k].wW, so p is good for
+// one launch.
 static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* W, int K, int64_t nW, int lmax,
                          bool host, int mode)
 {
@@ -475,11 +480,7 @@ static int stage_windows(ps_ctx* c, ps::CouplingParams& p, const double* const* 
             src[k] = c->d_raw + (size_t)k * nuse;
         }
         p.win[k].wW = c->d_win + (size_t)k * wlen;
-        if (mode == PS_MODE_CHOSEN) p.src[k] = src[k];
-    }
-    if (mode != PS_MODE_CHOSEN) {
-        PS_CUDA(c, ps::launch_prep_set(src, K, nuse, wlen, c->d_win, nullptr, c->stream));
-        c->launches += ps::set_launches(K);
+        p.src[k] = src[k];
     }
     return PS_OK;
 }

@@ -131,6 +131,7 @@ __global__ void k_prep_set(const SetPrep p)
 {
     const int k = blockIdx.y;
     int2* bf = p.bf ? p.bf + (size_t)k * p.wlen : nullptr;
+    let_next_start();
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p.wlen; j += gridDim.x * blockDim.x)
         prep_entry(p.src[k], p.nW, j, p.wW + (size_t)k * p.wlen, bf);
 }

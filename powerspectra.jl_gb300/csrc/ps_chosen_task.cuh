@@ -171,6 +171,9 @@ template <int NWIN, bool RAW>
 __global__ void __launch_bounds__(256) k_slices(const CouplingParams p)
 {
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5), k = blockIdx.y, lane = threadIdx.x & 31;
+    // The coupling kernel's blocks may take their places beside a small grid at once; beside a larger one they
+    // would hold up its blocks (EE x EE covariance, 8 slots at lmax 441: 282 us after, 305-322 at once).
+    if (gridDim.y == 1) let_next_start();
     if (i >= slice_count(p.lmax)) return;
     Slice<NWIN>& s = reinterpret_cast<Slice<NWIN>*>(p.slices)[i];
     if (RAW) {
@@ -185,6 +188,7 @@ __global__ void __launch_bounds__(256) k_slices(const CouplingParams p)
         const int2* __restrict__ bf = p.win[k].bf;
         put_slice<NWIN>(s, i, k, p.wlen, lane, [&](int j) { return __ldg(bf + j); });
     }
+    let_next_start();
 }
 
 // A slice into shared memory, asynchronously (it lands while the previous chunk computes).
@@ -784,7 +788,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NWIN <= 4 ? 5 : 4) k_coup
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the task list is tiled: kTileRows tasks per block, rows outside [lmin, lmax] as l1 = -1
     const int gw = (int)(blockIdx.x * (unsigned)kWarpsPerBlock) + warp;
-    const int2 task = gw < p.ntasks ? p.tasks[gw] : make_int2(-1, 0);
+    int2 task = gw < p.ntasks ? p.tasks[gw] : make_int2(-1, 0);
+    wait_for_previous(task.x);  // the slices and the padded windows
     double Xi[kMaxWin];
     bool active = false;
     if (task.x >= 0)  // warp-uniform
@@ -824,20 +829,17 @@ inline cudaError_t launch_cfg(const CouplingParams& p, bool n00, bool n22, cudaS
         (void)n00;
         (void)n22;
         if constexpr (kHasCoef<NWIN, SPEC>)
-            if (p.coef.f) {
-                k_coupling_chosen<NWIN, a, b, SPEC, true><<<blocks, threads, 0, s>>>(p);
-                return cudaGetLastError();
-            }
-        k_coupling_chosen<NWIN, a, b, SPEC, false><<<blocks, threads, 0, s>>>(p);
+            if (p.coef.f)
+                return launch_after(k_coupling_chosen<NWIN, a, b, SPEC, true>, dim3(blocks), dim3(threads), 0, s, p);
+        return launch_after(k_coupling_chosen<NWIN, a, b, SPEC, false>, dim3(blocks), dim3(threads), 0, s, p);
     } else {
         if (n00 && n22)
-            k_coupling_chosen<NWIN, true, true, 0, false><<<blocks, threads, 0, s>>>(p);
+            return launch_after(k_coupling_chosen<NWIN, true, true, 0, false>, dim3(blocks), dim3(threads), 0, s, p);
         else if (n22)
-            k_coupling_chosen<NWIN, false, true, 0, false><<<blocks, threads, 0, s>>>(p);
+            return launch_after(k_coupling_chosen<NWIN, false, true, 0, false>, dim3(blocks), dim3(threads), 0, s, p);
         else
-            k_coupling_chosen<NWIN, true, false, 0, false><<<blocks, threads, 0, s>>>(p);
+            return launch_after(k_coupling_chosen<NWIN, true, false, 0, false>, dim3(blocks), dim3(threads), 0, s, p);
     }
-    return cudaGetLastError();
 }
 
 

@@ -49,6 +49,37 @@ struct HalfTable {
     int top;
 };
 
+// A kernel launched by launch_after starts while the one before it in the stream still runs (once all of that
+// one's blocks have called let_next_start or ended), so its launch and the start of its blocks cost no time of
+// their own: TT at lmax 767 104.6 -> 96.8 us, the chain of short kernels of a 1532-row solve 6.32 -> 5.73 ms.
+// Not worth it beside kernels that fill the memory system (window spectra at lmax 2508 78.5 -> 84.9 us) nor
+// where a long kernel's addresses take the detour (tensor-core kernels at lmax 8191 424.5 -> 428.8 ms).  All of its threads call wait_for_previous before anything that the kernel
+// before it writes or reads; what came earlier in the stream is complete.  x: a value on which
+// the addresses of every load of such data depend (loads through the read-only path are otherwise free to move up).
+#ifdef __CUDACC__
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous(int& x) { asm volatile("griddepcontrol.wait;" : "+r"(x)::"memory"); }
+__device__ __forceinline__ void wait_for_previous(int& x, int& y)
+{
+    asm volatile("griddepcontrol.wait;" : "+r"(x), "+r"(y)::"memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 // The square-root ratios of the chosen kernels' recurrences (chosen_xi), float-float pairs (rho, r) of 16
 // bytes, for every row l1 <= lmax.  With F(a) = a (a + 2 l1 + 1) and G(t) = t (2 l1 + 1 - t):
 //   f, entry a:  -sqrt(F(a) / F(a + 1)), 1 / sqrt(F(a + 1))   a = -62 .. 2 lmax - l1 + 94, zeros below a = 0

@@ -118,6 +118,11 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
     const int nb = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
     const int q = warp & 3, group = warp >> 2, ngroup = nwarp >> 2, r = 32 * group + lane, nr = 32 * ngroup;
+    if (threadIdx.x == 0) {
+        umma::mbar_init(&sm.full[0]);
+        umma::mbar_init(&sm.full[1]);
+    }
+    wait_for_previous(j0);  // the update of these columns
     const int m = n - j0;
     const unsigned orig = (unsigned)(rank * rows + r);  // this thread's row
     unsigned at = orig;                                 // and its place
@@ -126,10 +131,6 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
     double v[kOwn];  // v[i]: column q + 4 i from the current four on
 #pragma unroll
     for (int i = 0; i < kOwn; ++i) v[i] = own && 4 * i + q < w ? A[(size_t)(4 * i + q) * n + orig] : 0.0;
-    if (threadIdx.x == 0) {
-        umma::mbar_init(&sm.full[0]);
-        umma::mbar_init(&sm.full[1]);
-    }
     cluster.sync();  // every block's barriers are up before any block writes to its shared memory
     bool ok = true;  // the same for every thread of a block
     for (int jq = 0; jq < w; jq += 4) {
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(256) k_lu_rows(double* __restrict__ a, double*
 {
     __shared__ double L[kPan][kPan + 1];  // [column][row]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    let_next_start();
     for (int k = warp; k < kPan; k += 8)
         L[k][lane] = k < lane && lane < w ? a[(size_t)(j0 + k) * n + j0 + lane] : 0.0;
     __syncthreads();
@@ -251,9 +253,12 @@ __global__ void __launch_bounds__(128) k_lu_update(double* __restrict__ a, doubl
                                                    int ce, int j0)
 {
     __shared__ __align__(16) double L[kPan][32], U[kPan][32 + 2];  // L[k][row], U[k][column]
-    const int i0 = j0 + kPan + blockIdx.x * 32, c0 = cb + blockIdx.y * 32;
+    int i0 = j0 + kPan + blockIdx.x * 32;
+    const int c0 = cb + blockIdx.y * 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    let_next_start();
     for (int k = warp; k < kPan; k += 4) L[k][lane] = i0 + lane < n ? a[(size_t)(j0 + k) * n + i0 + lane] : 0.0;
+    wait_for_previous(j0, i0);  // the rows of U (the panel itself was complete before that kernel)
     for (int q = warp; q < 32; q += 4) {
         const int c = c0 + q;
         U[lane][q] = c < ce ? (c < n ? a + (size_t)c * n : b + (size_t)(c - n) * n)[j0 + lane] : 0.0;
@@ -296,9 +301,16 @@ __global__ void __launch_bounds__(256) k_lu_back(const double* __restrict__ a, d
     __shared__ double U[kPan][kPan + 1];  // [column][row]
     __shared__ double sx[kPan];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int i = blockIdx.x * 256 + threadIdx.x;
+    let_next_start();
     b += (size_t)blockIdx.y * n;
+    // what the steps before do not change: the triangle and this thread's row
     for (int k = warp; k < kPan; k += 8)
         U[k][lane] = k < w && lane < w ? a[(size_t)(j0 + k) * n + j0 + lane] : 0.0;
+    double v[kPan];
+#pragma unroll
+    for (int k = 0; k < kPan; ++k) v[k] = i < j0 && k < w ? a[(size_t)(j0 + k) * n + i] : 0.0;
+    wait_for_previous(j0, i);
     __syncthreads();
     if (warp == 0) {
         const double r = lane < w ? 1.0 / U[lane][lane] : 0.0;
@@ -313,34 +325,31 @@ __global__ void __launch_bounds__(256) k_lu_back(const double* __restrict__ a, d
         if (blockIdx.x == 0 && lane < w) x[(size_t)blockIdx.y * n + j0 + lane] = y;
     }
     __syncthreads();
-    const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= j0) return;
     double s0 = 0.0, s1 = 0.0;
-    if (w == kPan) {
 #pragma unroll
-        for (int k = 0; k < kPan; k += 2) {
-            s0 = fma(a[(size_t)(j0 + k) * n + i], sx[k], s0);
-            s1 = fma(a[(size_t)(j0 + k + 1) * n + i], sx[k + 1], s1);
-        }
-    } else {
-        for (int k = 0; k < w; ++k) s0 = fma(a[(size_t)(j0 + k) * n + i], sx[k], s0);
+    for (int k = 0; k < kPan; k += 2) {  // v and sx are 0 beyond w
+        s0 = fma(v[k], sx[k], s0);
+        s1 = fma(v[k + 1], sx[k + 1], s1);
     }
     b[i] -= s0 + s1;
 }
 
 constexpr size_t panel_smem(int rows) { return (size_t)kPan * 32 * ((rows + 31) / 32) * sizeof(double); }
 
-cudaLaunchConfig_t panel_config(int blocks, int rows, cudaLaunchAttribute& at)
+cudaLaunchConfig_t panel_config(int blocks, int rows, cudaLaunchAttribute (&at)[2])
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3((unsigned)(128 * ((rows + 31) / 32)));
     cfg.dynamicSmemBytes = panel_smem(rows);
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_after
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
     return cfg;
 }
 
@@ -361,7 +370,7 @@ int cluster_blocks()
             cudaSuccess &&
         cudaFuncSetAttribute(k_lu_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
         for (int b = kMaxCluster; b >= 8 && !blocks; b /= 2) {
-            cudaLaunchAttribute at;
+            cudaLaunchAttribute at[2];
             const cudaLaunchConfig_t cfg = panel_config(b, kMaxRows, at);
             int nc = 0;
             if (cudaOccupancyMaxActiveClusters(&nc, k_lu_panel, &cfg) == cudaSuccess && nc > 0) blocks = b;
@@ -375,7 +384,7 @@ int cluster_blocks()
 
 // Beyond 4096 rows a panel does not fit the cluster's threads, and for many right-hand sides a solve is
 // mostly products: cuSOLVER takes those.  Measured as host calls with one right-hand side, cuSOLVER and
-// this: n = 96 0.36 and 0.30 ms, n = 400 1.97 and 1.17, n = 1532 11.5 and 6.5, n = 4000 67 and 45.
+// this: n = 96 0.36 and 0.27 ms, n = 400 1.97 and 1.04, n = 1532 11.5 and 5.7, n = 4000 67 and 44.
 bool lu_fits(int n, int nrhs) { return nrhs <= 32 && n <= cluster_blocks() * kMaxRows; }
 
 // x = a^-1 b for the n x n device matrix a and nrhs columns b (leading dimensions n), on stream s with the
@@ -396,6 +405,8 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
         const int below = n - j0 - kPan;
         if (below > 0) {
             const dim3 grid((unsigned)((below + 31) / 32), (unsigned)((ce - cb + 31) / 32));
+            // the next panel's columns are waited for; the rest has time, and its blocks would take their places
+            if (st == wk.side) return launch_after(k_lu_update, grid, dim3(128), 0, st, a, b, n, cb, ce, j0);
             k_lu_update<<<grid, 128, 0, st>>>(a, b, n, cb, ce, j0);
         }
         return cudaGetLastError();
@@ -405,9 +416,10 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
         int* perm = wk.perm + (j0 / kPan & 1) * 2 * kPan;  // the rest of this panel may run beside the next one
         // a cluster of 8 has the quicker barrier, 16 the shorter elimination: even at about 1000 rows
         const int blocks = nb > 8 && m > 1024 ? nb : 8, rows = (m + blocks - 1) / blocks;
-        cudaLaunchAttribute at;
+        cudaLaunchAttribute at[2];
         cudaLaunchConfig_t cfg = panel_config(blocks, rows, at);
         cfg.stream = wk.side;
+        if (j0 == 0) cfg.numAttrs = 1;  // the first one has no update before it
         LU_TRY(cudaLaunchKernelEx(&cfg, k_lu_panel, a, n, j0, w, rows, perm, wk.info));
         LU_TRY(cudaEventRecord(wk.panel, wk.side));
         LU_TRY(cudaStreamWaitEvent(s, wk.panel, 0));
@@ -420,8 +432,12 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
     for (int j0 = (n - 1) / kPan * kPan; j0 >= 0; j0 -= kPan) {
         const int w = n - j0 < kPan ? n - j0 : kPan;
         const dim3 grid((unsigned)(j0 > 0 ? (j0 + 255) / 256 : 1), (unsigned)nrhs);
-        k_lu_back<<<grid, 256, 0, s>>>(a, b, x, n, j0, w);
-        LU_TRY(cudaGetLastError());
+        if (j0 + kPan >= n) {  // the first one starts when the matrix is done
+            k_lu_back<<<grid, 256, 0, s>>>(a, b, x, n, j0, w);
+            LU_TRY(cudaGetLastError());
+        } else {
+            LU_TRY(launch_after(k_lu_back, grid, dim3(256), 0, s, a, b, x, n, j0, w));
+        }
     }
 #undef LU_TRY
     return cudaSuccess;

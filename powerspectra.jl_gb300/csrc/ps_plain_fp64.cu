@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const Pla
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the task list is tiled: kTileRows tasks per block, rows outside [lmin, lmax] as l1 = -1
     const int gw = (int)(blockIdx.x * (unsigned)kWarpsPerBlock) + warp;
-    const int2 task = gw < p.ntasks ? p.tasks[gw] : make_int2(-1, 0);
+    int2 task = gw < p.ntasks ? p.tasks[gw] : make_int2(-1, 0);
+    wait_for_previous(task.x);  // the padded windows
     const int l1 = task.x, l2raw = task.y + lane;
     const bool active = l1 >= 0 && l2raw >= l1 && l2raw <= p.lmax;
     double Xi[kMaxWin];
@@ -300,8 +301,7 @@ cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s)
         bool fits = true;
         for (int c = 0; c < kClasses; ++c) fits = fits && n[c] <= f.n[c];
         if (!fits) continue;
-        f.kernel<<<blocks, threads, 0, s>>>(P);
-        return cudaGetLastError();
+        return launch_after(f.kernel, dim3(blocks), dim3(threads), 0, s, P);
     }
     return cudaErrorInvalidValue;
 }
