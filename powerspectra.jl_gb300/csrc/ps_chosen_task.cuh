@@ -828,10 +828,17 @@ inline cudaError_t launch_cfg(const CouplingParams& p, bool n00, bool n22, cudaS
         constexpr bool a = spec_needs(SPEC, NWIN, true), b = spec_needs(SPEC, NWIN, false);
         (void)n00;
         (void)n22;
+        // Where all blocks of a launch fit the SMs at once (5 on each), the longest rows share an SM to the end;
+        // with fewer the rest spread as SMs come free.  ++/-- with 5, 4, 3 and 2: lmax 383 (624 blocks) 81, 80, 74,
+        // 72 us (TT 42, 43, 41, 44), 511 (1088) 113, 107, 113, 124; 767 (2400) 253, 258, 276, 309.
+        const int share = NWIN > 5 || blocks <= 2 * kSMs || blocks > 8 * kSMs ? 0 : (blocks <= 5 * kSMs ? 3 : 4);
+        const size_t fixed = kWarpsPerBlock * (4 * sizeof(Slice<NWIN>) + sizeof(CoefTab)) + sizeof(TileRows);
         if constexpr (kHasCoef<NWIN, SPEC>)
             if (p.coef.f)
-                return launch_after(k_coupling_chosen<NWIN, a, b, SPEC, true>, dim3(blocks), dim3(threads), 0, s, p);
-        return launch_after(k_coupling_chosen<NWIN, a, b, SPEC, false>, dim3(blocks), dim3(threads), 0, s, p);
+                return launch_after(k_coupling_chosen<NWIN, a, b, SPEC, true>, dim3(blocks), dim3(threads),
+                                    share ? pad_smem(share, fixed + kWarpsPerBlock * sizeof(CoefStage)) : 0, s, p);
+        return launch_after(k_coupling_chosen<NWIN, a, b, SPEC, false>, dim3(blocks), dim3(threads),
+                            share ? pad_smem(share, fixed) : 0, s, p);
     } else {
         if (n00 && n22)
             return launch_after(k_coupling_chosen<NWIN, true, true, 0, false>, dim3(blocks), dim3(threads), 0, s, p);

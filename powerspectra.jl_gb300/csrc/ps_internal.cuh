@@ -63,9 +63,24 @@ __device__ __forceinline__ void wait_for_previous(int& x, int& y)
 {
     asm volatile("griddepcontrol.wait;" : "+r"(x), "+r"(y)::"memory");
 }
+constexpr unsigned kSMs = 152;
+// Dynamic shared memory with which at most `blocks` blocks of a kernel with `fixed` bytes share an SM (228 KB,
+// 1 KB of it per block).
+constexpr size_t kSmemSM = 228 * 1024;
+constexpr size_t pad_smem(int blocks, size_t fixed)
+{
+    const size_t need = kSmemSM / (blocks + 1) / 128 * 128 + 128, have = 1024 + fixed;
+    return need > have ? need - have : 0;
+}
+template <class K>
+inline cudaError_t allow_smem(K kernel, size_t bytes)  // dynamic shared memory that the kernel may be launched with
+{
+    return bytes ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) : cudaSuccess;
+}
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
 {
+    if (cudaError_t e = allow_smem(kernel, smem)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;

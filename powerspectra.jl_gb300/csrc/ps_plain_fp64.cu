@@ -227,12 +227,15 @@ __device__ __forceinline__ void points00(const PlainParams& P, Factors& fc, int 
     }
 }
 
+struct __align__(16) PlainSmem {
+    Factors f[kWarpsPerBlock];
+    double stage[kWarpsPerBlock][kMaxWin * 32];
+    TileRows rows;
+};
 template <int N00, int N02, int N22E, int N22O, int N22A>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const PlainParams P)
 {
-    __shared__ Factors sf[kWarpsPerBlock];
-    __shared__ double stage[kWarpsPerBlock][kMaxWin * 32];
-    __shared__ TileRows rows;
+    __shared__ PlainSmem sm;
     const CouplingParams& p = P.c;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the task list is tiled: kTileRows tasks per block, rows outside [lmin, lmax] as l1 = -1
@@ -250,11 +253,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const Pla
         b.zero();
         // the points whose j a window reaches, for the warp's smallest d (the others' windows end in zeros)
         const int n = min(p.nw - 1 - (max(task.y, l1) - l1), 2 * l1);
-        if constexpr (N02 + N22E + N22O + N22A > 0) sweep22(P, sf[warp], l1, task.y, l2, n, lane, a, b);
-        else points00(P, sf[warp], l1, task.y, l2, n, lane, a, b);
+        if constexpr (N02 + N22E + N22O + N22A > 0) sweep22(P, sm.f[warp], l1, task.y, l2, n, lane, a, b);
+        else points00(P, sm.f[warp], l1, task.y, l2, n, lane, a, b);
         a.give(P, b, l1, Xi);
     }
-    write_tile<kMaxWin>(p, l1, task.y, active, Xi, &stage[0][0], kMaxWin * 32, rows, warp, lane);
+    write_tile<kMaxWin>(p, l1, task.y, active, Xi, &sm.stage[0][0], kMaxWin * 32, sm.rows, warp, lane);
 }
 
 struct Form {
@@ -301,7 +304,14 @@ cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s)
         bool fits = true;
         for (int c = 0; c < kClasses; ++c) fits = fits && n[c] <= f.n[c];
         if (!fits) continue;
-        return launch_after(f.kernel, dim3(blocks), dim3(threads), 0, s, P);
+        // Blocks that share an SM: one warp per quarter of an SM keeps its FP64 pipe busy for all but the refills
+        // (64 cycles an instruction), and the fewer share it, the sooner the longest rows, which come first,
+        // are done and the better the rest spread over the SMs.  ++/-- at nW = lmax + 1, with as many as fit (8), 1, 2
+        // and 3: lmax 255 (288 blocks) 109, 94, 110, 110 us; 383 (624) 271, 231, 206, 225; 511 (1088) 534, 483, 429,
+        // 426; 767 (2400) 1366, 1481, 1301, 1302; 1001 (4224) 2797, 3166, 2772, 2777.
+        const int share = blocks <= 2 * kSMs ? 1 : (blocks <= 8 * kSMs ? 2 : 3);
+        const size_t pad = blocks > kSMs ? pad_smem(share, sizeof(PlainSmem)) : 0;
+        return launch_after(f.kernel, dim3(blocks), dim3(threads), pad, s, P);
     }
     return cudaErrorInvalidValue;
 }

@@ -218,9 +218,18 @@ cudaError_t launch_quickpol(const double* W, long long nW, int lmax, int bl, int
     const long long total = (long long)(lmax - 1) * width;  // < 2^31 for lmax <= 16383
     const unsigned blocks = (unsigned)((total + 127) / 128);
     const bool same = s1 == s2 && nu1 == nu2, hasm = p.m3[0] != 0 || p.m3[1] != 0;
-    if (same) hasm ? k_quickpol_fp64<true, true><<<blocks, 128, 0, s>>>(p) : k_quickpol_fp64<true, false><<<blocks, 128, 0, s>>>(p);
-    else hasm ? k_quickpol_fp64<false, true><<<blocks, 128, 0, s>>>(p) : k_quickpol_fp64<false, false><<<blocks, 128, 0, s>>>(p);
-    return cudaGetLastError();
+    // Two blocks, two warps per quarter of an SM, keep its FP64 pipe busy (64 cycles an instruction); the fewer share
+    // it, the sooner the longest rows, which come first, are done and the better the rest spread over the SMs.
+    // Equal spins, band 201, as many blocks as fit and 2: lmax 300 656 and 515 us, 723 2915 and 2268, 999 4574 and
+    // 4368, 1999 17.60 and 17.37 ms (1: 19.2).
+    const size_t pad = blocks > 2 * kSMs ? pad_smem(2, 0) : 0;
+    auto go = [&](void (*kernel)(QpParams)) -> cudaError_t {
+        if (cudaError_t e = allow_smem(kernel, pad)) return e;
+        kernel<<<blocks, 128, pad, s>>>(p);
+        return cudaGetLastError();
+    };
+    if (same) return hasm ? go(k_quickpol_fp64<true, true>) : go(k_quickpol_fp64<true, false>);
+    return hasm ? go(k_quickpol_fp64<false, true>) : go(k_quickpol_fp64<false, false>);
 }
 
 }  // namespace ps
