@@ -274,7 +274,7 @@ int ps_batch_autotune(ps_ctx *ctx, const ps_problem *probs, int nprob, int *best
  * device-wide synchronisation cudaMalloc/cudaFree may cause.  It computes the
  * same matrices as ps_mcm_multi_device with PS_MODE_CHOSEN (same kernel, same
  * results) on the caller's current device and `stream` (a cudaStream_t), with
- * no context and no allocation: its scratch (padded windows and the work list,
+ * no context and no allocation: its scratch (padded windows, their slices and the work list,
  * 10.9 MB) is a fixed array in the library's device image, which every GPU that
  * loads the library keeps until the process exits.  Limits: lmax <= 4095 (a
  * larger lmax returns PS_ERR_ARG); `stream` must belong to the current device

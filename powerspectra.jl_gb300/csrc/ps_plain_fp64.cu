@@ -42,7 +42,8 @@
 // integer-to-double conversions.  Measured with it, with this form in two sweeps
 // that meet in the middle, and now: all spin cases at lmax 1999, lmin 2, nW 3999
 // 123.7, 34.9 and 32.1 ms; a whole host call (nW = lmax + 1, so that a quarter of the family lies beyond
-// the windows), TT at lmax 95 130, 47 and 44 us, EE/BB at lmax 767 8.0, 3.0 and 2.8 ms.  Errors against 128-bit
+// the windows), TT at lmax 95 130, 47 and 44 us, EE/BB at lmax 767 8.0, 3.0 and 2.8 ms (1.45
+// with its blocks copied whole and fewer blocks per SM, below).  Errors against 128-bit
 // arithmetic are smaller than the recurrence's (lmax 2000, all points: 7e-15 at
 // most, 1.5e-14 before).
 #include "ps_internal.cuh"

@@ -29,7 +29,7 @@
 // family (tau 3, mu, b, h, two products, two sums), 8 when m3 = 0, 17 for two; the
 // recurrence this replaced took a square root and a division per family and point.
 // Measured with it and now, 1000 x 1000 with band (100, 100), as a whole host call:
-// 26.9 -> 4.6 ms for nu = 0, s = 2 (one family), 26.7 -> 7.1 ms for nu = -1, 2, s = -2, 2.
+// 26.9 -> 4.4 ms for nu = 0, s = 2 (one family), 26.7 -> 6.8 ms for nu = -1, 2, s = -2, 2.
 #include "ps_internal.cuh"
 
 namespace ps {
