@@ -72,11 +72,15 @@ constexpr size_t pad_smem(int blocks, size_t fixed)
     const size_t need = kSmemSM / (blocks + 1) / 128 * 128 + 128, have = 1024 + fixed;
     return need > have ? need - have : 0;
 }
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  The limit set is the same for every launch, so
+// that of one thread never undercuts another's (with 48 KB of static memory it stays within a block's 227 KB).
+constexpr size_t kDynLimit = 160 * 1024;
 template <class K>
-inline cudaError_t allow_smem(K kernel, size_t bytes)  // dynamic shared memory that the kernel may be launched with
+inline cudaError_t allow_smem(K kernel, size_t bytes)
 {
-    return bytes ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) : cudaSuccess;
+    return bytes ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynLimit) : cudaSuccess;
 }
+static_assert(pad_smem(1, 0) <= kDynLimit, "one block per SM is the largest pad");
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
 {
