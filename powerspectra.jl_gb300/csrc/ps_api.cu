@@ -26,6 +26,7 @@ int ps_linalg_decouple(ps_linalg* L, const double* Y, const double* B1, const do
                        double* out, int64_t ldout, cudaStream_t s, char* err, size_t errn, bool on_device);
 int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const double* b, int nrhs, int64_t ldb,
                     double* x, int64_t ldx, cudaStream_t s, char* err, size_t errn);
+void ps_linalg_wait_limit(ps_linalg* L, int limit);
 
 // Largest lmax the kernels accept: the integer products in P(j) stay below 2^63
 // and every index stays in 32 bits.
@@ -1713,6 +1714,16 @@ int ps_solve(ps_ctx* c, const double* M, int64_t n, int64_t ldm, const double* b
     int st = ps_linalg_solve(c->la, M, (int)n, ldm, b, nrhs, ldb, x, ldx, c->stream, c->err, sizeof(c->err));
     if (!st) c->launches += 2;
     return st;
+}
+
+// Not part of the interface (the header has no such call): the polls after which the waits of this context's LU
+// panels give up, so that what follows can be tested.
+int ps_lu_wait_limit(ps_ctx* c, int limit)
+{
+    if (!c) return PS_ERR_ARG;
+    if (!c->la) c->la = ps_linalg_new();
+    ps_linalg_wait_limit(c->la, limit);
+    return PS_OK;
 }
 
 // The Xi kernel of either arithmetic on a device W (nW entries) into c->d_out.

@@ -204,7 +204,9 @@ struct LuWork {
     cudaEvent_t panel, rest;
     int* perm;                 // 128 ints
     int* info;
+    int wait_limit;            // polls of a panel's waits
 };
+constexpr int kLuWaitLimit = 1 << 22;
 cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s);
 cudaError_t launch_transpose(double* dst, const double* src, int n, cudaStream_t s);
 cudaError_t launch_negate(const double* src, double* dst, long long count, cudaStream_t s);

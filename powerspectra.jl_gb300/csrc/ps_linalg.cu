@@ -72,7 +72,11 @@ struct ps_linalg {
     size_t cap = 0;       // elements of a / x / t
     cudaStream_t side = nullptr;  // ps_lu.cu's panels
     cudaEvent_t ev_panel = nullptr, ev_rest = nullptr;
+    int wait_limit = ps::kLuWaitLimit;
 };
+
+// How often the LU panels' waits poll before they give up (0: at once), for the test of what follows.
+void ps_linalg_wait_limit(ps_linalg* L, int limit) { L->wait_limit = limit; }
 
 static int la_err(char* err, size_t n, int code, const char* fmt, ...)
 {
@@ -218,7 +222,7 @@ int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const dou
     if ((st = la_in(L->x, b, n, nrhs, ldb, s, err, errn))) return st;
     const double* res = L->x;
     if (own) {
-        const ps::LuWork wk = {L->side, L->ev_panel, L->ev_rest, L->ipiv, L->info};
+        const ps::LuWork wk = {L->side, L->ev_panel, L->ev_rest, L->ipiv, L->info, L->wait_limit};
         LA_CUDA(ps::launch_lu_solve(L->a, n, L->x, nrhs, L->t, wk, s));
         int info = 0;
         LA_CUDA(cudaMemcpyAsync(&info, L->info, sizeof(int), cudaMemcpyDeviceToHost, s));

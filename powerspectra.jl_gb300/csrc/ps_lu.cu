@@ -10,7 +10,7 @@
 //   * k_lu_panel: one thread-block cluster, four threads per row with the row's 32 values in registers.
 //     Per column every block finds its largest entry (warp reductions on the bits of |a|) and sends that
 //     row, its key and the pivot's reciprocal to all blocks' shared memory in words that count towards an
-//     mbarrier there (bounded wait; a wait that gives up is reported).  So every block knows the pivot row
+//     mbarrier there (bounded wait; a wait that gives up is reported, see below).  So every block knows the pivot row
 //     without a cluster barrier (whose memory fence took 0.2 us per column) and eliminates its own rows.  Two sets of
 //     buffers alternate: a block sends for column j + 1 only after all of its threads have read column
 //     j's, so column j + 2's words meet free buffers.  The kernel leaves the panel's net permutation.
@@ -28,6 +28,9 @@
 //
 // The pivot is the entry of largest magnitude, the uppermost one among equals.  A zero pivot is
 // reported (info), as getrf does.
+//
+// When a wait gives up, the panel leaves the rows of the columns beyond it where they are (perm the identity), info
+// becomes -1 and the panels after it do nothing, so that everything queued behind stays inside the matrix and ends.
 #include "ps_internal.cuh"
 #include "ps_umma.cuh"
 
@@ -45,7 +48,6 @@ constexpr int kPan = 32;          // columns of a panel
 constexpr int kMaxCluster = 16;
 constexpr int kMaxRows = 256;     // rows per block of the panel kernel, four threads each
 constexpr unsigned kNoRow = 0x7fffffffu;
-constexpr int kWaitLimit = 1 << 22;
 
 // What a block sends to every block of the cluster for one column: its best row.
 struct Cand {
@@ -61,6 +63,7 @@ struct PanelSmem {
     double row[kPan];           // this block's candidate before it is sent
     double col[2][kMaxRows];    // a column of this block's rows; two, since a slow warp may still read the last one
     unsigned whi[kMaxRows / 32], wlo[kMaxRows / 32], wat[kMaxRows / 32];  // per 32 rows
+    int sent[kMaxCluster];      // columns each block has sent, negative where one of its waits gave up
 };
 
 // The largest (hi, lo) of the lanes and the smallest `at` among those that hold it.
@@ -83,11 +86,11 @@ __device__ __forceinline__ void send(void* at, uint64_t* full, int d, unsigned l
 }
 // Bounded wait of the whole block for phase `parity`, with the other blocks' words visible after it;
 // the same answer for every thread.
-__device__ __forceinline__ bool wait_full(uint64_t* bar, uint32_t parity)
+__device__ __forceinline__ bool wait_full(uint64_t* bar, uint32_t parity, int limit)
 {
     const uint32_t a = umma::smem_addr(bar);
     bool done = false;
-    for (int it = 0; it < kWaitLimit && !done; ++it) {
+    for (int it = 0; it < limit && !done; ++it) {
         uint32_t p;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
@@ -108,8 +111,11 @@ __device__ __forceinline__ bool is_inf(double x) { return (__double2hiint(x) & 0
 // a swap exchanges places only, and the finished columns wait in shared memory for the final places.
 // The columns run in a loop over four at a time (the registers move up): unrolled over all 32, every
 // instruction ran once per panel and its fetch cost more than its work.
+// OTHER_LIMIT: the waits give up after `limit` polls, else after kLuWaitLimit (as a number in a register the limit
+// costs 1 % of a solve).
+template <bool OTHER_LIMIT>
 __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict__ a, int n, int j0, int w, int rows,
-                                                           int* __restrict__ perm, int* __restrict__ info)
+                                                           int* __restrict__ perm, int* info, int limit)
 {
     constexpr int kOwn = kPan / 4;  // columns per thread
     extern __shared__ __align__(16) double fin[];  // [column][row of this block, in whole warps]
@@ -124,6 +130,14 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
     }
     wait_for_previous(j0);  // the update of these columns
     const int m = n - j0;
+    auto leave_rows = [&] {  // a panel without a factorisation
+        if (rank == 0 && threadIdx.x < kPan) {
+            perm[threadIdx.x] = (int)threadIdx.x;
+            perm[kPan + threadIdx.x] = -1;
+        }
+    };
+    // set by an earlier panel (this one sets it behind the cluster's last barrier but one): the same for every block
+    const int state = *(volatile int*)info;
     const unsigned orig = (unsigned)(rank * rows + r);  // this thread's row
     unsigned at = orig;                                 // and its place
     const bool own = r < rows && orig < (unsigned)m;
@@ -131,8 +145,14 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
     double v[kOwn];  // v[i]: column q + 4 i from the current four on
 #pragma unroll
     for (int i = 0; i < kOwn; ++i) v[i] = own && 4 * i + q < w ? A[(size_t)(4 * i + q) * n + orig] : 0.0;
+    if (state < 0) {  // looked at here, its load runs beside the others (ahead of them: 1 us per panel)
+        leave_rows();
+        return;
+    }
     cluster.sync();  // every block's barriers are up before any block writes to its shared memory
     bool ok = true;  // the same for every thread of a block
+    int sent = 0;    // columns sent: a block sends one only when it has everyone's of the one before, so that the
+                     // blocks' counts differ by one at most
     for (int jq = 0; jq < w; jq += 4) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -179,7 +199,9 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
                     if (lane == 1) send(&c.at, &sm.full[buf], d, row);
                     if (lane == 2 && row == kNoRow) send(&c.rcp, &sm.full[buf], d, 0ull);  // no row left here
                 }
-                ok = wait_full(&sm.full[buf], (unsigned)(j >> 1) & 1u);
+                sent = j + 1;
+                ok = wait_full(&sm.full[buf], (unsigned)(j >> 1) & 1u, OTHER_LIMIT ? limit : kLuWaitLimit);
+                if (!ok) continue;  // the candidates are not all here; the columns left are passed over
                 // ---- the pivot, the places, the elimination ----
                 const unsigned long long kb = lane < nb ? sm.cand[buf][lane].bits : 0ull;
                 hi = (unsigned)(kb >> 32);
@@ -207,7 +229,8 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
 #pragma unroll
         for (int i = 0; i + 1 < kOwn; ++i) v[i] = v[i + 1];
     }
-    if (own) {
+    // a block that has every column knows its rows' places, whatever becomes of the others
+    if (own && ok) {
 #pragma unroll
         for (int i = 0; i < kOwn; ++i)
             if (4 * i + q < w) A[(size_t)(4 * i + q) * n + at] = fin[(4 * i + q) * nr + r];
@@ -216,8 +239,30 @@ __global__ void __launch_bounds__(4 * kMaxRows, 1) k_lu_panel(double* __restrict
             if (orig < (unsigned)kPan) perm[kPan + orig] = at < (unsigned)kPan ? -1 : (int)at;
         }
     }
-    if (!ok && threadIdx.x == 0) atomicMin(info, -1);
+    // ---- the end, for all blocks alike ----
+    if (threadIdx.x < nb) *cluster.map_shared_rank(&sm.sent[rank], (int)threadIdx.x) = ok ? sent : -sent;
     cluster.sync();  // no block leaves while another may write to it
+    int top = 0;
+    bool all = true;
+    for (int b = 0; b < nb; ++b) {
+        top = max(top, abs(sm.sent[b]));
+        all &= sm.sent[b] > 0;
+    }
+    if (!all) {
+        // No block may leave while words are under way to it.  Those of the last column, top - 1, come from the
+        // blocks that sent it; the others send words without a meaning, so that it completes everywhere.
+        if (sent < top) {
+            uint64_t* full = &sm.full[(top - 1) & 1];
+            Cand& c = sm.cand[(top - 1) & 1][rank];
+            if (threadIdx.x == 0) umma::mbar_expect_tx(full, (unsigned)nb * kCandBytes);
+            for (int e = threadIdx.x; e < nb * (kPan + 3); e += blockDim.x)
+                send(&c.row[0] + e % (kPan + 3), full, e / (kPan + 3), 0ull);
+        }
+        for (int j = max(top - 2, 0); j < top; ++j) wait_full(&sm.full[j & 1], (unsigned)(j >> 1) & 1u, kLuWaitLimit);
+        leave_rows();
+        if (threadIdx.x == 0) atomicMin(info, -1);
+        cluster.sync();
+    }
 }
 
 // The columns cb .. ce - 1 beyond the panel: rows permuted, then the first w of them solved with the
@@ -366,14 +411,18 @@ int cluster_blocks()
     }
     if (const int b = known[dev].load()) return b - 1;
     int blocks = 0;
-    if (cudaFuncSetAttribute(k_lu_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem(kMaxRows)) ==
-            cudaSuccess &&
-        cudaFuncSetAttribute(k_lu_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+    bool ready = true;
+    for (auto kernel : {k_lu_panel<false>, k_lu_panel<true>})
+        ready = ready &&
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem(kMaxRows)) ==
+                    cudaSuccess &&
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (ready)
         for (int b = kMaxCluster; b >= 8 && !blocks; b /= 2) {
             cudaLaunchAttribute at[2];
             const cudaLaunchConfig_t cfg = panel_config(b, kMaxRows, at);
             int nc = 0;
-            if (cudaOccupancyMaxActiveClusters(&nc, k_lu_panel, &cfg) == cudaSuccess && nc > 0) blocks = b;
+            if (cudaOccupancyMaxActiveClusters(&nc, k_lu_panel<false>, &cfg) == cudaSuccess && nc > 0) blocks = b;
         }
     cudaGetLastError();
     known[dev].store(blocks + 1);
@@ -388,8 +437,8 @@ int cluster_blocks()
 bool lu_fits(int n, int nrhs) { return nrhs <= 32 && n <= cluster_blocks() * kMaxRows; }
 
 // x = a^-1 b for the n x n device matrix a and nrhs columns b (leading dimensions n), on stream s with the
-// panels on w.side; a and b are overwritten.  *w.info becomes the first zero pivot's index from 1, or
-// stays INT_MAX.
+// panels on w.side; a and b are overwritten.  *w.info becomes the first zero pivot's index from 1, -1 when a
+// wait gave up (x then holds nothing of use), or stays INT_MAX.
 cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s)
 {
     static const int kNone = INT_MAX;
@@ -420,7 +469,8 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
         cudaLaunchConfig_t cfg = panel_config(blocks, rows, at);
         cfg.stream = wk.side;
         if (j0 == 0) cfg.numAttrs = 1;  // the first one has no update before it
-        LU_TRY(cudaLaunchKernelEx(&cfg, k_lu_panel, a, n, j0, w, rows, perm, wk.info));
+        const auto kernel = wk.wait_limit == kLuWaitLimit ? k_lu_panel<false> : k_lu_panel<true>;
+        LU_TRY(cudaLaunchKernelEx(&cfg, kernel, a, n, j0, w, rows, perm, wk.info, wk.wait_limit));
         LU_TRY(cudaEventRecord(wk.panel, wk.side));
         LU_TRY(cudaStreamWaitEvent(s, wk.panel, 0));
         const int c1 = j0 + w, c2 = c1 + kPan < n ? c1 + kPan : (n > c1 ? n : c1);  // the next panel: c1 .. c2 - 1
