@@ -37,10 +37,13 @@ struct ps_ctx {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     char err[512] = {0};
-    // warp task list for the current (lmin, lmax)
-    int2* d_tiles = nullptr;
-    size_t tiles_cap = 0;
-    int ntiles = 0, tile_lmin = -1, tile_lmax = -1;
+    // warp task lists for the current (lmin, lmax) of the plain and of the chosen calls: one each, so that a
+    // graph recorded from the one arithmetic does not see the other's calls
+    struct Tiles {
+        int2* d = nullptr;
+        size_t cap = 0;
+        int n = 0, lmin = -1, lmax = -1;
+    } tiles[2];
     // the plain kernels' HalfTable, for lmax up to half_lmax
     double* d_half = nullptr;
     size_t half_cap = 0;
@@ -205,16 +208,16 @@ static int upload_tasks(ps_ctx* c, const std::vector<int2>& t, int2** d, size_t*
     return PS_OK;
 }
 
-static int ensure_tiles(ps_ctx* c, int lmin, int lmax)
+static int ensure_tiles(ps_ctx* c, ps_ctx::Tiles& L, int lmin, int lmax)
 {
-    if (c->tile_lmin == lmin && c->tile_lmax == lmax && c->d_tiles) return PS_OK;
+    if (L.lmin == lmin && L.lmax == lmax && L.d) return PS_OK;
     std::vector<int2> t;
     tile_task_list(lmin, lmax, t);
-    c->tile_lmin = c->tile_lmax = -1;
-    if (int st = upload_tasks(c, t, &c->d_tiles, &c->tiles_cap)) return st;
-    c->ntiles = (int)t.size();
-    c->tile_lmin = lmin;
-    c->tile_lmax = lmax;
+    L.lmin = L.lmax = -1;
+    if (int st = upload_tasks(c, t, &L.d, &L.cap)) return st;
+    L.n = (int)t.size();
+    L.lmin = lmin;
+    L.lmax = lmax;
     return PS_OK;
 }
 
@@ -395,10 +398,11 @@ static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
 
 static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first = true, bool last = true)
 {
-    int st = ensure_tiles(c, p.lmin, p.lmax);
+    ps_ctx::Tiles& tiles = c->tiles[mode == PS_MODE_CHOSEN];
+    int st = ensure_tiles(c, tiles, p.lmin, p.lmax);
     if (st) return st;
-    p.tasks = c->d_tiles;
-    p.ntasks = c->ntiles;
+    p.tasks = tiles.d;
+    p.ntasks = tiles.n;
     if (mode == PS_MODE_CHOSEN) {
         if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, ps::slice_table_bytes(p)))) return st;
         p.slices = c->d_slices;
@@ -654,7 +658,7 @@ void ps_destroy(ps_ctx* c)
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->d_half);
-    cudaFree(c->d_tiles);
+    for (auto& t : c->tiles) cudaFree(t.d);
     cudaFree(c->d_win);
     cudaFree(c->d_raw);
     cudaFree(c->d_spec);

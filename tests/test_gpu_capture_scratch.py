@@ -1,0 +1,69 @@
+"""Graphs recorded from context calls, and what later calls on the same context do to them: calls that use none of a
+recorded call's scratch leave its replays as they were, and a call of the same shape is enough to warm up a capture.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+class Call:
+    """ps_mcm_multi_device of some spins on one grid, with its own windows and matrices."""
+
+    def __init__(self, ctx, spins, lmax, mode, lmin=0, seed=1):
+        from powerspectra_gpu import synthetic as syn
+        self.ctx, self.spins, self.lmin, self.lmax, self.mode = ctx, spins, lmin, lmax, mode
+        self.nW, self.n = 2 * lmax + 1, lmax - lmin + 1
+        self.W = torch.tensor(np.stack([syn.mask_spectrum(self.nW, 0.5, self.nW / 3.0, seed=seed + s) for s in spins]),
+                              device="cuda")
+        self.M = torch.zeros((len(spins), self.n, self.n), dtype=torch.float64, device="cuda")
+
+    def __call__(self):
+        self.ctx.mcm_multi_device({s: self.W[i].data_ptr() for i, s in enumerate(self.spins)}, self.nW, self.lmin,
+                                  self.lmax, {s: self.M[i].data_ptr() for i, s in enumerate(self.spins)}, self.n,
+                                  mode=self.mode)
+
+    def direct(self):
+        self()
+        torch.cuda.synchronize()
+        return self.M.clone()
+
+    def record(self, stream):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            self()
+        return g
+
+    def replayed(self, g):
+        self.M.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        return self.M
+
+
+@pytest.fixture
+def own():
+    """A context of its own on a stream that can be captured."""
+    from powerspectra_gpu import Context
+    ctx, s = Context(0), torch.cuda.Stream()
+    ctx.set_stream(s.cuda_stream)
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        yield ctx, s
+        torch.cuda.synchronize()
+    ctx.close()
+
+
+@pytest.mark.parametrize("first,second", [("plain", "chosen"), ("chosen", "plain")])
+def test_one_arithmetic_beside_the_other(own, first, second):
+    ctx, s = own
+    a, b = Call(ctx, (0, 2), 90, first), Call(ctx, (0, 2), 60, second, lmin=2, seed=7)
+    want_a, want_b = a.direct(), b.direct()
+    ga = a.record(s)  # the other arithmetic's call on another grid came last
+    assert bool((a.replayed(ga) == want_a).all())
+    assert bool((b.direct() == want_b).all())
+    gb = b.record(s)
+    for _ in range(2):
+        assert bool((a.replayed(ga) == want_a).all())
+        assert bool((b.replayed(gb) == want_b).all())
