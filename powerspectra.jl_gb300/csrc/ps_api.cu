@@ -44,9 +44,9 @@ struct ps_ctx {
         size_t cap = 0;
         int n = 0, lmin = -1, lmax = -1;
     } tiles[2];
-    // the plain kernels' HalfTable, for lmax up to half_lmax
-    double* d_half = nullptr;
-    size_t half_cap = 0;
+    // the plain kernels' HalfTables: the last one is in use, for lmax up to half_lmax.  The ones it replaced stay
+    // until the context goes: a recorded graph may read them (lengths double, so together they are no larger)
+    std::vector<double*> halves;
     int half_lmax = -1;
     // padded windows, raw inputs, spectra, outputs (element counts)
     double* d_win = nullptr;
@@ -251,16 +251,21 @@ static void half_table(int top, int nw, std::vector<double>& t)
 static int ensure_half(ps_ctx* c, int lmax, ps::HalfTable* out)
 {
     if (c->half_lmax < lmax) {
+        const int top_lmax = std::max(lmax, std::min(2 * c->half_lmax, PS_MAX_LMAX));
         std::vector<double> t;
-        half_table(4 * lmax, 2 * lmax + 2, t);
+        half_table(4 * top_lmax, 2 * top_lmax + 2, t);
+        double* d = nullptr;
+        size_t cap = 0;
+        if (int st = ensure(c, &d, &cap, t.size())) return st;
+        c->halves.push_back(d);
         c->half_lmax = -1;
-        if (int st = ensure(c, &c->d_half, &c->half_cap, t.size())) return st;
-        PS_CUDA(c, cudaMemcpyAsync(c->d_half, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        PS_CUDA(c, cudaMemcpyAsync(d, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
         PS_CUDA(c, cudaStreamSynchronize(c->stream));
-        c->half_lmax = lmax;
+        c->half_lmax = top_lmax;
     }
     const int top = 4 * c->half_lmax;
-    *out = ps::HalfTable{c->d_half, c->d_half + top + 1, c->d_half + 2 * ((size_t)top + 1), top};
+    const double* d = c->halves.back();
+    *out = ps::HalfTable{d, d + top + 1, d + 2 * ((size_t)top + 1), top};
     return PS_OK;
 }
 
@@ -657,7 +662,7 @@ void ps_destroy(ps_ctx* c)
     if (!c) return;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    cudaFree(c->d_half);
+    for (double* d : c->halves) cudaFree(d);
     for (auto& t : c->tiles) cudaFree(t.d);
     cudaFree(c->d_win);
     cudaFree(c->d_raw);

@@ -67,3 +67,17 @@ def test_one_arithmetic_beside_the_other(own, first, second):
     for _ in range(2):
         assert bool((a.replayed(ga) == want_a).all())
         assert bool((b.replayed(gb) == want_b).all())
+
+
+def test_plain_graph_beside_a_larger_quickpol(own):
+    """QuickPol in FP64 reads the same factors as the plain kernels, and for a larger lmax needs more of them."""
+    ctx, s = own
+    a = Call(ctx, (0, 1, 2, 3), 70, "plain")
+    want = a.direct()
+    g = a.record(s)
+    for lmax in (71, 150, 900):
+        ctx.quickpol_xi(0, 0, 2, 2, np.ones(2 * lmax + 1), lmax, 3, 3)
+        junk = torch.full((1 << 16,), np.nan, dtype=torch.float64, device="cuda")  # fresh memory, were any given back
+        assert bool((a.replayed(g) == want).all())
+        assert bool((a.direct() == want).all())
+        del junk
