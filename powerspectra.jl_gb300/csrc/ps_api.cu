@@ -382,13 +382,23 @@ void cov_window_spec(int kind, int k, int* product, int* parity)
 // bracket all of its coupling kernels (ps_last_kernel_ms).
 static int ensure_bytes(ps_ctx* c, unsigned char** p, size_t* cap, size_t need);
 
+// Whether work on s is being recorded (or can't be asked for, as for the legacy stream while another records).
+static bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // The chosen kernels' square-root ratios for rows up to lmax, kept by the context and replaced by larger ones.
-// None beyond kCoefMaxLmax or where there is no room: the kernels then make them chunk by chunk.
+// None beyond kCoefMaxLmax, where there is no room, or in a capture (a table can't be made there, and a recorded
+// graph must not hold the address of one that may be replaced): the kernels then make them chunk by chunk.
 static const int kCoefMaxLmax = 4096;
 static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
 {
     *out = ps::CoefRows{};
-    if (lmax > kCoefMaxLmax) return PS_OK;
+    if (lmax > kCoefMaxLmax || capturing(c->stream)) return PS_OK;
     if (c->coef_lmax < lmax) {
         c->coef_lmax = -1;
         if (ensure_bytes(c, &c->d_coef, &c->coef_cap, ps::coef_bytes(lmax))) return PS_OK;
@@ -409,7 +419,8 @@ static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first =
     p.tasks = tiles.d;
     p.ntasks = tiles.n;
     if (mode == PS_MODE_CHOSEN) {
-        if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, ps::slice_table_bytes(p)))) return st;
+        // room for any list of slots on this grid, so that one call of a grid is enough before a capture
+        if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, ps::slice_table_most(p.lmax)))) return st;
         p.slices = c->d_slices;
         if (ps::reads_coef(p) && (st = ensure_coef(c, p.lmax, &p.coef))) return st;
     } else if ((st = ensure_half(c, p.lmax, &p.half))) {

@@ -52,6 +52,7 @@ size_t slice_table_bytes(const CouplingParams& p)
     const Inst* i = find_inst(p, spec_of(p));
     return slice_bytes(i ? i->n : 8) * (size_t)slice_count(p.lmax);
 }
+size_t slice_table_most(int lmax) { return slice_bytes(8) * (size_t)slice_count(lmax); }
 
 namespace {
 

@@ -176,6 +176,7 @@ cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s);
 // Two launches: the table of window slices into p.slices (16-byte aligned), then the coupling kernel.
 cudaError_t launch_chosen(const CouplingParams& p, cudaStream_t s);
 size_t slice_table_bytes(const CouplingParams& p);
+size_t slice_table_most(int lmax);  // for any list of slots
 // The table of square-root ratios (coef_bytes(lmax)), and whether launch_chosen reads one if p.coef has it.
 cudaError_t launch_coef(float4* t, int lmax, cudaStream_t s);
 bool reads_coef(const CouplingParams& p);

@@ -81,3 +81,23 @@ def test_plain_graph_beside_a_larger_quickpol(own):
         assert bool((a.replayed(g) == want).all())
         assert bool((a.direct() == want).all())
         del junk
+
+
+@pytest.mark.parametrize("lmax", [64, 520])  # without and with the table of square-root ratios
+@pytest.mark.parametrize("warm,then", [((0,), (2,)), ((2, 3), (0, 1)), ((0, 2, 3), (1, 2, 3))])
+def test_one_call_warms_up_the_grid(own, lmax, warm, then):
+    """A call with as many windows on the same grid is enough before a capture, whatever its spins."""
+    from powerspectra_gpu import Context
+    ctx, s = own
+    Call(ctx, warm, lmax, "chosen").direct()
+    b = Call(ctx, then, lmax, "chosen", seed=5)
+    g = b.record(s)
+    got = b.replayed(g).clone()
+    assert bool((got == b.direct()).all())
+    assert bool((b.replayed(g) == got).all())
+    Call(ctx, (2, 3), lmax + 100, "chosen").direct()  # its own, larger table
+    ref = Context(0)
+    ref.set_stream(s.cuda_stream)
+    c = Call(ref, then, lmax, "chosen", seed=5)
+    assert bool((c.direct() == got).all())
+    ref.close()
