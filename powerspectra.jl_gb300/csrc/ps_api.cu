@@ -32,6 +32,9 @@ void ps_linalg_wait_limit(ps_linalg* L, int limit);
 // and every index stays in 32 bits.
 #define PS_MAX_LMAX 16383
 
+// Largest lmax with a table of square-root ratios (961 MB).
+static const int kCoefMaxLmax = 4096;
+
 struct ps_ctx {
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -61,11 +64,12 @@ struct ps_ctx {
     int2* d_bf = nullptr;  // split (mantissa, exponent) windows for the chosen kernel
     size_t bf_cap = 0;
     unsigned char* d_slices = nullptr;  // its table of window slices, one launch at a time
-    // the chosen kernels' square-root ratios, for lmax up to coef_lmax
-    unsigned char* d_coef = nullptr;
-    size_t coef_cap = 0;
-    int coef_lmax = -1;
     size_t slices_cap = 0;
+    // the chosen kernels' square-root ratios, for lmax up to coef_lmax; none of coef_refused or more (no room), and
+    // the work done without since the last one was made
+    unsigned char* d_coef = nullptr;
+    int coef_lmax = -1, coef_refused = kCoefMaxLmax + 1;
+    double coef_due = 0.0;
     double* d_alm = nullptr;  // harmonic coefficients copied in by ps_window_W (2 doubles each)
     size_t alm_cap = 0;
     double* d_part = nullptr;  // alm2cl partial sums
@@ -144,13 +148,45 @@ static int set_err(ps_ctx* c, int code, const char* fmt, ...)
                            #call, cudaGetErrorString(e_), __FILE__, __LINE__);                               \
     } while (0)
 
+// Gives back what the context can do without (its streams are waited for by cudaFree); whether there was any.
+static bool give_back(ps_ctx* c)
+{
+    if (!c->d_coef) return false;
+    cudaFree(c->d_coef);
+    c->d_coef = nullptr;
+    c->coef_lmax = -1;
+    c->coef_refused = 0;  // and makes no other
+    return true;
+}
+
+// cudaMalloc for what a call needs: before it fails, the tables that only save time are given back.
+static cudaError_t dev_malloc(ps_ctx* c, void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back(c)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+// The same for a call that allocates by itself (ps_linalg.cu) before it does anything else.
+template <class Call>
+static int with_room(ps_ctx* c, Call call)
+{
+    const int st = call();
+    if (st != PS_ERR_OOM || !give_back(c)) return st;
+    cudaGetLastError();
+    return call();
+}
+
 static int ensure(ps_ctx* c, double** p, size_t* cap, size_t need)
 {
     if (need <= *cap) return PS_OK;
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc((void**)p, need * sizeof(double));
+    cudaError_t e = dev_malloc(c, (void**)p, need * sizeof(double));
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
@@ -195,7 +231,7 @@ static int upload_tasks(ps_ctx* c, const std::vector<int2>& t, int2** d, size_t*
         if (*d) cudaFree(*d);
         *d = nullptr;
         *cap = 0;
-        cudaError_t e = cudaMalloc((void**)d, t.size() * sizeof(int2));
+        cudaError_t e = dev_malloc(c, (void**)d, t.size() * sizeof(int2));
         if (e != cudaSuccess) {
             *d = nullptr;
             cudaGetLastError();
@@ -295,7 +331,7 @@ static int ensure_mtiles(ps_ctx* c, int lmin, int lmax)
 static int alloc_status(ps_ctx* c)
 {
     if (c->d_status) return PS_OK;
-    cudaError_t e = cudaMalloc((void**)&c->d_status, sizeof(unsigned));
+    cudaError_t e = dev_malloc(c, (void**)&c->d_status, sizeof(unsigned));
     if (e != cudaSuccess) {
         cudaGetLastError();
         c->d_status = nullptr;
@@ -377,9 +413,6 @@ void cov_window_spec(int kind, int k, int* product, int* parity)
 }
 }  // namespace ps
 
-// Launch the coupling kernel with event timing on the context stream.  A call
-// that launches several groups passes first/last so that the two events
-// bracket all of its coupling kernels (ps_last_kernel_ms).
 static int ensure_bytes(ps_ctx* c, unsigned char** p, size_t* cap, size_t need);
 
 // Whether work on s is being recorded (or can't be asked for, as for the legacy stream while another records).
@@ -394,14 +427,27 @@ static bool capturing(cudaStream_t s)
 // The chosen kernels' square-root ratios for rows up to lmax, kept by the context and replaced by larger ones.
 // None beyond kCoefMaxLmax, where there is no room, or in a capture (a table can't be made there, and a recorded
 // graph must not hold the address of one that may be replaced): the kernels then make them chunk by chunk.
-static const int kCoefMaxLmax = 4096;
+// A table costs some 110 us (allocation, fill, a synchronisation; measured at lmax 600, where it turned a first call of 237
+// us into one of 347) and saves about 2.2e-5 (lmax / 1000)^3 s a call, so it is made when the calls that went
+// without have lost what it costs: at once from lmax 1651 on, after 21 calls at lmax 600.
+static const double kCoefWork = 4.5e9;
 static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
 {
     *out = ps::CoefRows{};
-    if (lmax > kCoefMaxLmax || capturing(c->stream)) return PS_OK;
+    if (lmax >= c->coef_refused || capturing(c->stream)) return PS_OK;
     if (c->coef_lmax < lmax) {
+        c->coef_due += (double)lmax * lmax * lmax;
+        if (c->coef_due < kCoefWork) return PS_OK;
+        unsigned char* t = nullptr;
+        if (cudaMalloc((void**)&t, ps::coef_bytes(lmax)) != cudaSuccess) {
+            cudaGetLastError();
+            c->coef_refused = lmax;  // a smaller table stays
+            return PS_OK;
+        }
+        cudaFree(c->d_coef);
+        c->d_coef = t;
         c->coef_lmax = -1;
-        if (ensure_bytes(c, &c->d_coef, &c->coef_cap, ps::coef_bytes(lmax))) return PS_OK;
+        c->coef_due = 0.0;
         PS_CUDA(c, ps::launch_coef((float4*)c->d_coef, lmax, c->stream));
         PS_CUDA(c, cudaStreamSynchronize(c->stream));  // later calls may be on other streams
         c->launches++;
@@ -411,6 +457,9 @@ static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
     return PS_OK;
 }
 
+// Launch the coupling kernel with event timing on the context stream.  A call
+// that launches several groups passes first/last so that the two events
+// bracket all of its coupling kernels (ps_last_kernel_ms).
 static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first = true, bool last = true)
 {
     ps_ctx::Tiles& tiles = c->tiles[mode == PS_MODE_CHOSEN];
@@ -450,7 +499,7 @@ static int ensure_bytes(ps_ctx* c, unsigned char** p, size_t* cap, size_t need)
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc((void**)p, need);
+    cudaError_t e = dev_malloc(c, (void**)p, need);
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
@@ -466,7 +515,7 @@ static int ensure_int2(ps_ctx* c, int2** p, size_t* cap, size_t need)
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc((void**)p, need * sizeof(int2));
+    cudaError_t e = dev_malloc(c, (void**)p, need * sizeof(int2));
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
@@ -528,7 +577,7 @@ template <typename T>
 static int dev_upload(ps_ctx* c, T** dst, const std::vector<T>& v)
 {
     if (v.empty()) return PS_OK;
-    cudaError_t e = cudaMalloc((void**)dst, v.size() * sizeof(T));
+    cudaError_t e = dev_malloc(c, (void**)dst, v.size() * sizeof(T));
     if (e != cudaSuccess) {
         cudaGetLastError();
         *dst = nullptr;
@@ -1358,9 +1407,9 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         rows += (size_t)probs[i].K * wlen;
         max_wlen = std::max(max_wlen, wlen);
     }
-    cudaError_t e = cudaMalloc((void**)&b.d_win, rows * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b.d_bf, rows * sizeof(int2));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b.d_counter, sizeof(unsigned));
+    cudaError_t e = dev_malloc(c, (void**)&b.d_win, rows * sizeof(double));
+    if (e == cudaSuccess) e = dev_malloc(c, (void**)&b.d_bf, rows * sizeof(int2));
+    if (e == cudaSuccess) e = dev_malloc(c, (void**)&b.d_counter, sizeof(unsigned));
     if (e != cudaSuccess) {
         cudaGetLastError();
         batch_release(c);
@@ -1704,7 +1753,9 @@ int ps_decouple_covmat(ps_ctx* c, const double* Y, const double* B1, const doubl
     if (n < 1 || n > 65535 || ld < n || ldout < n) return set_err(c, PS_ERR_ARG, "need 1 <= n <= 65535, ld >= n");
     PS_CUDA(c, cudaSetDevice(c->device));
     if (!c->la) c->la = ps_linalg_new();
-    int st = ps_linalg_decouple(c->la, Y, B1, B2, (int)n, ld, out, ldout, c->stream, c->err, sizeof(c->err), false);
+    int st = with_room(c, [&] {
+        return ps_linalg_decouple(c->la, Y, B1, B2, (int)n, ld, out, ldout, c->stream, c->err, sizeof(c->err), false);
+    });
     if (!st) c->launches += 6;
     return st;
 }
@@ -1717,7 +1768,9 @@ int ps_decouple_covmat_device(ps_ctx* c, const double* dY, const double* dB1, co
     if (n < 1 || n > 65535 || ld < n || ldout < n) return set_err(c, PS_ERR_ARG, "need 1 <= n <= 65535, ld >= n");
     PS_CUDA(c, cudaSetDevice(c->device));
     if (!c->la) c->la = ps_linalg_new();
-    int st = ps_linalg_decouple(c->la, dY, dB1, dB2, (int)n, ld, dout, ldout, c->stream, c->err, sizeof(c->err), true);
+    int st = with_room(c, [&] {
+        return ps_linalg_decouple(c->la, dY, dB1, dB2, (int)n, ld, dout, ldout, c->stream, c->err, sizeof(c->err), true);
+    });
     if (!st) c->launches += 6;
     return st;
 }
@@ -1731,7 +1784,9 @@ int ps_solve(ps_ctx* c, const double* M, int64_t n, int64_t ldm, const double* b
         return set_err(c, PS_ERR_ARG, "need 1 <= n <= 65535, nrhs >= 1, leading dimensions >= n");
     PS_CUDA(c, cudaSetDevice(c->device));
     if (!c->la) c->la = ps_linalg_new();
-    int st = ps_linalg_solve(c->la, M, (int)n, ldm, b, nrhs, ldb, x, ldx, c->stream, c->err, sizeof(c->err));
+    int st = with_room(c, [&] {
+        return ps_linalg_solve(c->la, M, (int)n, ldm, b, nrhs, ldb, x, ldx, c->stream, c->err, sizeof(c->err));
+    });
     if (!st) c->launches += 2;
     return st;
 }
