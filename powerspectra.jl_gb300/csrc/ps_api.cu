@@ -88,6 +88,7 @@ struct ps_ctx {
     // batched workload state (ps_batch_*)
     struct Batch {
         bool ready = false;
+        bool recorded = false;  // a caller's graph may hold the addresses of its tables
         int nitems = 0, npreps = 0, max_wlen = 0, group_slots = 4, blocks = 0;
         ps::CouplingParams* d_groups = nullptr;
         int4* d_items = nullptr;
@@ -148,15 +149,37 @@ static int set_err(ps_ctx* c, int code, const char* fmt, ...)
                            #call, cudaGetErrorString(e_), __FILE__, __LINE__);                               \
     } while (0)
 
-// Gives back what the context can do without (its streams are waited for by cudaFree); whether there was any.
+// Gives back what the context can do without; whether there was any.
 static bool give_back(ps_ctx* c)
 {
-    if (!c->d_coef) return false;
-    cudaFree(c->d_coef);
-    c->d_coef = nullptr;
-    c->coef_lmax = -1;
-    c->coef_refused = 0;  // and makes no other
-    return true;
+    bool any = false;
+    auto drop = [&](unsigned char*& p) {
+        if (!p) return;
+        cudaFree(p);  // waits for what runs
+        p = nullptr;
+        any = true;
+    };
+    drop(c->d_coef);
+    if (any) {
+        c->coef_lmax = -1;
+        c->coef_refused = 0;  // and makes no other
+    }
+    ps_ctx::Batch& b = c->batch;
+    if (b.ready && !b.recorded && (b.d_coef || (b.d_slices && !b.launches))) {
+        drop(b.d_coef);
+        if (!b.launches) drop(b.d_slices);  // one launch per group needs its slices
+        b.max_slice_lmax = 0;
+        for (auto& g : b.host_groups) {
+            g.coef = ps::CoefRows{};
+            if (!b.launches) g.slices = nullptr;
+        }
+        cudaMemcpyAsync(b.d_groups, b.host_groups.data(), b.host_groups.size() * sizeof(ps::CouplingParams),
+                        cudaMemcpyHostToDevice, c->stream);
+        cudaStreamSynchronize(c->stream);
+        if (b.exec) cudaGraphExecDestroy(b.exec);  // recorded anew by the next launch
+        b.exec = nullptr;
+    }
+    return any;
 }
 
 // cudaMalloc for what a call needs: before it fails, the tables that only save time are given back.
@@ -573,8 +596,9 @@ static void batch_release(ps_ctx* c)
     b = ps_ctx::Batch();
 }
 
+// Room for a vector on the device, and its copy.
 template <typename T>
-static int dev_upload(ps_ctx* c, T** dst, const std::vector<T>& v)
+static int dev_room(ps_ctx* c, T** dst, const std::vector<T>& v)
 {
     if (v.empty()) return PS_OK;
     cudaError_t e = dev_malloc(c, (void**)dst, v.size() * sizeof(T));
@@ -583,6 +607,12 @@ static int dev_upload(ps_ctx* c, T** dst, const std::vector<T>& v)
         *dst = nullptr;
         return set_err(c, PS_ERR_OOM, "cudaMalloc of %zu bytes failed: %s", v.size() * sizeof(T), cudaGetErrorString(e));
     }
+    return PS_OK;
+}
+template <typename T>
+static int dev_upload(ps_ctx* c, T** dst, const std::vector<T>& v)
+{
+    if (v.empty()) return PS_OK;
     PS_CUDA(c, cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
     return PS_OK;
 }
@@ -1524,39 +1554,6 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
             }
         }
     }
-    // the groups' tables of window slices: one for the launches in turn; one each for the persistent
-    // kernel, whose groups run side by side (none for small lmax, or where there is no room)
-    size_t slice_bytes = 0, slice_cap = 0;
-    std::vector<size_t> slice_at(groups.size(), 0);
-    for (size_t g = 0; g < groups.size(); ++g) {
-        if (bps < 0) {
-            slice_bytes = std::max(slice_bytes, ps::slice_table_bytes(groups[g]));
-            continue;
-        }
-        const size_t need = (ps::batch_slice_bytes(groups[g].lmax, gs) + 255) / 256 * 256;
-        const bool has = groups[g].lmax >= ps::kSliceMinLmax && slice_bytes + need <= kBatchSliceBytes;
-        slice_at[g] = has ? slice_bytes : kNone;
-        if (has) slice_bytes += need;
-    }
-    if (slice_bytes && (st = ensure_bytes(c, &b.d_slices, &slice_cap, slice_bytes)) && bps < 0) {
-        batch_release(c);
-        return st;
-    }
-    for (size_t g = 0; g < groups.size() && b.d_slices; ++g) {
-        if (slice_at[g] == kNone) continue;
-        groups[g].slices = b.d_slices + slice_at[g];
-        b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
-    }
-    // and one table of the square-root ratios (the batch's own: a context's may be replaced by a larger one)
-    int max_lmax = 0;
-    for (const auto& g : groups) max_lmax = std::max(max_lmax, g.lmax);
-    if (!groups.empty() && max_lmax <= kCoefMaxLmax) {
-        size_t cap = 0;
-        if (ensure_bytes(c, &b.d_coef, &cap, ps::coef_bytes(max_lmax)) == PS_OK) {
-            PS_CUDA(c, ps::launch_coef((float4*)b.d_coef, max_lmax, c->stream));
-            for (auto& g : groups) g.coef = ps::coef_rows((const float4*)b.d_coef, max_lmax);
-        }
-    }
     b.ngroups = (int)groups.size();
     // items of one kernel body together (warps of an SM then share their
     // instruction stream), longest first within each body
@@ -1582,24 +1579,61 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         tasks.insert(tasks.end(), one.begin(), one.end());
         task_of.push_back({key, {off, (int)(tasks.size() - off)}});
     }
+    // what the batch needs, then what only saves time
+    int tab_lmax = 0;  // one table of B tiles for the tensor-core launches in turn: the size of the largest lmax
+    for (const auto& mp : b.host_mma) tab_lmax = std::max(tab_lmax, mp.lmax);
+    size_t btab_cap = 0;
+    if ((st = dev_room(c, &b.d_groups, groups)) || (st = dev_room(c, &b.d_items, sorted)) ||
+        (st = dev_room(c, &b.d_preps, preps)) || (st = dev_room(c, &b.d_tasks, tasks)) ||
+        (st = dev_room(c, &b.d_mtiles, mtiles)) || (!b.host_mma.empty() && (st = alloc_status(c))) ||
+        (!b.host_mma.empty() && (st = ensure_bytes(c, &b.d_btab, &btab_cap, ps::mma_table_bytes(tab_lmax))))) {
+        batch_release(c);
+        return st;
+    }
+    // the groups' tables of window slices: one for the launches in turn; one each for the persistent
+    // kernel, whose groups run side by side (none for small lmax, or where there is no room)
+    size_t slice_bytes = 0, slice_cap = 0;
+    std::vector<size_t> slice_at(groups.size(), 0);
+    for (size_t g = 0; g < groups.size(); ++g) {
+        if (bps < 0) {
+            slice_bytes = std::max(slice_bytes, ps::slice_table_bytes(groups[g]));
+            continue;
+        }
+        const size_t need = (ps::batch_slice_bytes(groups[g].lmax, gs) + 255) / 256 * 256;
+        const bool has = groups[g].lmax >= ps::kSliceMinLmax && slice_bytes + need <= kBatchSliceBytes;
+        slice_at[g] = has ? slice_bytes : kNone;
+        if (has) slice_bytes += need;
+    }
+    if (slice_bytes && bps < 0 && (st = ensure_bytes(c, &b.d_slices, &slice_cap, slice_bytes))) {
+        batch_release(c);
+        return st;
+    }
+    auto optional = [](unsigned char** p, size_t bytes) {
+        if (cudaMalloc((void**)p, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+        return false;
+    };
+    if (slice_bytes && bps >= 0) optional(&b.d_slices, slice_bytes);
+    for (size_t g = 0; g < groups.size() && b.d_slices; ++g) {
+        if (slice_at[g] == kNone) continue;
+        groups[g].slices = b.d_slices + slice_at[g];
+        b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
+    }
+    // and one table of the square-root ratios (the batch's own: a context's may be replaced by a larger one)
+    int max_lmax = 0;
+    for (const auto& g : groups) max_lmax = std::max(max_lmax, g.lmax);
+    if (!groups.empty() && max_lmax <= kCoefMaxLmax) {
+        if (optional(&b.d_coef, ps::coef_bytes(max_lmax))) {
+            PS_CUDA(c, ps::launch_coef((float4*)b.d_coef, max_lmax, c->stream));
+            for (auto& g : groups) g.coef = ps::coef_rows((const float4*)b.d_coef, max_lmax);
+        }
+    }
     if ((st = dev_upload(c, &b.d_groups, groups)) || (st = dev_upload(c, &b.d_items, sorted)) ||
         (st = dev_upload(c, &b.d_preps, preps)) || (st = dev_upload(c, &b.d_tasks, tasks)) ||
         (st = dev_upload(c, &b.d_mtiles, mtiles))) {
         batch_release(c);
         return st;
-    }
-    if (!b.host_mma.empty() && (st = alloc_status(c))) {
-        batch_release(c);
-        return st;
-    }
-    if (!b.host_mma.empty()) {  // one table for the launches in turn: the size of the largest lmax
-        int tab_lmax = 0;
-        for (const auto& mp : b.host_mma) tab_lmax = std::max(tab_lmax, mp.lmax);
-        size_t cap = 0;
-        if ((st = ensure_bytes(c, &b.d_btab, &cap, ps::mma_table_bytes(tab_lmax)))) {
-            batch_release(c);
-            return st;
-        }
     }
     for (size_t m = 0; m < b.host_mma.size(); ++m) {
         b.host_mma[m].tiles = b.d_mtiles + mma_tile_off[m];
@@ -1671,6 +1705,7 @@ int ps_batch_run(ps_ctx* c)
     if (!c->batch.ready) return set_err(c, PS_ERR_ARG, "ps_batch_prepare has not been called");
     PS_CUDA(c, cudaSetDevice(c->device));
     int st;
+    if (capturing(c->stream)) c->batch.recorded = true;
     if (!c->batch.host_mma.empty() && (st = arm_status(c, c->stream))) return st;
     if ((st = batch_enqueue(c, c->stream))) return st;
     c->launches += batch_kernel_count(c->batch);

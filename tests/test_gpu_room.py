@@ -33,6 +33,7 @@ class Pair:
         self.M = torch.zeros((2, self.n, self.n), dtype=torch.float64, device="cuda")
 
     def __call__(self):
+        torch.cuda.synchronize()  # the context has a stream of its own
         self.ctx.mcm_multi_device({2: self.W.data_ptr(), 3: self.W.data_ptr()}, self.nW, 0, self.lmax,
                                   {2: self.M[0].data_ptr(), 3: self.M[1].data_ptr()}, self.n, mode="chosen")
         torch.cuda.synchronize()
@@ -41,9 +42,7 @@ class Pair:
 
 def _context():
     from powerspectra_gpu import Context
-    ctx = Context(0)
-    ctx.set_stream(torch.cuda.current_stream().cuda_stream)
-    return ctx
+    return Context(0)
 
 
 def test_no_table_for_one_call():
@@ -95,6 +94,76 @@ def test_no_room_for_a_table():
         assert bool((b() == want[1]).all())
         assert bool((a() == want[0]).all())
     assert _free() == before
+    del hold
+    torch.cuda.empty_cache()
+    ctx.close()
+
+
+class Batch:
+    """TT, TE, ++ and -- of one window each on uneven grids."""
+
+    def __init__(self, ctx, sizes):
+        from powerspectra_gpu import synthetic as syn
+        self.ctx, self.probs, self.keep = ctx, [], []
+        for i, lmax in enumerate(sizes):
+            n = lmax + 1
+            W = torch.tensor(syn.mask_spectrum(n, 0.5, n / 3.0, seed=i), device="cuda")
+            M = torch.zeros((4, n, n), dtype=torch.float64, device="cuda")
+            self.keep.append((W, M))
+            self.probs.append({"lmin": 0, "lmax": lmax, "cases": 0xF, "nW": n, "ldm": n, "W": [W.data_ptr()],
+                               "M": [M[s].data_ptr() for s in range(4)]})
+
+    def prepare(self, **kw):
+        self.ctx.batch_prepare(self.probs, **kw)
+
+    def run(self, how):
+        for _, M in self.keep:
+            M.zero_()
+        torch.cuda.synchronize()  # the context has a stream of its own
+        how()
+        torch.cuda.synchronize()
+
+    def matrices(self):
+        return [M.clone() for _, M in self.keep]
+
+    def equal(self, want):
+        return all(bool((M == w).all()) for (_, M), w in zip(self.keep, want))
+
+
+@pytest.mark.parametrize("form", [0, -1])
+def test_batch_with_little_room(form):
+    ctx = _context()
+    b = Batch(ctx, range(900, 964))  # 131 MB of slices and 55 of ratios; 20 MB of what it needs
+    b.prepare(blocks_per_sm=form)
+    b.run(ctx.batch_run)
+    want = b.matrices()
+    for leave in range(230, 30, -20):
+        ctx2 = _context()
+        b.ctx = ctx2
+        hold = _hold(leave << 20)
+        b.prepare(blocks_per_sm=form)
+        b.run(ctx2.batch_run)
+        del hold
+        torch.cuda.empty_cache()
+        ctx2.close()
+        assert b.equal(want), leave
+    ctx.close()
+
+
+@pytest.mark.parametrize("form", [0, -1])
+def test_batch_tables_given_back(form):
+    ctx = _context()
+    b = Batch(ctx, range(900, 964))
+    b.prepare(blocks_per_sm=form)
+    b.run(ctx.batch_graph_launch)
+    want = b.matrices()
+    hold = _hold(64 << 20)
+    x = np.linspace(1.0, 2.0, 3800)
+    lmax = 3799 if form == 0 else 3199  # 115 MB, or 82 where the ratios alone come back
+    assert np.all(np.isfinite(ctx.mcm(0, x, 0, lmax, mode="chosen")))
+    for how in (ctx.batch_run, ctx.batch_graph_launch):
+        b.run(how)
+        assert b.equal(want)
     del hold
     torch.cuda.empty_cache()
     ctx.close()
