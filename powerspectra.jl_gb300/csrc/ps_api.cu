@@ -102,8 +102,9 @@ struct ps_ctx {
         bool launches = false;
         std::vector<ps::CouplingParams> host_groups;
         int2* d_tasks = nullptr;
-        unsigned char* d_slices = nullptr;  // the groups' tables of window slices
-        unsigned char* d_coef = nullptr;    // the square-root ratios of all of them
+        unsigned char* d_slices = nullptr;  // the launches' table of window slices (one at a time)
+        unsigned char* d_tables = nullptr;  // what only saves time: slices of the queue's groups, square-root ratios
+        bool coef = false;                  // there are ratios among them
         int ngroups = 0, max_slice_lmax = 0;  // the largest lmax with a table (0: no tables)
         // tensor-core launches (the problems' TT slots and ++/-- slots when there are
         // mma_min_slots of them), enqueued before the CUDA-core part,
@@ -165,9 +166,9 @@ static bool give_back(ps_ctx* c)
         c->coef_refused = 0;  // and makes no other
     }
     ps_ctx::Batch& b = c->batch;
-    if (b.ready && !b.recorded && (b.d_coef || (b.d_slices && !b.launches))) {
-        drop(b.d_coef);
-        if (!b.launches) drop(b.d_slices);  // one launch per group needs its slices
+    if (b.ready && !b.recorded && b.d_tables) {
+        drop(b.d_tables);
+        b.coef = false;
         b.max_slice_lmax = 0;
         for (auto& g : b.host_groups) {
             g.coef = ps::CoefRows{};
@@ -590,7 +591,7 @@ static void batch_release(ps_ctx* c)
     cudaFree(b.d_bf);
     cudaFree(b.d_tasks);
     cudaFree(b.d_slices);
-    cudaFree(b.d_coef);
+    cudaFree(b.d_tables);
     cudaFree(b.d_mtiles);
     cudaFree(b.d_btab);
     b = ps_ctx::Batch();
@@ -1414,6 +1415,41 @@ int ps_mcm_set(ps_ctx* c, unsigned cases, const double* const* W, int K, int64_t
 // Groups past it have none.
 static const size_t kBatchSliceBytes = (size_t)2 << 30, kNone = ~(size_t)0;
 
+// Whether one launch per group is worth a table of square-root ratios, which costs the preparation some 100 us.  In a row
+// of launches it saves about 1 us a launch and 2.2e-5 (lmax / 1000)^3 s (200 ++/-- of lmax 20-200 3432 us without and 3214
+// with it, 8 of all spins and lmax 100-600 852 and 805): it is made where ten runs pay for it.
+static bool launches_read_coef(const std::vector<ps::CouplingParams>& groups, int* lmax)
+{
+    double us = 0.0;
+    for (const auto& g : groups)
+        if (ps::has_coef(g)) {
+            us += 1.0 + 2.2e-8 * g.lmax * g.lmax * g.lmax;
+            *lmax = std::max(*lmax, g.lmax);
+        }
+    return us >= 10.0;
+}
+// Whether the persistent kernel's groups with a (2 -2 0) family read one.  The table saves instructions and costs a
+// task's first chunk a wait for its copies.  So it is for queues that keep the warps busy while the longest item
+// runs (n x lmax, ++/-- without and with: 1 x 1000 1.54 and 1.64 ms, 2 x 1000 1.74 and 1.84, 4 x 1000 2.38 and 2.33, 8 x 1000
+// 4.40 and 4.20; 4 x 500 656 and 688 us, 8 x 500 747 and 712) and whose tasks are some 70 steps long on average (2000 x 32
+// 330 and 458 us, 800 x 64 443 and 457, 300 x 100 423 and 410, 64 x 400 2.62 and 2.49 ms).  One problem beyond
+// kCoefMaxLmax leaves the others without: the kernel reads it for all or none.
+static bool queue_reads_coef(const std::vector<ps::CouplingParams>& groups, const std::vector<int4>& items, int gs,
+                             int nsm, int* lmax)
+{
+    double work = 0.0, tasks = 0.0, longest = 0.0;
+    for (const int4& it : items) {
+        if (!(it.w >> 8 & 2)) continue;  // the (0 0 0) family alone
+        const double n = it.w & 0xff, w = n * (2.0 * it.y + 1.0);
+        work += w;
+        tasks += n;
+        longest = std::max(longest, w);
+        *lmax = std::max(*lmax, groups[it.x].lmax);
+    }
+    const double warps = (double)nsm * ps::batch_blocks_per_sm(gs, true) * ps::kWarpsPerBlock;
+    return gs <= 4 && tasks > 0.0 && work >= 0.7 * warps * longest && work >= 70.0 * tasks;
+}
+
 int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int bps)
 {
     if (!c) return PS_ERR_ARG;
@@ -1425,6 +1461,8 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
     if (gs != 2 && gs != 4 && gs != 8) return set_err(c, PS_ERR_ARG, "group_slots must be 2, 4 or 8 (got %d)", gs);
     if (bps == 0) bps = c->tuned_blocks_per_sm;
     PS_CUDA(c, cudaSetDevice(c->device));
+    int nsm = 0;
+    PS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     batch_release(c);
     ps_ctx::Batch& b = c->batch;
     // window rows
@@ -1590,44 +1628,54 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         batch_release(c);
         return st;
     }
-    // the groups' tables of window slices: one for the launches in turn; one each for the persistent
-    // kernel, whose groups run side by side (none for small lmax, or where there is no room)
+    // window slices: the launches share one table in turn, which they need; the persistent kernel's groups run side by
+    // side, with a table each for all but the smallest
     size_t slice_bytes = 0, slice_cap = 0;
-    std::vector<size_t> slice_at(groups.size(), 0);
+    std::vector<size_t> slice_at(groups.size(), kNone);
     for (size_t g = 0; g < groups.size(); ++g) {
         if (bps < 0) {
             slice_bytes = std::max(slice_bytes, ps::slice_table_bytes(groups[g]));
             continue;
         }
         const size_t need = (ps::batch_slice_bytes(groups[g].lmax, gs) + 255) / 256 * 256;
-        const bool has = groups[g].lmax >= ps::kSliceMinLmax && slice_bytes + need <= kBatchSliceBytes;
-        slice_at[g] = has ? slice_bytes : kNone;
-        if (has) slice_bytes += need;
+        if (groups[g].lmax < ps::slice_min_lmax(groups[g]) || slice_bytes + need > kBatchSliceBytes) continue;
+        slice_at[g] = slice_bytes;
+        slice_bytes += need;
     }
-    if (slice_bytes && bps < 0 && (st = ensure_bytes(c, &b.d_slices, &slice_cap, slice_bytes))) {
-        batch_release(c);
-        return st;
+    if (bps < 0 && slice_bytes) {
+        if ((st = ensure_bytes(c, &b.d_slices, &slice_cap, slice_bytes))) {
+            batch_release(c);
+            return st;
+        }
+        for (auto& g : groups) g.slices = b.d_slices;
+        slice_bytes = 0;
     }
-    auto optional = [](unsigned char** p, size_t bytes) {
-        if (cudaMalloc((void**)p, bytes) == cudaSuccess) return true;
+    // and one table of the square-root ratios (the batch's own: a context's may be replaced by a larger one), as
+    // long as the groups that read it need.  One allocation for both (some 100 us); without room for both, slices alone
+    int coef_lmax = 0;
+    const bool use_coef = bps < 0 ? launches_read_coef(groups, &coef_lmax)
+                                  : queue_reads_coef(groups, items, gs, nsm, &coef_lmax);
+    const size_t coef_bytes = use_coef && coef_lmax <= kCoefMaxLmax ? ps::coef_bytes(coef_lmax) : 0;
+    auto optional = [&](size_t bytes) {
+        if (!bytes) return false;
+        if (cudaMalloc((void**)&b.d_tables, bytes) == cudaSuccess) return true;
         cudaGetLastError();
-        *p = nullptr;
+        b.d_tables = nullptr;
         return false;
     };
-    if (slice_bytes && bps >= 0) optional(&b.d_slices, slice_bytes);
-    for (size_t g = 0; g < groups.size() && b.d_slices; ++g) {
-        if (slice_at[g] == kNone) continue;
-        groups[g].slices = b.d_slices + slice_at[g];
-        b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
-    }
-    // and one table of the square-root ratios (the batch's own: a context's may be replaced by a larger one)
-    int max_lmax = 0;
-    for (const auto& g : groups) max_lmax = std::max(max_lmax, g.lmax);
-    if (!groups.empty() && max_lmax <= kCoefMaxLmax) {
-        if (optional(&b.d_coef, ps::coef_bytes(max_lmax))) {
-            PS_CUDA(c, ps::launch_coef((float4*)b.d_coef, max_lmax, c->stream));
-            for (auto& g : groups) g.coef = ps::coef_rows((const float4*)b.d_coef, max_lmax);
+    b.coef = coef_bytes && optional(slice_bytes + coef_bytes);
+    if (b.coef || optional(slice_bytes)) {
+        for (size_t g = 0; g < groups.size(); ++g) {
+            if (slice_at[g] == kNone) continue;
+            groups[g].slices = b.d_tables + slice_at[g];
+            b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
         }
+    }
+    if (b.coef) {
+        const float4* t = (const float4*)(b.d_tables + slice_bytes);
+        PS_CUDA(c, ps::launch_coef((float4*)t, coef_lmax, c->stream));
+        for (auto& g : groups)
+            if (g.lmax <= coef_lmax) g.coef = ps::coef_rows(t, coef_lmax);
     }
     if ((st = dev_upload(c, &b.d_groups, groups)) || (st = dev_upload(c, &b.d_items, sorted)) ||
         (st = dev_upload(c, &b.d_preps, preps)) || (st = dev_upload(c, &b.d_tasks, tasks)) ||
@@ -1650,9 +1698,7 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
             }
     }
     PS_CUDA(c, cudaStreamSynchronize(c->stream));
-    int nsm = 0;
-    PS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    int occ = ps::batch_blocks_per_sm(gs);
+    const int occ = ps::batch_blocks_per_sm(gs, b.coef);
     if (bps == 0) bps = occ;
     b.launches = bps < 0;
     if (!b.launches && (bps < 1 || bps > occ)) bps = occ;
@@ -1682,7 +1728,7 @@ static int batch_enqueue(ps_ctx* c, cudaStream_t s)
         bp.groups = b.d_groups;
         bp.items = b.d_items;
         bp.nitems = b.nitems;
-        bp.coef = b.d_coef != nullptr;
+        bp.coef = b.coef;
         bp.counter = b.d_counter;
         if (b.max_slice_lmax)
             PS_CUDA(c, ps::launch_batch_slices(b.d_groups, b.ngroups, b.max_slice_lmax, b.group_slots, s));
@@ -1755,7 +1801,7 @@ int ps_batch_autotune(ps_ctx* c, const ps_problem* probs, int nprob, int* best_g
     double best = 1e300;
     int bg = 4, bb = 0, st;
     for (int gi = 0; gi < 3; ++gi) {
-        int occ = ps::batch_blocks_per_sm(cand_gs[gi]);
+        const int occ = std::max(ps::batch_blocks_per_sm(cand_gs[gi], false), ps::batch_blocks_per_sm(cand_gs[gi], true));
         for (int bps = -1; bps <= occ; ++bps) {  // -1: one launch per group
             if (bps == 0) continue;
             if ((st = ps_batch_prepare(c, probs, nprob, cand_gs[gi], bps))) return st;

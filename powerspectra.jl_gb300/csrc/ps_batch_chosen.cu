@@ -112,12 +112,11 @@ cudaError_t launch_batch_chosen(const BatchParams& bp, int blocks, int nwin, cud
     return cudaGetLastError();
 }
 
-int batch_blocks_per_sm(int nwin)
+int batch_blocks_per_sm(int nwin, bool coef)
 {
     int n = 0;
-    cudaError_t e = nwin > 4 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_chosen<8, false>, kWarpsPerBlock * 32, 0)
-                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_chosen<4, true>, kWarpsPerBlock * 32, 0);
-    if (e != cudaSuccess) {
+    const auto kernel = nwin > 4 ? k_batch_chosen<8, false> : (coef ? k_batch_chosen<4, true> : k_batch_chosen<4, false>);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kWarpsPerBlock * 32, 0) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }

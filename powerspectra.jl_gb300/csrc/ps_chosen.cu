@@ -41,11 +41,12 @@ const Inst* find_inst(const CouplingParams& p, uint32_t spec)  // null: launch_c
 // Below lmax 512 the copies of a warp's first chunk wait longer than its square roots take (TT, TE and ++/--
 // together, without and with the table: lmax 95 55.8 and 55.6 us, ++ alone 38.0 and 43.3; 383 83.7 and 84.8; 767
 // 268.0 and 258.5).
-bool reads_coef(const CouplingParams& p)
+bool has_coef(const CouplingParams& p)
 {
     const Inst* i = find_inst(p, spec_of(p));
-    return p.lmax >= 512 && i && i->coef;
+    return i && i->coef;
 }
+bool reads_coef(const CouplingParams& p) { return p.lmax >= 512 && has_coef(p); }
 
 size_t slice_table_bytes(const CouplingParams& p)
 {

@@ -169,7 +169,7 @@ struct BatchParams {
 // Launchers (ps_plain_fp64.cu, ps_chosen.cu).
 // The batched kernel with NWIN = 4 or 8 slots per group (nwin > 4 selects 8).
 cudaError_t launch_batch_chosen(const BatchParams& bp, int blocks, int nwin, cudaStream_t s);
-int batch_blocks_per_sm(int nwin);
+int batch_blocks_per_sm(int nwin, bool coef);  // of the kernel that launch_batch_chosen takes
 int chosen_batch_template(const CouplingParams& p, int nwin);  // compile-time slot set of a batch group (0: none fits)
 cudaError_t launch_prep_windows(const WinPrep* list, int n, int max_wlen, cudaStream_t s);
 cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s);
@@ -180,10 +180,17 @@ size_t slice_table_most(int lmax);  // for any list of slots
 // The table of square-root ratios (coef_bytes(lmax)), and whether launch_chosen reads one if p.coef has it.
 cudaError_t launch_coef(float4* t, int lmax, cudaStream_t s);
 bool reads_coef(const CouplingParams& p);
+bool has_coef(const CouplingParams& p);  // ... at any lmax
 // Smaller lmax in a batch: no table, each warp makes its few slices itself.  Then a table holds more slices than are
-// read: 2000 problems up to lmax 32 took 158 us without and 224 with tables, 64 of lmax 96-128 167 and 169,
-// 256 of lmax 128-200 1252 and 1232.
-constexpr int kSliceMinLmax = 128;
+// read (its launch on top: all spins, n x lmax, without and with, 2000 x 32 516 and 607 us, 300 x 100 612 and 629, 200 x 127 660
+// and 662, 100 x 250 1496 and 1420; the (0 0 0) family alone, with half the steps, 4 x 200 93 and 101, 100 x 250 777 and 779, 64 x 400
+// 1540 and 1519, 1 x 500 279 and 260).
+inline int slice_min_lmax(const CouplingParams& g)
+{
+    for (int k = 0; k < g.nwin; ++k)
+        if (g.win[k].product != PROD_00_00) return 128;
+    return 300;
+}
 // The slice tables of a batch's groups (NWIN = 4 or 8 as for launch_batch_chosen), each into its group's
 // own p.slices of batch_slice_bytes(lmax, nwin).
 cudaError_t launch_batch_slices(const CouplingParams* groups, int ngroups, int max_lmax, int nwin, cudaStream_t s);
