@@ -105,7 +105,8 @@ struct ps_ctx {
         unsigned char* d_slices = nullptr;  // the launches' table of window slices (one at a time)
         unsigned char* d_tables = nullptr;  // what only saves time: slices of the queue's groups, square-root ratios
         bool coef = false;                  // there are ratios among them
-        int ngroups = 0, max_slice_lmax = 0;  // the largest lmax with a table (0: no tables)
+        const int2* d_sblocks = nullptr;    // which slices each block of their kernel makes (none: no slices)
+        int nsblocks = 0;
         // tensor-core launches (the problems' TT slots and ++/-- slots when there are
         // mma_min_slots of them), enqueued before the CUDA-core part,
         // with the block lists of every distinct (lmin, lmax) in d_mtiles
@@ -169,7 +170,7 @@ static bool give_back(ps_ctx* c)
     if (b.ready && !b.recorded && b.d_tables) {
         drop(b.d_tables);
         b.coef = false;
-        b.max_slice_lmax = 0;
+        b.nsblocks = 0;
         for (auto& g : b.host_groups) {
             g.coef = ps::CoefRows{};
             if (!b.launches) g.slices = nullptr;
@@ -1592,7 +1593,6 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
             }
         }
     }
-    b.ngroups = (int)groups.size();
     // items of one kernel body together (warps of an SM then share their
     // instruction stream), longest first within each body
     std::vector<int> order(items.size());
@@ -1642,6 +1642,14 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         slice_at[g] = slice_bytes;
         slice_bytes += need;
     }
+    std::vector<int2> sblocks;
+    for (size_t g = 0; g < groups.size(); ++g)
+        if (slice_at[g] != kNone)
+            for (int k = 0; k < groups[g].nwin; ++k)
+                for (int i = 0; i < ps::slice_entries(groups[g].lmax); i += ps::kSliceBlock)
+                    sblocks.push_back(make_int2((int)g, k << 24 | i));
+    const size_t sblocks_at = slice_bytes;
+    slice_bytes += (sblocks.size() * sizeof(int2) + 255) / 256 * 256;
     if (bps < 0 && slice_bytes) {
         if ((st = ensure_bytes(c, &b.d_slices, &slice_cap, slice_bytes))) {
             batch_release(c);
@@ -1668,8 +1676,14 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
         for (size_t g = 0; g < groups.size(); ++g) {
             if (slice_at[g] == kNone) continue;
             groups[g].slices = b.d_tables + slice_at[g];
-            b.max_slice_lmax = std::max(b.max_slice_lmax, groups[g].lmax);
         }
+        int2* list = (int2*)(b.d_tables + sblocks_at);
+        if ((st = dev_upload(c, &list, sblocks))) {
+            batch_release(c);
+            return st;
+        }
+        b.d_sblocks = list;
+        b.nsblocks = (int)sblocks.size();
     }
     if (b.coef) {
         const float4* t = (const float4*)(b.d_tables + slice_bytes);
@@ -1730,8 +1744,7 @@ static int batch_enqueue(ps_ctx* c, cudaStream_t s)
         bp.nitems = b.nitems;
         bp.coef = b.coef;
         bp.counter = b.d_counter;
-        if (b.max_slice_lmax)
-            PS_CUDA(c, ps::launch_batch_slices(b.d_groups, b.ngroups, b.max_slice_lmax, b.group_slots, s));
+        if (b.nsblocks) PS_CUDA(c, ps::launch_batch_slices(b.d_groups, b.d_sblocks, b.nsblocks, b.group_slots, s));
         PS_CUDA(c, ps::launch_batch_chosen(bp, b.blocks, b.group_slots, s));
     }
     PS_CUDA(c, cudaEventRecord(c->ev1, s));
@@ -1741,7 +1754,7 @@ static int batch_enqueue(ps_ctx* c, cudaStream_t s)
 // kernels one run of the batch launches (window preparation included)
 static size_t batch_kernel_count(const ps_ctx::Batch& b)
 {
-    const size_t one = b.nitems > 0 ? 1 + (b.max_slice_lmax != 0) : 0;  // the persistent kernel and its tables
+    const size_t one = b.nitems > 0 ? 1 + (b.nsblocks != 0) : 0;  // the persistent kernel and its tables
     return 1 + 2 * b.host_mma.size() + (b.launches ? 2 * b.host_groups.size() : one);
 }
 

@@ -191,9 +191,12 @@ inline int slice_min_lmax(const CouplingParams& g)
         if (g.win[k].product != PROD_00_00) return 128;
     return 300;
 }
-// The slice tables of a batch's groups (NWIN = 4 or 8 as for launch_batch_chosen), each into its group's
-// own p.slices of batch_slice_bytes(lmax, nwin).
-cudaError_t launch_batch_slices(const CouplingParams* groups, int ngroups, int max_lmax, int nwin, cudaStream_t s);
+// The slice tables of a batch's groups (NWIN = 4 or 8 as for launch_batch_chosen), each into its group's own p.slices
+// of batch_slice_bytes(lmax, nwin): block b makes kSliceBlock entries of group blocks[b].x, from entry blocks[b].y &
+// 0xffffff of slice_entries(lmax), of window blocks[b].y >> 24.
+constexpr int kSliceBlock = 64;
+cudaError_t launch_batch_slices(const CouplingParams* groups, const int2* blocks, int nblocks, int nwin, cudaStream_t s);
+int slice_entries(int lmax);
 size_t batch_slice_bytes(int lmax, int nwin);
 // K windows of nW entries (device pointers in a host array) into padded rows wW + k wlen of (2l+1) W[l]
 // and, when bf is given, their split copies bf + k wlen, one launch per kSetWindows windows.
