@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) k_batch_slices(const CouplingParams* __re
     const int n = min(slice_count(p.lmax), i0 + kSliceBlock), wlen = p.wlen;
     Slice<NWIN>* table = reinterpret_cast<Slice<NWIN>*>(p.slices);
     for (int i = i0 + (threadIdx.x >> 5); i < n; i += 8)
-        put_slice<NWIN>(table[i], i, k, wlen, lane, [&](int j) { return __ldg(bf + j); });
+        put_slice<NWIN>(table[i], k, load_split(i + kSlice0, wlen, lane, [&](int j) { return __ldg(bf + j); }), lane);
 }
 
 size_t batch_slice_bytes(int lmax, int nwin)

@@ -141,24 +141,34 @@ __device__ __forceinline__ int2 split_entry(double v)
     return v == 0.0 ? make_int2(0, kZeroExp) : make_int2(__float_as_int((float)m), e);
 }
 
-// One warp per entry and window: entry `i`, window `k`, at(j) its split value at l3 = j (inside 0 .. wlen - 1).
-template <int NWIN, class At>
-__device__ __forceinline__ void put_slice(Slice<NWIN>& s, int i, int k, int wlen, int lane, At at)
-{
+// One window's 64 split values from l3 on, zero outside 0 .. wlen - 1, two per lane: at(j) gives the one at j.
+struct SplitSlice {
     int2 v[kStagePerLane];
-    int emax = kZeroExp;
+};
+template <class At>
+__device__ __forceinline__ SplitSlice load_split(int l3, int wlen, int lane, At at)
+{
+    SplitSlice x;
 #pragma unroll
     for (int q = 0; q < kStagePerLane; ++q) {
-        const int j = i + kSlice0 + lane + 32 * q;
-        v[q] = j >= 0 && j < wlen ? at(j) : make_int2(0, kZeroExp);
-        emax = max(emax, v[q].y);
+        const int j = l3 + lane + 32 * q;
+        x.v[q] = j >= 0 && j < wlen ? at(j) : make_int2(0, kZeroExp);
     }
+    return x;
+}
+// They become window k of a slice, by one warp.
+template <int NWIN>
+__device__ __forceinline__ void put_slice(Slice<NWIN>& s, int k, const SplitSlice& x, int lane)
+{
+    int emax = kZeroExp;
+#pragma unroll
+    for (int q = 0; q < kStagePerLane; ++q) emax = max(emax, x.v[q].y);
     emax = __reduce_max_sync(0xffffffffu, emax);
 #pragma unroll
     for (int q = 0; q < kStagePerLane; ++q) {
         const int slot = lane + 32 * q;
         s.v[slots_interleaved<NWIN>() ? slot * NWIN + k : k * kSlots + slot] =
-            __int_as_float(v[q].x) * pow2f_or_zero(v[q].y - emax);
+            __int_as_float(x.v[q].x) * pow2f_or_zero(x.v[q].y - emax);
     }
     if (lane == 0) s.E[k] = emax;
 }
@@ -179,14 +189,14 @@ __global__ void __launch_bounds__(256) k_slices(const CouplingParams p)
     if (RAW) {
         const double* __restrict__ W = p.src[k];
         auto value = [&](int j) { return j < p.nw ? (2.0 * j + 1.0) * __ldg(W + j) : 0.0; };
-        put_slice<NWIN>(s, i, k, p.wlen, lane, [&](int j) { return split_entry(value(j)); });
+        put_slice<NWIN>(s, k, load_split(i + kSlice0, p.wlen, lane, [&](int j) { return split_entry(value(j)); }), lane);
         // entry i writes the row's value at its first l3, the last entry those that follow
         const int end = i + 1 == slice_count(p.lmax) ? p.wlen : i + kSlice0 + 1;
         for (int j = i + kSlice0 + lane; j < end; j += 32)
             if (j >= 0) const_cast<double*>(p.win[k].wW)[j] = value(j);
     } else {
         const int2* __restrict__ bf = p.win[k].bf;
-        put_slice<NWIN>(s, i, k, p.wlen, lane, [&](int j) { return __ldg(bf + j); });
+        put_slice<NWIN>(s, k, load_split(i + kSlice0, p.wlen, lane, [&](int j) { return __ldg(bf + j); }), lane);
     }
     let_next_start();
 }
@@ -204,18 +214,24 @@ __device__ __forceinline__ void fetch_slice(Slice<NWIN>& dst, const unsigned cha
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o), "l"(src + o) : "memory");
     }
 }
-// A slice from the table or, with OWN, made here for a group that has none.  A compile-time choice, as the
-// launches always have a table; the branch moves their kernels by -2 % (all spin cases) to +3 % (TT, 02).
+// A chunk's two slices (forward from l3 = lf, backward from lb), from the table or, with OWN, made here for a group that
+// has none: the values of both are on their way before either is scaled (one after the other, TT of 4 x lmax 200 took
+// 94 us against 86, all spins 180 against 170).  OWN is a compile-time choice, as the launches always have a table;
+// the branch moves their kernels by -2 % (all spin cases) to +3 % (TT, 02).
 template <int NWIN, bool OWN>
-__device__ __forceinline__ void get_slice(const CouplingParams& p, Slice<NWIN>& dst, int l3, int lane)
+__device__ __forceinline__ void get_slices(const CouplingParams& p, Slice<NWIN> (&dst)[2], int lf, int lb, int lane)
 {
     if (!OWN || p.slices) {
-        fetch_slice<NWIN>(dst, p.slices, l3, lane);
+        fetch_slice<NWIN>(dst[0], p.slices, lf, lane);
+        fetch_slice<NWIN>(dst[1], p.slices, lb, lane);
     } else {
 #pragma unroll 1
         for (int k = 0; k < p.nwin; ++k) {
             const int2* __restrict__ bf = p.win[k].bf;
-            put_slice<NWIN>(dst, l3 - kSlice0, k, p.wlen, lane, [&](int j) { return __ldg(bf + j); });
+            auto at = [&](int j) { return __ldg(bf + j); };
+            const SplitSlice f = load_split(lf, p.wlen, lane, at), b = load_split(lb, p.wlen, lane, at);
+            put_slice<NWIN>(dst[0], k, f, lane);
+            put_slice<NWIN>(dst[1], k, b, lane);
         }
     }
 }
@@ -601,8 +617,7 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
     SBN0.zero();
     SBN2.zero();
 
-    get_slice<NWIN, OWN>(p, sl[0][0], jmin0, lane);
-    get_slice<NWIN, OWN>(p, sl[0][1], jmax0 - kChunk + 1, lane);
+    get_slices<NWIN, OWN>(p, sl[0], jmin0, jmax0 - kChunk + 1, lane);
     const CoefSrc cs = TAB ? coef_src(p.coef, l1, l2_0) : CoefSrc{};
     if constexpr (TAB) fetch_first(tb, *st, cs, lane);
     fetch_commit();
@@ -615,8 +630,7 @@ __device__ __forceinline__ bool chosen_xi(const CouplingParams& p, const int l1,
         else if (t0 > 0) place_next(tb, *st, lane);
         __syncwarp();
         if (t0 + kChunk < T) {  // the next chunk's slices land while this one computes
-            get_slice<NWIN, OWN>(p, sl[cur ^ 1][0], jmin0 + t0 + kChunk, lane);
-            get_slice<NWIN, OWN>(p, sl[cur ^ 1][1], jmax0 - t0 - 2 * kChunk + 1, lane);
+            get_slices<NWIN, OWN>(p, sl[cur ^ 1], jmin0 + t0 + kChunk, jmax0 - t0 - 2 * kChunk + 1, lane);
             if constexpr (TAB) fetch_next(*st, cs, t0 + kChunk, lane);
         }
         fetch_commit();

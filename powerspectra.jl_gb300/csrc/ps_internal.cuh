@@ -182,14 +182,14 @@ cudaError_t launch_coef(float4* t, int lmax, cudaStream_t s);
 bool reads_coef(const CouplingParams& p);
 bool has_coef(const CouplingParams& p);  // ... at any lmax
 // Smaller lmax in a batch: no table, each warp makes its few slices itself.  Then a table holds more slices than are
-// read (its launch on top: all spins, n x lmax, without and with, 2000 x 32 516 and 607 us, 300 x 100 612 and 629, 200 x 127 660
-// and 662, 100 x 250 1496 and 1420; the (0 0 0) family alone, with half the steps, 4 x 200 93 and 101, 100 x 250 777 and 779, 64 x 400
-// 1540 and 1519, 1 x 500 279 and 260).
+// read, and its kernel comes on top.  Without and with tables, n x lmax, all spins: 2000 x 32 516 and 607 us, 300 x 100 612
+// and 629, 200 x 127 660 and 662, 100 x 250 1496 and 1420.  The (0 0 0) family alone has half the steps: one window 4 x 200 93 and
+// 101, 100 x 250 777 and 779, 1 x 500 279 and 260; four windows 100 x 160 334 and 337, 4 x 200 100 and 92; eight 100 x 160 776 and 694.
 inline int slice_min_lmax(const CouplingParams& g)
 {
     for (int k = 0; k < g.nwin; ++k)
         if (g.win[k].product != PROD_00_00) return 128;
-    return 300;
+    return g.nwin > 4 ? 128 : (g.nwin > 2 ? 192 : 300);
 }
 // The slice tables of a batch's groups (NWIN = 4 or 8 as for launch_batch_chosen), each into its group's own p.slices
 // of batch_slice_bytes(lmax, nwin): block b makes kSliceBlock entries of group blocks[b].x, from entry blocks[b].y &

@@ -55,7 +55,8 @@ def test_long_queue(ctx, sizes, K, gs):
 def test_short_tasks_and_few_problems(ctx, gs):  # no ratios, slices for some
     _check(ctx, [1, 2, 30, 31, 33, 63, 64, 95, 127, 128, 129] * 9, MIX, 1, group_slots=gs)
     _check(ctx, [700, 127, 300], MIX[:3], 2, group_slots=gs)
-    _check(ctx, [299, 300], [0x1], 2, group_slots=gs)
+    for edge, K in ((300, 2), (192, 4), (128, 8)):  # slices of the (0 0 0) family alone
+        _check(ctx, [edge - 1, edge], [0x1], K, group_slots=gs)
 
 
 @pytest.mark.parametrize("sizes", [[40] * 3, list(range(60, 72)), [530, 90, 20]])  # without and with ratios
