@@ -1961,7 +1961,7 @@ static int window_run(ps_ctx* c, const double* const* dA, const double* const* d
         p.a[t] = (const double2*)dA[t];
         p.b[t] = (const double2*)dB[t];
     }
-    int st = ensure(c, &c->d_part, &c->part_cap, (size_t)nterms * p.nmchunks * ((size_t)lout + 1));
+    int st = ensure(c, &c->d_part, &c->part_cap, (size_t)nterms * ps::alm2cl_partials(mmax, lout));
     if (st) return st;
     p.partial = c->d_part;
     // the context's kernel time is the partial-sum kernel's (the reduction is small)

@@ -242,6 +242,7 @@ struct AlmParams {
     double* partial;  // nterms * nmchunks * (lout + 1)
 };
 int alm2cl_chunk(int mmax, int lout);  // m values per chunk
+size_t alm2cl_partials(int mmax, int lout);  // room for a term's partial sums
 // after_partial, when given, is recorded between the partial-sum kernel and the reduction.
 cudaError_t launch_alm2cl(const AlmParams& p, double scale, bool per_l, double* W, cudaStream_t s,
                           cudaEvent_t after_partial = nullptr);

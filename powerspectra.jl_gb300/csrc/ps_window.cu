@@ -128,6 +128,15 @@ int alm2cl_chunk(int mmax, int lout)
     return chunk;
 }
 
+// A bound that grows with mmax and lout, as the partial sums themselves do not (more chunks where there are few
+// blocks): a call then has room enough after any larger one, in a capture too.  With the chunk halved to c from
+// nb (mmax / 2c + 1) < 152 blocks, there are mmax / c + 1 <= 2 x 151 / nb chunks of lout + 1 <= nb kAlmThreads sums.
+size_t alm2cl_partials(int mmax, int lout)
+{
+    const size_t whole = (size_t)(mmax / kAlmChunk + 1) * ((size_t)lout + 1), fine = (size_t)302 * kAlmThreads;
+    return whole > fine ? whole : fine;
+}
+
 cudaError_t launch_alm2cl(const AlmParams& p, double scale, bool per_l, double* W, cudaStream_t s,
                           cudaEvent_t after_partial)
 {

@@ -101,3 +101,28 @@ def test_one_call_warms_up_the_grid(own, lmax, warm, then):
     c = Call(ref, then, lmax, "chosen", seed=5)
     assert bool((c.direct() == got).all())
     ref.close()
+
+
+@pytest.mark.parametrize("larger,lmax", [(1300, 1000), (2000, 1100), (300, 20)])
+def test_window_spectrum_after_a_larger_one(own, larger, lmax):
+    """The scratch of a larger call is enough for a smaller one, whose sums are cut finer."""
+    ctx, s = own
+
+    def call(lm, seed):
+        a = torch.tensor(np.random.default_rng(seed).normal(size=(lm + 1) * (lm + 2)), device="cuda")
+        out = torch.zeros(lm + 1, dtype=torch.float64, device="cuda")
+        return a, out, lambda: ctx.window_W_device([a.data_ptr()], [a.data_ptr()], lm, lm, lm, out.data_ptr())
+
+    *keep, big = call(larger, 1)
+    big()
+    a, out, run = call(lmax, 2)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        run()
+    g.replay()
+    torch.cuda.synchronize()
+    got = out.clone()
+    run()
+    torch.cuda.synchronize()
+    assert bool((got == out).all()) and bool((got > 0).all())
