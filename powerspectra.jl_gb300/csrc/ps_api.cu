@@ -860,14 +860,18 @@ struct HostOut {
     const double* src;
     int64_t lds;
 };
-static int copy_out(ps_ctx* c, const HostOut* out, int K, long long n)
+static int copy_only(ps_ctx* c, const HostOut* out, int K, long long n)
 {
-    for (int k = 0; k < K; ++k) back_pages(out[k].dst, out[k].ld, n);
     for (int k = 0; k < K; ++k)
         PS_CUDA(c, cudaMemcpy2DAsync(out[k].dst, (size_t)out[k].ld * sizeof(double), out[k].src,
                                      (size_t)out[k].lds * sizeof(double), (size_t)n * sizeof(double), (size_t)n,
                                      cudaMemcpyDeviceToHost, c->stream));
     return PS_OK;
+}
+static int copy_out(ps_ctx* c, const HostOut* out, int K, long long n)
+{
+    for (int k = 0; k < K; ++k) back_pages(out[k].dst, out[k].ld, n);
+    return copy_only(c, out, K, n);
 }
 
 static double* mapped_host(double* h)
@@ -982,24 +986,24 @@ int ps_mcm_blocks(ps_ctx* c, const double* W, int64_t nW, int lmin, int lmax, in
     spin_window(PS_SPIN_MM, &p.win[1].product, &p.win[1].parity);
     const double* both[2] = {W, W};
     if ((st = stage_windows(c, p, both, 2, nW, lmax, true, mode))) return st;
-    if ((st = ensure(c, &c->d_out, &c->out_cap, (size_t)(EB_BE ? 3 : 2) * n * n))) return st;
+    if ((st = ensure(c, &c->d_out, &c->out_cap, (size_t)2 * n * n))) return st;
     for (int k = 0; k < 2; ++k) p.out[k] = c->d_out + (size_t)k * n * n;
     p.ldo = n;
     if ((st = run_coupling(c, p, mode))) return st;
-    const double *pp = p.out[0], *mm = p.out[1];
-    HostOut out[8];
-    int K = 0;
-    auto put = [&](double* M, const double* off) {  // [pp off; off pp]
-        for (int b = 0; b < 4; ++b) out[K++] = {M + (b & 1) * n + (b >> 1) * n * ld, ld, b == 0 || b == 3 ? pp : off, n};
-    };
-    if (EE_BB) put(EE_BB, mm);
-    if (EB_BE) {
-        double* neg = c->d_out + (size_t)2 * n * n;
-        PS_CUDA(c, ps::launch_negate(mm, neg, n * n, c->stream));
-        c->launches++;
-        put(EB_BE, neg);
+    double *pp = p.out[0], *mm = p.out[1];
+    HostOut out[2][4];  // [pp mm; mm pp], of EE_BB and of EB_BE
+    for (int b = 0; b < 8; ++b) {
+        double* M = b < 4 ? EE_BB : EB_BE;
+        if (!M) continue;
+        out[b >> 2][b & 3] = {M + (b & 1) * n + (b >> 1 & 1) * n * ld, ld, (b & 3) == 0 || (b & 3) == 3 ? pp : mm, n};
+        back_pages(out[b >> 2][b & 3].dst, ld, n);
     }
-    if ((st = copy_out(c, out, K, n))) return st;
+    if (EE_BB && (st = copy_only(c, out[0], 4, n))) return st;
+    if (EB_BE) {  // -- turns into its negative where it is, behind its copies
+        PS_CUDA(c, ps::launch_negate(mm, n * n, c->stream));
+        c->launches++;
+        if ((st = copy_only(c, out[1], 4, n))) return st;
+    }
     PS_CUDA(c, cudaStreamSynchronize(c->stream));
     return PS_OK;
 }

@@ -220,7 +220,7 @@ struct LuWork {
 constexpr int kLuWaitLimit = 1 << 22;
 cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s);
 cudaError_t launch_transpose(double* dst, const double* src, int n, cudaStream_t s);
-cudaError_t launch_negate(const double* src, double* dst, long long count, cudaStream_t s);
+cudaError_t launch_negate(double* a, long long count, cudaStream_t s);
 // scratch: quickpol_scratch(lmax) doubles; half: for lmax
 size_t quickpol_scratch(int lmax);
 cudaError_t launch_quickpol(const double* W, long long nW, int lmax, int bl, int bu, int nu1, int nu2, int s1, int s2,

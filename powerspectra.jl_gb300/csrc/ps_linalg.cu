@@ -20,13 +20,14 @@
 
 namespace ps {
 
-// dst (n x n, ld n) = src^T (n x n, ld n), 32 x 32 tiles through shared memory
-__global__ void k_negate(const double* __restrict__ src, double* __restrict__ dst, long long count)
+// a = -a
+__global__ void k_negate(double* a, long long count)
 {
     const long long step = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) dst[i] = -src[i];
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) a[i] = -a[i];
 }
 
+// dst (n x n, ld n) = src^T (n x n, ld n), 32 x 32 tiles through shared memory
 __global__ void k_transpose(double* __restrict__ dst, const double* __restrict__ src, int n)
 {
     __shared__ double tile[32][33];
@@ -42,10 +43,10 @@ __global__ void k_transpose(double* __restrict__ dst, const double* __restrict__
     }
 }
 
-cudaError_t launch_negate(const double* src, double* dst, long long count, cudaStream_t s)
+cudaError_t launch_negate(double* a, long long count, cudaStream_t s)
 {
     const long long blocks = (count + 255) / 256;
-    k_negate<<<(unsigned)(blocks < 1216 ? blocks : 1216), 256, 0, s>>>(src, dst, count);
+    k_negate<<<(unsigned)(blocks < 1216 ? blocks : 1216), 256, 0, s>>>(a, count);
     return cudaGetLastError();
 }
 

@@ -167,3 +167,22 @@ def test_batch_tables_given_back(form, graph):
     torch.cuda.empty_cache()
     assert b.equal(want)
     ctx.close()
+
+
+def test_blocks_stage_two_matrices():
+    """[++ -(--); -(--) ++] needs no more on the device than ++ and --."""
+    import powerspectra_gpu as pg
+    lmax = 3599
+    n = lmax + 1
+    x = np.linspace(2.0, 1.0, n)
+    ctx = _context()
+    want = pg.mcm(("EE_BB", "EB_BE"), x, lmax=lmax, mode="chosen", ctx=ctx)
+    assert np.array_equal(want[0].parent[:n], np.hstack([want[1].parent[:n, :n], -want[1].parent[:n, n:]]))
+    ctx.close()
+    ctx = _context()
+    hold = _hold(280 << 20)  # two of 104 MB and the slices; three do not fit
+    got = pg.mcm("EB_BE", x, lmax=lmax, mode="chosen", ctx=ctx)
+    del hold
+    torch.cuda.empty_cache()
+    assert np.array_equal(got.parent, want[1].parent)
+    ctx.close()
