@@ -7,17 +7,16 @@
 namespace ps {
 
 // X[k] are the Xi of windows W1..Wk (already divided by 4pi), Sa, Sb, Ra, Rb the spectra and noise
-// ratios at l1 = a and l2 = b, g[i] = sqrt(Sa[i] Sb[i]) for the spectra that need it (cov_roots).  The
-// reference's sqrt of a product of two such pairs is the product of their roots here (equal to rounding;
-// a pair of unequal signs makes the element NaN either way, through the terms with its own root).
+// ratios at l1 = a and l2 = b, g[i] = sqrt(Sa[i] Sb[i]) for the spectra that need it (cov_roots), and gg[i] = sqrt of
+// the product of the pairs 2 i and 2 i + 1 (kinds with two such pairs).
 __device__ __forceinline__ double cov_form(int kind, const double* Sa, const double* Sb, const double* g,
-                                           const double* Ra, const double* Rb, const double* X)
+                                           const double* gg, const double* Ra, const double* Rb, const double* X)
 {
     switch (kind) {
     case PS_COV_TTTT:
     case PS_COV_EEEE: {  // src/covariance.jl:110-118 (TTTT), :171-179 (EEEE); ip, jq, iq, jp
         const double ip = Ra[0] * Rb[0], jq = Ra[1] * Rb[1], iq = Ra[2] * Rb[2], jp = Ra[3] * Rb[3];
-        return g[0] * g[1] * X[0] + g[2] * g[3] * X[1] + g[0] * X[2] * jq + g[1] * X[3] * ip + g[2] * X[4] * jp +
+        return gg[0] * X[0] + gg[1] * X[1] + g[0] * X[2] * jq + g[1] * X[3] * ip + g[2] * X[4] * jp +
                g[3] * X[5] * iq + X[6] * (ip * jq) + X[7] * (iq * jp);
     }
     case PS_COV_TTTE:  // src/covariance.jl:225-230; TTip, TTjp, TEiq, TEjq; r_ip, r_jp
@@ -25,7 +24,7 @@ __device__ __forceinline__ double cov_form(int kind, const double* Sa, const dou
                 (Sa[2] + Sb[2]) * X[3] * Ra[1] * Rb[1]) / 2;
     case PS_COV_TETE: {  // src/covariance.jl:292-297; TTip, EEjq, TEiq, TEjp; r_TT, r_PP
         const double rT = Ra[0] * Rb[0], rP = Ra[1] * Rb[1];
-        return g[0] * g[1] * X[0] + 0.5 * (Sa[2] * Sb[3] + Sa[3] * Sb[2]) * X[1] + g[0] * X[2] * rP + g[1] * X[3] * rT +
+        return gg[0] * X[0] + 0.5 * (Sa[2] * Sb[3] + Sa[3] * Sb[2]) * X[1] + g[0] * X[2] * rP + g[1] * X[3] * rT +
                X[4] * (rT * rP);
     }
     case PS_COV_TEEE:
@@ -42,6 +41,11 @@ __host__ __device__ constexpr int cov_roots(int kind)
 {
     return kind == PS_COV_TTTT || kind == PS_COV_EEEE ? 4 : (kind == PS_COV_TTEE ? 0 : 2);
 }
+// ... how many products of two of them it takes the root of: 0 and 1, 2 and 3 ...
+__host__ __device__ constexpr int cov_products(int kind)
+{
+    return kind == PS_COV_TTTT || kind == PS_COV_EEEE ? 2 : (kind == PS_COV_TETE ? 1 : 0);
+}
 // ... and how many noise ratios it has.
 __host__ __device__ constexpr int cov_ratios(int kind)
 {
@@ -52,7 +56,7 @@ __host__ __device__ constexpr int cov_ratios(int kind)
 __device__ __forceinline__ double cov_combine(int kind, const double* const* S, const double* const* R,
                                               const double* X, int a, int b)
 {
-    double Sa[4], Sb[4], g[4], Ra[4], Rb[4];
+    double Sa[4], Sb[4], g[4], gg[2], Ra[4], Rb[4];
     const int ng = cov_roots(kind), nr = cov_ratios(kind);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -62,7 +66,11 @@ __device__ __forceinline__ double cov_combine(int kind, const double* const* S, 
         Ra[i] = i < nr ? R[i][a] : 0.0;
         Rb[i] = i < nr ? R[i][b] : 0.0;
     }
-    return cov_form(kind, Sa, Sb, g, Ra, Rb, X);
+    // one root of the whole product, as the reference takes it: the product of two roots has two roundings more
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        gg[i] = i < cov_products(kind) ? sqrt(Sa[2 * i] * Sb[2 * i] * Sa[2 * i + 1] * Sb[2 * i + 1]) : 0.0;
+    return cov_form(kind, Sa, Sb, g, gg, Ra, Rb, X);
 }
 
 }  // namespace ps
