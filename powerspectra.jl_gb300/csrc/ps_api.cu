@@ -25,7 +25,7 @@ void ps_linalg_free(ps_linalg* L);
 int ps_linalg_decouple(ps_linalg* L, const double* Y, const double* B1, const double* B2, int n, int64_t ldin,
                        double* out, int64_t ldout, cudaStream_t s, char* err, size_t errn, bool on_device);
 int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const double* b, int nrhs, int64_t ldb,
-                    double* x, int64_t ldx, cudaStream_t s, char* err, size_t errn);
+                    double* x, int64_t ldx, cudaStream_t s, char* err, size_t errn, int* launches);
 void ps_linalg_wait_limit(ps_linalg* L, int limit);
 
 // Largest lmax the kernels accept: the integer products in P(j) stay below 2^63
@@ -1882,10 +1882,11 @@ int ps_solve(ps_ctx* c, const double* M, int64_t n, int64_t ldm, const double* b
         return set_err(c, PS_ERR_ARG, "need 1 <= n <= 65535, nrhs >= 1, leading dimensions >= n");
     PS_CUDA(c, cudaSetDevice(c->device));
     if (!c->la) c->la = ps_linalg_new();
+    int launches = 0;
     int st = with_room(c, [&] {
-        return ps_linalg_solve(c->la, M, (int)n, ldm, b, nrhs, ldb, x, ldx, c->stream, c->err, sizeof(c->err));
+        return ps_linalg_solve(c->la, M, (int)n, ldm, b, nrhs, ldb, x, ldx, c->stream, c->err, sizeof(c->err), &launches);
     });
-    if (!st) c->launches += 2;
+    c->launches += (unsigned)launches;
     return st;
 }
 

@@ -218,7 +218,8 @@ struct LuWork {
     int wait_limit;            // polls of a panel's waits
 };
 constexpr int kLuWaitLimit = 1 << 22;
-cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s);
+cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s,
+                            int* launches);
 cudaError_t launch_transpose(double* dst, const double* src, int n, cudaStream_t s);
 cudaError_t launch_negate(double* a, long long count, cudaStream_t s);
 // scratch: quickpol_scratch(lmax) doubles; half: for lmax

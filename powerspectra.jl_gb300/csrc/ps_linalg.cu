@@ -213,7 +213,7 @@ int ps_linalg_decouple(ps_linalg* L, const double* Y, const double* B1, const do
 }
 
 int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const double* b, int nrhs, int64_t ldb,
-                    double* x, int64_t ldx, cudaStream_t s, char* err, size_t errn)
+                    double* x, int64_t ldx, cudaStream_t s, char* err, size_t errn, int* launches)
 {
     size_t need = (size_t)n * (size_t)(n > nrhs ? n : nrhs);
     const bool own = ps::lu_fits(n, nrhs);
@@ -224,7 +224,7 @@ int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const dou
     const double* res = L->x;
     if (own) {
         const ps::LuWork wk = {L->side, L->ev_panel, L->ev_rest, L->ipiv, L->info, L->wait_limit};
-        LA_CUDA(ps::launch_lu_solve(L->a, n, L->x, nrhs, L->t, wk, s));
+        LA_CUDA(ps::launch_lu_solve(L->a, n, L->x, nrhs, L->t, wk, s, launches));
         int info = 0;
         LA_CUDA(cudaMemcpyAsync(&info, L->info, sizeof(int), cudaMemcpyDeviceToHost, s));
         LA_CUDA(cudaStreamSynchronize(s));
@@ -233,6 +233,8 @@ int ps_linalg_solve(ps_linalg* L, const double* M, int n, int64_t ldm, const dou
         res = L->t;
     } else if ((st = la_lu_solve(L, n, nrhs, L->x, s, "M", err, errn))) {
         return st;
+    } else {
+        *launches += 2;  // getrf and getrs
     }
     LA_CUDA(cudaMemcpy2DAsync(x, (size_t)ldx * sizeof(double), res, (size_t)n * sizeof(double),
                               (size_t)n * sizeof(double), (size_t)nrhs, cudaMemcpyDeviceToHost, s));

@@ -438,8 +438,8 @@ bool lu_fits(int n, int nrhs) { return nrhs <= 32 && n <= cluster_blocks() * kMa
 
 // x = a^-1 b for the n x n device matrix a and nrhs columns b (leading dimensions n), on stream s with the
 // panels on w.side; a and b are overwritten.  *w.info becomes the first zero pivot's index from 1, -1 when a
-// wait gave up (x then holds nothing of use), or stays INT_MAX.
-cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s)
+// wait gave up (x then holds nothing of use), or stays INT_MAX.  *launches grows by the kernels launched.
+cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, const LuWork& wk, cudaStream_t s, int* launches)
 {
     static const int kNone = INT_MAX;
 #define LU_TRY(call) \
@@ -450,9 +450,11 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
     const int nb = cluster_blocks(), ncol = n + nrhs;
     auto beyond = [&](int cb, int ce, int j0, int w, const int* perm, cudaStream_t st) -> cudaError_t {
         if (cb >= ce) return cudaSuccess;
+        ++*launches;
         k_lu_rows<<<(unsigned)((ce - cb + 7) / 8), 256, 0, st>>>(a, b, n, cb, ce, j0, w, perm);
         const int below = n - j0 - kPan;
         if (below > 0) {
+            ++*launches;
             const dim3 grid((unsigned)((below + 31) / 32), (unsigned)((ce - cb + 31) / 32));
             // the next panel's columns are waited for; the rest has time, and its blocks would take their places
             if (st == wk.side) return launch_after(k_lu_update, grid, dim3(128), 0, st, a, b, n, cb, ce, j0);
@@ -470,6 +472,7 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
         cfg.stream = wk.side;
         if (j0 == 0) cfg.numAttrs = 1;  // the first one has no update before it
         const auto kernel = wk.wait_limit == kLuWaitLimit ? k_lu_panel<false> : k_lu_panel<true>;
+        ++*launches;
         LU_TRY(cudaLaunchKernelEx(&cfg, kernel, a, n, j0, w, rows, perm, wk.info, wk.wait_limit));
         LU_TRY(cudaEventRecord(wk.panel, wk.side));
         LU_TRY(cudaStreamWaitEvent(s, wk.panel, 0));
@@ -482,6 +485,7 @@ cudaError_t launch_lu_solve(double* a, int n, double* b, int nrhs, double* x, co
     for (int j0 = (n - 1) / kPan * kPan; j0 >= 0; j0 -= kPan) {
         const int w = n - j0 < kPan ? n - j0 : kPan;
         const dim3 grid((unsigned)(j0 > 0 ? (j0 + 255) / 256 : 1), (unsigned)nrhs);
+        ++*launches;
         if (j0 + kPan >= n) {  // the first one starts when the matrix is done
             k_lu_back<<<grid, 256, 0, s>>>(a, b, x, n, j0, w);
             LU_TRY(cudaGetLastError());
