@@ -66,9 +66,7 @@ __global__ void __launch_bounds__(kTile * kRows) k_cov_combine(const CovCombineP
                 Ra[k] = sR[0][k][tx];
                 Rb[k] = sR[1][k][c];
             }
-            // products of roots: their two roundings of 1e-16 are nothing beside the Xi's 1e-7 of the fast arithmetic
-            const double gg[2] = {g[0] * g[1], g[2] * g[3]};
-            e = cov_form(KIND, Sa, Sb, g, gg, Ra, Rb, x);
+            e = cov_form<false>(KIND, Sa, Sb, g, Ra, Rb, x);
             p.C[i + (long long)j * p.ldc] = e;
         }
         sC[c][tx] = e;

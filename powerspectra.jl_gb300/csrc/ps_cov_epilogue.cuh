@@ -7,16 +7,23 @@
 namespace ps {
 
 // X[k] are the Xi of windows W1..Wk (already divided by 4pi), Sa, Sb, Ra, Rb the spectra and noise
-// ratios at l1 = a and l2 = b, g[i] = sqrt(Sa[i] Sb[i]) for the spectra that need it (cov_roots), and gg[i] = sqrt of
-// the product of the pairs 2 i and 2 i + 1 (kinds with two such pairs).
+// ratios at l1 = a and l2 = b, g[i] = sqrt(Sa[i] Sb[i]) for the spectra that need it (cov_roots).
+// ONE_ROOT: the root of a product of two such pairs as one root, as the reference takes it, for the FP64 kernels; the
+// product of the two roots has two roundings of 1e-16 more, which Xi with the fast arithmetic's 1e-7 do not show (the
+// further roots would cost TTTT and EEEE at lmax 700 3 %).  The roots are taken inside their case: ahead of the
+// switch, as predicated instructions or a loop, they cost every kind (TTEE at lmax 700 in FP64 364 -> 377 us).
+template <bool ONE_ROOT>
 __device__ __forceinline__ double cov_form(int kind, const double* Sa, const double* Sb, const double* g,
-                                           const double* gg, const double* Ra, const double* Rb, const double* X)
+                                           const double* Ra, const double* Rb, const double* X)
 {
+    auto product = [&](int i) {  // of the pairs i and i + 1
+        return ONE_ROOT ? sqrt(Sa[i] * Sb[i] * Sa[i + 1] * Sb[i + 1]) : g[i] * g[i + 1];
+    };
     switch (kind) {
     case PS_COV_TTTT:
     case PS_COV_EEEE: {  // src/covariance.jl:110-118 (TTTT), :171-179 (EEEE); ip, jq, iq, jp
         const double ip = Ra[0] * Rb[0], jq = Ra[1] * Rb[1], iq = Ra[2] * Rb[2], jp = Ra[3] * Rb[3];
-        return gg[0] * X[0] + gg[1] * X[1] + g[0] * X[2] * jq + g[1] * X[3] * ip + g[2] * X[4] * jp +
+        return product(0) * X[0] + product(2) * X[1] + g[0] * X[2] * jq + g[1] * X[3] * ip + g[2] * X[4] * jp +
                g[3] * X[5] * iq + X[6] * (ip * jq) + X[7] * (iq * jp);
     }
     case PS_COV_TTTE:  // src/covariance.jl:225-230; TTip, TTjp, TEiq, TEjq; r_ip, r_jp
@@ -24,7 +31,7 @@ __device__ __forceinline__ double cov_form(int kind, const double* Sa, const dou
                 (Sa[2] + Sb[2]) * X[3] * Ra[1] * Rb[1]) / 2;
     case PS_COV_TETE: {  // src/covariance.jl:292-297; TTip, EEjq, TEiq, TEjp; r_TT, r_PP
         const double rT = Ra[0] * Rb[0], rP = Ra[1] * Rb[1];
-        return gg[0] * X[0] + 0.5 * (Sa[2] * Sb[3] + Sa[3] * Sb[2]) * X[1] + g[0] * X[2] * rP + g[1] * X[3] * rT +
+        return product(0) * X[0] + 0.5 * (Sa[2] * Sb[3] + Sa[3] * Sb[2]) * X[1] + g[0] * X[2] * rP + g[1] * X[3] * rT +
                X[4] * (rT * rP);
     }
     case PS_COV_TEEE:
@@ -41,11 +48,6 @@ __host__ __device__ constexpr int cov_roots(int kind)
 {
     return kind == PS_COV_TTTT || kind == PS_COV_EEEE ? 4 : (kind == PS_COV_TTEE ? 0 : 2);
 }
-// ... how many products of two of them it takes the root of: 0 and 1, 2 and 3 ...
-__host__ __device__ constexpr int cov_products(int kind)
-{
-    return kind == PS_COV_TTTT || kind == PS_COV_EEEE ? 2 : (kind == PS_COV_TETE ? 1 : 0);
-}
 // ... and how many noise ratios it has.
 __host__ __device__ constexpr int cov_ratios(int kind)
 {
@@ -53,10 +55,11 @@ __host__ __device__ constexpr int cov_ratios(int kind)
 }
 
 // The element of one pair (l1 = a, l2 = b), a <= b.
+template <bool ONE_ROOT>
 __device__ __forceinline__ double cov_combine(int kind, const double* const* S, const double* const* R,
                                               const double* X, int a, int b)
 {
-    double Sa[4], Sb[4], g[4], gg[2], Ra[4], Rb[4];
+    double Sa[4], Sb[4], g[4], Ra[4], Rb[4];
     const int ng = cov_roots(kind), nr = cov_ratios(kind);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -66,11 +69,7 @@ __device__ __forceinline__ double cov_combine(int kind, const double* const* S, 
         Ra[i] = i < nr ? R[i][a] : 0.0;
         Rb[i] = i < nr ? R[i][b] : 0.0;
     }
-    // one root of the whole product, as the reference takes it: the product of two roots has two roundings more
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-        gg[i] = i < cov_products(kind) ? sqrt(Sa[2 * i] * Sb[2 * i] * Sa[2 * i + 1] * Sb[2 * i + 1]) : 0.0;
-    return cov_form(kind, Sa, Sb, g, gg, Ra, Rb, X);
+    return cov_form<ONE_ROOT>(kind, Sa, Sb, g, Ra, Rb, X);
 }
 
 }  // namespace ps

@@ -28,7 +28,7 @@ __device__ __forceinline__ void write_pair(const CouplingParams& p, int l1, int 
             }
         }
     } else {
-        double c = cov_combine(p.cov_kind, p.S, p.R, Xi, l1, l2);
+        double c = cov_combine<false>(p.cov_kind, p.S, p.R, Xi, l1, l2);
         p.out[0][r1 + r2 * p.ldo] = c;
         p.out[0][r2 + r1 * p.ldo] = c;
     }
@@ -51,7 +51,7 @@ static_assert(kTileRows == kWarpsPerBlock, "one tile row per warp");
 // `stage` holds each warp's row-half values: warp w's at stage + w * stride,
 // [NOUT][32] doubles, in shared memory that warp w no longer uses.  All threads
 // of the block call this once.
-template <int NOUT>
+template <int NOUT, bool ONE_ROOT = false>
 __device__ __forceinline__ void write_tile(const CouplingParams& p, int l1, int l2_0, bool active, const double* Xi,
                                            double* stage, int stride, TileRows& rows, int warp, int lane)
 {
@@ -61,7 +61,7 @@ __device__ __forceinline__ void write_tile(const CouplingParams& p, int l1, int 
         const long long r1 = l1 - p.lmin, r2 = l2 - p.lmin;
         double* st = stage + warp * stride;
         if (p.epilogue == EPI_COV) {
-            const double c = active ? cov_combine(p.cov_kind, p.S, p.R, Xi, l1, l2) : 0.0;
+            const double c = active ? cov_combine<ONE_ROOT>(p.cov_kind, p.S, p.R, Xi, l1, l2) : 0.0;
             if (active) p.out[0][r2 + r1 * p.ldo] = c;
             st[lane] = c;
         } else {

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_coupling_fp64(const Pla
         else points00(P, sm.f[warp], l1, task.y, l2, n, lane, a, b);
         a.give(P, b, l1, Xi);
     }
-    write_tile<kMaxWin>(p, l1, task.y, active, Xi, &sm.stage[0][0], kMaxWin * 32, sm.rows, warp, lane);
+    write_tile<kMaxWin, true>(p, l1, task.y, active, Xi, &sm.stage[0][0], kMaxWin * 32, sm.rows, warp, lane);
 }
 
 struct Form {

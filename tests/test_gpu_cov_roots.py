@@ -1,6 +1,6 @@
 """The roots in the covariance formulas.
 
-One root per product: spectra of 1 and 2 only, so that S1(a) S1(b) S2(a) S2(b) is 1, 4 or 16 and its root exact where
+One root per product in FP64: spectra of 1 and 2 only, so that S1(a) S1(b) S2(a) S2(b) is 1, 4 or 16 and its root exact where
 the roots of the two pairs are not, and windows of zeros but for one.  An element is then that window's Xi times 1, 2
 or 4, to the last bit.
 
@@ -20,8 +20,7 @@ ROOTS = {"TTTT": ((0, 0), ((0, 0, 1), (1, 2, 3))), "EEEE": ((1, 1), ((0, 0, 1), 
 
 
 @pytest.mark.parametrize("kind", list(ROOTS))
-@pytest.mark.parametrize("mode", ["plain", "chosen"])
-def test_one_root_of_a_product(ctx, kind, mode):
+def test_one_root_of_a_product(ctx, kind):
     from powerspectra_gpu import synthetic as syn
     L = 70
     (product, parity), pairs = ROOTS[kind]
@@ -33,10 +32,10 @@ def test_one_root_of_a_product(ctx, kind, mode):
     for k, i, j in pairs:
         Ws = [W if q == k else zero for q in range(nw)]
         S = [s if q in (i, j) else np.zeros(L + 1) for q in range(4)]
-        C = ctx.coupledcov(kind, S, R, Ws, 0, L, mode=mode)
-        X = ctx.xi(product, parity, Ws[k:] + Ws[:k], 0, L, mode=mode)[0] if kind != "TETE" else None
+        C = ctx.coupledcov(kind, S, R, Ws, 0, L)
+        X = ctx.xi(product, parity, Ws[k:] + Ws[:k], 0, L)[0] if kind != "TETE" else None
         if X is None:  # TETE mixes families: its own element for spectra of ones
-            X = ctx.coupledcov(kind, [np.ones(L + 1) if q in (i, j) else S[q] for q in range(4)], R, Ws, 0, L, mode=mode)
+            X = ctx.coupledcov(kind, [np.ones(L + 1) if q in (i, j) else S[q] for q in range(4)], R, Ws, 0, L)
         assert np.array_equal(C, np.outer(s, s) * X)
 
 
