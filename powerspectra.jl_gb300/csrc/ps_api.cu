@@ -493,8 +493,13 @@ static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first =
     p.tasks = tiles.d;
     p.ntasks = tiles.n;
     if (mode == PS_MODE_CHOSEN) {
-        // room for any list of slots on this grid, so that one call of a grid is enough before a capture
-        if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, ps::slice_table_most(p.lmax)))) return st;
+        // room for any list of slots on this grid, so that one call of a grid is enough before a capture; doubled as
+        // it grows, since an allocation takes some 100 us (21 sizes from lmax 600 to 700: 8.2 ms without)
+        const size_t most = ps::slice_table_most(p.lmax);
+        if (most > c->slices_cap) {
+            const size_t twice = std::min(2 * c->slices_cap, ps::slice_table_most(PS_MAX_LMAX));
+            if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, std::max(most, twice)))) return st;
+        }
         p.slices = c->d_slices;
         if (ps::reads_coef(p) && (st = ensure_coef(c, p.lmax, &p.coef))) return st;
     } else if ((st = ensure_half(c, p.lmax, &p.half))) {
