@@ -1431,6 +1431,7 @@ static const size_t kBatchSliceBytes = (size_t)2 << 30, kNone = ~(size_t)0;
 static bool launches_read_coef(const std::vector<ps::CouplingParams>& groups, int* lmax)
 {
     double us = 0.0;
+    *lmax = 0;
     for (const auto& g : groups)
         if (ps::has_coef(g)) {
             us += 1.0 + 2.2e-8 * g.lmax * g.lmax * g.lmax;
@@ -1438,26 +1439,29 @@ static bool launches_read_coef(const std::vector<ps::CouplingParams>& groups, in
         }
     return us >= 10.0;
 }
+// A queue's items with a (2 -2 0) family, in steps of the recurrence.
+struct QueueWork {
+    double work = 0.0, tasks = 0.0, longest = 0.0;
+    int lmax = 0;
+    void add(int ntask, int l1)
+    {
+        const double w = ntask * (2.0 * l1 + 1.0);
+        work += w;
+        tasks += ntask;
+        longest = std::max(longest, w);
+    }
+};
 // Whether the persistent kernel's groups with a (2 -2 0) family read one.  The table saves instructions and costs a
 // task's first chunk a wait for its copies.  So it is for queues that keep the warps busy while the longest item
 // runs (n x lmax, ++/-- without and with: 1 x 1000 1.54 and 1.64 ms, 2 x 1000 1.74 and 1.84, 4 x 1000 2.38 and 2.33, 8 x 1000
 // 4.40 and 4.20; 4 x 500 656 and 688 us, 8 x 500 747 and 712) and whose tasks are some 70 steps long on average (2000 x 32
 // 330 and 458 us, 800 x 64 443 and 457, 300 x 100 423 and 410, 64 x 400 2.62 and 2.49 ms).  One problem beyond
 // kCoefMaxLmax leaves the others without: the kernel reads it for all or none.
-static bool queue_reads_coef(const std::vector<ps::CouplingParams>& groups, const std::vector<int4>& items, int gs,
-                             int nsm, int* lmax)
+static bool queue_reads_coef(const QueueWork& q, int gs, int nsm)
 {
-    double work = 0.0, tasks = 0.0, longest = 0.0;
-    for (const int4& it : items) {
-        if (!(it.w >> 8 & 2)) continue;  // the (0 0 0) family alone
-        const double n = it.w & 0xff, w = n * (2.0 * it.y + 1.0);
-        work += w;
-        tasks += n;
-        longest = std::max(longest, w);
-        *lmax = std::max(*lmax, groups[it.x].lmax);
-    }
+    if (gs > 4 || q.tasks == 0.0) return false;
     const double warps = (double)nsm * ps::batch_blocks_per_sm(gs, true) * ps::kWarpsPerBlock;
-    return gs <= 4 && tasks > 0.0 && work >= 0.7 * warps * longest && work >= 70.0 * tasks;
+    return q.work >= 0.7 * warps * q.longest && q.work >= 70.0 * q.tasks;
 }
 
 int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int bps)
@@ -1497,6 +1501,7 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
     std::vector<ps::CouplingParams> groups;
     std::vector<int4> items;
     std::vector<float> cost;
+    QueueWork queue;
     std::vector<int2> mtiles, one_mt;
     std::vector<std::pair<long long, int2>> mtile_of;  // (lmin, lmax) key -> (offset in mtiles, count)
     std::vector<size_t> mma_tile_off;                   // per tensor-core launch
@@ -1592,12 +1597,14 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
             }
             const int gid = (int)groups.size();
             groups.push_back(g);
+            if (f22) queue.lmax = std::max(queue.lmax, g.lmax);
             // items: up to 8 warp tasks (256 consecutive l2) of one row
             for (int l1 = P.lmin; l1 <= P.lmax; ++l1) {
                 for (int l2 = l1; l2 <= P.lmax; l2 += 256) {
                     int ntask = std::min(8, (P.lmax - l2) / 32 + 1);
                     items.push_back(make_int4(gid, l1, l2, ntask | (fam << 8) | (tmpl << 12)));
                     cost.push_back((float)ntask * (2.0f * l1 + 1.0f) * (f22 ? 1.0f : 0.5f));
+                    if (f22) queue.add(ntask, l1);
                 }
             }
         }
@@ -1669,9 +1676,8 @@ int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int 
     }
     // and one table of the square-root ratios (the batch's own: a context's may be replaced by a larger one), as
     // long as the groups that read it need.  One allocation for both (some 100 us); without room for both, slices alone
-    int coef_lmax = 0;
-    const bool use_coef = bps < 0 ? launches_read_coef(groups, &coef_lmax)
-                                  : queue_reads_coef(groups, items, gs, nsm, &coef_lmax);
+    int coef_lmax = queue.lmax;
+    const bool use_coef = bps < 0 ? launches_read_coef(groups, &coef_lmax) : queue_reads_coef(queue, gs, nsm);
     const size_t coef_bytes = use_coef && coef_lmax <= kCoefMaxLmax ? ps::coef_bytes(coef_lmax) : 0;
     auto optional = [&](size_t bytes) {
         if (!bytes) return false;
