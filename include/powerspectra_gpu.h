@@ -81,7 +81,16 @@ int ps_create(int device, ps_ctx **out);
 void ps_destroy(ps_ctx *ctx);
 const char *ps_last_error(const ps_ctx *ctx);
 /* Use an external cudaStream_t (passed as void*) for all later work; NULL
- * restores the context's own stream. */
+ * restores the context's own stream.
+ *
+ * The _device calls can be recorded into a CUDA graph on that stream.  A call
+ * of the same arithmetic, (lmin, lmax) and at least as many windows must have
+ * run on the context before, outside the capture, and directly before among
+ * the calls of that arithmetic: lists and buffers of a grid are made then, and
+ * a capture cannot allocate.  The graph keeps the addresses of that scratch, so its replays
+ * are valid until a call of the same arithmetic on another grid, or any call
+ * that needs more of the scratch, runs on the context: keep a context per
+ * recorded grid. */
 int ps_set_stream(ps_ctx *ctx, void *cuda_stream);
 int ps_synchronize(ps_ctx *ctx);
 
@@ -295,8 +304,11 @@ int ps_set_tensor_cores(ps_ctx *ctx, int enable);
 
 /* Instrumentation: device time of the coupling kernels of the last call (CUDA
  * events on the launching stream, from the first coupling launch of the call
- * to the end of its last), number of kernels this context has launched, and a
- * measured FMA-pipe peak (flop/s, FMA = 2 flops) of this GPU in FP64 (fp64=1)
+ * to the end of its last; the window preparation of a call with one coupling
+ * launch, which the launch overlaps, is inside, that of ps_mcm_set and of a
+ * batch is not, and a covariance set is timed whole), number of kernels this
+ * context has launched, and a measured FMA-pipe peak (flop/s, FMA = 2 flops)
+ * of this GPU in FP64 (fp64=1)
  * or FP32 (fp64=0). */
 double ps_last_kernel_ms(const ps_ctx *ctx);
 uint64_t ps_launch_count(const ps_ctx *ctx);

@@ -824,9 +824,6 @@ double ps_last_kernel_ms(const ps_ctx* c)
 
 uint64_t ps_launch_count(const ps_ctx* c) { return c ? (uint64_t)c->launches : 0; }
 
-// The device address of a page-locked host buffer that is mapped into the
-// device's address space (cudaHostAlloc / cudaHostRegister memory under unified
-// addressing), or nullptr for ordinary pageable memory.
 // Whether p (a host or device address) lies in host memory.
 static bool host_resident(const void* p)
 {
@@ -879,6 +876,9 @@ static int copy_out(ps_ctx* c, const HostOut* out, int K, long long n)
     return copy_only(c, out, K, n);
 }
 
+// The device address of a page-locked host buffer that is mapped into the
+// device's address space (cudaHostAlloc / cudaHostRegister memory under unified
+// addressing), or nullptr for ordinary pageable memory.
 static double* mapped_host(double* h)
 {
     cudaPointerAttributes a;

@@ -5,8 +5,11 @@
 //
 // Same work and mapping as the plain kernel (one warp = 32 consecutive l2 of one
 // l1 row; families (l1 l2 l3; 0 0 0) and (l1 l2 l3; -2 2 0) in registers,
-// contracted on the fly; see ps_plain_fp64.cu for the recurrence), with the
-// arithmetic moved off the FP64 pipe:
+// contracted on the fly), off the FP64 pipe and by another route to the families: the
+// Schulten-Gordon relation a(j+1) f(j+1) + c (2j+1) f(j) + a(j) f(j-1) = 0 itself, with
+// a(j)^2 = (j^2 - (l1 - l2)^2) ((l1 + l2 + 1)^2 - j^2) and c = 4 for (2 -2 0), 0 for (0 0 0),
+// forward from the smallest and backward from the largest j, matched in the middle and
+// normalised by the sum of (2j+1) f^2 (ps_plain_fp64.cu needs none of that):
 //
 //  * recurrence state and coefficients are float-float values (ps_ff.cuh), so
 //    each step carries ~2^-46 relative error instead of FP32's 2^-24.  The

@@ -353,7 +353,6 @@ __device__ __forceinline__ RingIdx ring_idx(int tf_even, int tb_even, int l2)
     return RingIdx{ring_slot(tf_even), ring_slot(2 * l2 + tf_even), ring_slot(tb_even), kGuard + ring_slot(u0),
                    kGuard + ring_slot(u0 - 1)};
 }
-// forward step of parity p in pair k: g[t] and f[2 l2 + t]
 // The same entries as addresses, for the loop of a steady block: they move with the steps, which spares
 // it the index arithmetic (with moving indices in the (0 0 0) loop, the 20 matrices at lmax 8191: 440.5 ->
 // 426.1 ms; in the checked loop the addresses cost registers that the 16-column kernel does not have).
@@ -373,23 +372,24 @@ __device__ __forceinline__ RingPtr ring_ptr(const CoefRing& R, const RingIdx& q)
     return RingPtr{R.g[0] + q.g, R.f[0] + q.f, R.g[0] + q.gb, R.fb[0] + q.fb0, R.fb[1] + q.fb1};
 }
 constexpr int kRow = kRing + kGuard;  // entries from the table of the even values to that of the odd ones
+// forward step of parity p in pair k: g[t] and f[2 l2 + t]
 __device__ __forceinline__ void fwd_step(Sweep22& S, const RingPtr& r, int p, int k)
 {
     const ffpair g = r.g[p * kRow + k], f = r.f[p * kRow + k];
     step22(S, ff_mul_raw(g.rho, f.rho), ff_mul_raw(g.r, f.r), 8.0f);
 }
+// backward step of parity p in pair k: g[t] and fb[2 l2 - t]
 __device__ __forceinline__ void bwd_step(Sweep22& S, const RingPtr& r, int p, int k)
 {
     const ffpair g = r.gb[p * kRow + k], f = (p ? r.fb1 : r.fb0)[-k];
     step22(S, ff_mul_raw(g.rho, f.rho), ff_mul_raw(g.r, f.r), -8.0f);
 }
-// forward step of parity p in pair k: g[t] and f[2 l2 + t]
+// The same two steps with indices.
 __device__ __forceinline__ void fwd_step(Sweep22& S, const CoefRing& R, int p, const RingIdx& q, int k)
 {
     const ffpair g = R.g[p][q.g + k], f = R.f[p][q.f + k];
     step22(S, ff_mul_raw(g.rho, f.rho), ff_mul_raw(g.r, f.r), 8.0f);
 }
-// backward step of parity p in pair k: g[t] and fb[2 l2 - t]
 __device__ __forceinline__ void bwd_step(Sweep22& S, const CoefRing& R, int p, const RingIdx& q, int k)
 {
     const ffpair g = R.g[p][q.gb + k], f = R.fb[p][(p ? q.fb1 : q.fb0) - k];

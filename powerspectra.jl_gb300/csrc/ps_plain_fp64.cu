@@ -309,7 +309,9 @@ cudaError_t launch_plain_fp64(const CouplingParams& p, cudaStream_t s)
         // (64 cycles an instruction), and the fewer share it, the sooner the longest rows, which come first,
         // are done and the better the rest spread over the SMs.  ++/-- at nW = lmax + 1, with as many as fit (8), 1, 2
         // and 3: lmax 255 (288 blocks) 109, 94, 110, 110 us; 383 (624) 271, 231, 206, 225; 511 (1088) 534, 483, 429,
-        // 426; 767 (2400) 1366, 1481, 1301, 1302; 1001 (4224) 2797, 3166, 2772, 2777.
+        // 426; 767 (2400) 1366, 1481, 1301, 1302; 1001 (4224) 2797, 3166, 2772, 2777.  The other forms agree: with TT, 8 TT, TE,
+        // 8 TE, all spins of one and two windows and TT and TE of four, at lmax 255 to 1400, the rule is within 3 % of the best
+        // of 1, 2, 3, 4 and as many as fit (TT at 383 41.6 us, 51.9 with as many as fit; all spins 220 and 296).
         const int share = blocks <= 2 * kSMs ? 1 : (blocks <= 8 * kSMs ? 2 : 3);
         const size_t pad = blocks > kSMs ? pad_smem(share, sizeof(PlainSmem)) : 0;
         return launch_after(f.kernel, dim3(blocks), dim3(threads), pad, s, P);

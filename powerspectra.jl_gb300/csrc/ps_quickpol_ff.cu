@@ -3,10 +3,11 @@
 // float-float, FP64 only where the FP64 kernel (ps_quickpol.cu) needs range or
 // one-off precision.
 //
-// Same mapping and algorithm as k_quickpol_fp64 (one thread per band element (l'', l),
-// rows from the top; both
-// families forward from their own jmin and backward from jmax, matched at one
-// common point; here the two sweeps run interleaved in one loop), with:
+// Same mapping as k_quickpol_fp64 (one thread per band element (l'', l), rows from the top; both
+// families forward from their own jmin and backward from jmax, matched at one common point; here the
+// two sweeps run interleaved in one loop), on the Schulten-Gordon relation itself,
+//   j A(j+1) f(j+1) + B(j) f(j) + (j+1) A(j) f(j-1) = 0,
+// where the FP64 kernel runs a scaled form without roots and divisions.  Here:
 //   * P(j) = A(j)^2 = (j-|d|)(j+|d|)(s-j)(s+j)(j-|m3|)(j+|m3|) formed from its
 //     six exact integer factors (d = l1 - l2, s = l1 + l2 + 1): three exact
 //     two_prod pairs and two float-float products;
