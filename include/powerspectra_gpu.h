@@ -308,8 +308,7 @@ int ps_set_tensor_cores(ps_ctx *ctx, int enable);
  * launch, which the launch overlaps, is inside, that of ps_mcm_set and of a
  * batch is not, and a covariance set is timed whole), number of kernels this
  * context has launched, and a measured FMA-pipe peak (flop/s, FMA = 2 flops)
- * of this GPU in FP64 (fp64=1)
- * or FP32 (fp64=0). */
+ * of this GPU in FP64 (fp64=1) or FP32 (fp64=0). */
 double ps_last_kernel_ms(const ps_ctx *ctx);
 uint64_t ps_launch_count(const ps_ctx *ctx);
 int ps_probe_fma_peak(ps_ctx *ctx, int fp64, double *flops_per_s);
