@@ -456,6 +456,12 @@ static bool capturing(cudaStream_t s)
 // us into one of 347) and saves about 2.2e-5 (lmax / 1000)^3 s a call, so it is made when the calls that went
 // without have lost what it costs: at once from lmax 1651 on, after 21 calls at lmax 600.
 static const double kCoefWork = 4.5e9;
+// It may so come in a call long after the first: without disturbing a capture that another thread has begun.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
 {
     *out = ps::CoefRows{};
@@ -464,6 +470,7 @@ static int ensure_coef(ps_ctx* c, int lmax, ps::CoefRows* out)
         c->coef_due += (double)lmax * lmax * lmax;
         if (c->coef_due < kCoefWork) return PS_OK;
         unsigned char* t = nullptr;
+        const RelaxedCapture relaxed;
         if (cudaMalloc((void**)&t, ps::coef_bytes(lmax)) != cudaSuccess) {
             cudaGetLastError();
             c->coef_refused = lmax;  // a smaller table stays

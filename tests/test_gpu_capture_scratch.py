@@ -126,3 +126,42 @@ def test_window_spectrum_after_a_larger_one(own, larger, lmax):
     run()
     torch.cuda.synchronize()
     assert bool((got == out).all()) and bool((got > 0).all())
+
+
+def test_warm_calls_beside_another_threads_capture(own):
+    """Calls of a warmed-up context never end a capture that another thread has begun, also when a table is made or
+    replaced by one of them."""
+    import threading
+    from powerspectra_gpu import Context
+    ctx, s = own
+    a = Call(ctx, (0,), 80, "chosen")
+    want = a.direct()
+    other = Context(0)  # its own stream
+    b, c = Call(other, (2, 3), 600, "chosen"), Call(other, (2, 3), 640, "chosen")
+    torch.cuda.synchronize()
+    for x in (c, b):
+        x()
+        other.synchronize()
+    errors = []
+
+    def work():
+        try:
+            for _ in range(50):  # enqueued only: waiting is not allowed during another thread's capture
+                b()
+        except BaseException as e:  # reported by the test's own thread
+            errors.append(repr(e))
+
+    for _ in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            a()
+            t = threading.Thread(target=work)
+            t.start()
+            t.join()
+        other.synchronize()
+        assert not errors, errors
+        assert bool((a.replayed(g) == want).all())
+        b = c  # a larger table in the second capture
+        b()
+        other.synchronize()
+    other.close()
