@@ -505,7 +505,9 @@ static int run_coupling(ps_ctx* c, ps::CouplingParams& p, int mode, bool first =
         const size_t most = ps::slice_table_most(p.lmax);
         if (most > c->slices_cap) {
             const size_t twice = std::min(2 * c->slices_cap, ps::slice_table_most(PS_MAX_LMAX));
-            if ((st = ensure_bytes(c, &c->d_slices, &c->slices_cap, std::max(most, twice)))) return st;
+            if ((twice <= most || ensure_bytes(c, &c->d_slices, &c->slices_cap, twice)) &&
+                (st = ensure_bytes(c, &c->d_slices, &c->slices_cap, most)))
+                return st;
         }
         p.slices = c->d_slices;
         if (ps::reads_coef(p) && (st = ensure_coef(c, p.lmax, &p.coef))) return st;
@@ -1823,6 +1825,7 @@ int ps_batch_graph_launch(ps_ctx* c)
         int st = arm_status(c, c->stream);
         if (st) return st;
     }
+    if (capturing(c->stream)) b.recorded = true;
     PS_CUDA(c, cudaGraphLaunch(b.exec, c->stream));
     c->launches += batch_kernel_count(b);
     c->timed = true;
