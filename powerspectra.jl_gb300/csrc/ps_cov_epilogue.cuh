@@ -6,18 +6,23 @@
 
 namespace ps {
 
+// The FP64 kernels' root.  One function for the six of an element: a kernel of some 100 us runs its epilogue a few times,
+// and the code of six inlined roots took longer to arrive than to run (EE x EE at lmax 230 211 us, 187 with the function;
+// TT x EE at lmax 700 364 and 355; TE x TE at 230 154 and 155).
+static __device__ __noinline__ double root(double x) { return sqrt(x); }
+
 // X[k] are the Xi of windows W1..Wk (already divided by 4pi), Sa, Sb, Ra, Rb the spectra and noise
 // ratios at l1 = a and l2 = b, g[i] = sqrt(Sa[i] Sb[i]) for the spectra that need it (cov_roots).
 // ONE_ROOT: the root of a product of two such pairs as one root, as the reference takes it, for the FP64 kernels; the
 // product of the two roots has two roundings of 1e-16 more, which Xi with the fast arithmetic's 1e-7 do not show (the
-// further roots would cost TTTT and EEEE at lmax 700 3 %).  The roots are taken inside their case: ahead of the
+// further roots would cost TTTT and EEEE at lmax 700 3 %).  They are taken inside their case: ahead of the
 // switch, as predicated instructions or a loop, they cost every kind (TTEE at lmax 700 in FP64 364 -> 377 us).
 template <bool ONE_ROOT>
 __device__ __forceinline__ double cov_form(int kind, const double* Sa, const double* Sb, const double* g,
                                            const double* Ra, const double* Rb, const double* X)
 {
     auto product = [&](int i) {  // of the pairs i and i + 1
-        return ONE_ROOT ? sqrt(Sa[i] * Sb[i] * Sa[i + 1] * Sb[i + 1]) : g[i] * g[i + 1];
+        return ONE_ROOT ? root(Sa[i] * Sb[i] * Sa[i + 1] * Sb[i + 1]) : g[i] * g[i + 1];
     };
     switch (kind) {
     case PS_COV_TTTT:
@@ -65,7 +70,8 @@ __device__ __forceinline__ double cov_combine(int kind, const double* const* S, 
     for (int i = 0; i < 4; ++i) {
         Sa[i] = S[i][a];
         Sb[i] = S[i][b];
-        g[i] = i < ng ? sqrt(Sa[i] * Sb[i]) : 0.0;
+        const double p = Sa[i] * Sb[i];
+        g[i] = i < ng ? (ONE_ROOT ? root(p) : sqrt(p)) : 0.0;
         Ra[i] = i < nr ? R[i][a] : 0.0;
         Rb[i] = i < nr ? R[i][b] : 0.0;
     }
