@@ -1468,9 +1468,9 @@ struct QueueWork {
 // kCoefMaxLmax leaves the others without: the kernel reads it for all or none.
 static bool queue_reads_coef(const QueueWork& q, int gs, int nsm)
 {
-    if (gs > 4 || q.tasks == 0.0) return false;
-    const double warps = (double)nsm * ps::batch_blocks_per_sm(gs, true) * ps::kWarpsPerBlock;
-    return q.work >= 0.7 * warps * q.longest && q.work >= 70.0 * q.tasks;
+    const double warps = (double)nsm * ps::kWarpsPerBlock;  // of one block per SM
+    if (gs > 4 || q.tasks == 0.0 || q.work < 70.0 * q.tasks || q.work < 0.7 * warps * q.longest) return false;
+    return q.work >= 0.7 * warps * ps::batch_blocks_per_sm(gs, true) * q.longest;
 }
 
 int ps_batch_prepare(ps_ctx* c, const ps_problem* probs, int nprob, int gs, int bps)
